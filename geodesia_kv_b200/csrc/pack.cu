@@ -329,15 +329,133 @@ struct PagedUnpackParams {
     int D, group, G, gv;
 };
 
-__global__ void __launch_bounds__(kPackThreads) paged_unpack_kernel(PagedUnpackParams p) {
-    const int i = blockIdx.x, D = p.D;
-    const int lv = p.level[i];
+// ---- unpack, head dims 64 and 128 ----------------------------------------------------------------------
+// Bound: the fp32 stores (64 KB per block at D = 128 against at most 32 KB read).  One CTA per HALF of a
+// block (K or V), so that two thousand blocks already fill the chip several times over.  A thread owns four
+// neighbouring channels (one 16-byte store per token, a warp's store covers whole rows) of NI consecutive
+// tokens, which lie in one token group: its K scales are read once, and the codes of all its tokens are
+// requested before the first is used.  Codes become floats by the 2^23 trick (an OR and a subtraction, both
+// exact) and go through the same fused multiply-add as everywhere else, so the values are the same bits as
+// dequant_block_to_tiles gives; that remains for other shapes and for blocks, planes or outputs that are not
+// aligned for these loads.
+// Measured on 16 rows of 5000 tokens at 4 bits per value, D = 128, fp32 out (94 MB in all): 99 us with a thread per
+// element and byte loads, 17 us this way (5.5 TB/s).
+struct UnpackAt {
+    const uint8_t* blk; const __half* klo; const __half* kstep; const __half* vlo; const __half* vstep;
+    float* k_out; float* v_out; int lv;
+};
+template <int D>
+__device__ __forceinline__ bool locate(const UnpackParams& p, int i, UnpackAt& a) {
+    const int row = i / p.nb, blk = i - row * p.nb;
+    const size_t mi = (size_t)(p.per_row_meta ? row : 0) * p.nb + blk, sb = (size_t)i;
+    a.lv = p.level[mi];
+    if (!level_ok(a.lv)) return false;
+    a.blk = p.data + (size_t)row * p.stride_bh + p.offs[mi];
+    a.klo = p.klo + sb * p.G * D; a.kstep = p.kstep + sb * p.G * D;
+    a.vlo = p.vlo + sb * kP * p.gv; a.vstep = p.vstep + sb * kP * p.gv;
+    a.k_out = p.k_out + sb * kP * D; a.v_out = p.v_out + sb * kP * D;
+    return true;
+}
+template <int D>
+__device__ __forceinline__ bool locate(const PagedUnpackParams& p, int i, UnpackAt& a) {
+    a.lv = p.level[i];
     const int64_t off = p.offs[i];
-    if (!level_ok(lv) || off < 0) return;
-    const __half *klo, *kstep, *vlo, *vstep;
-    scales_behind(p.pool + off, lv, D, p.G, p.gv, klo, kstep, vlo, vstep);
-    dequant_block_to_tiles(p.pool + off, lv, D, p.group, p.gv, klo, kstep, vlo, vstep,
-                           p.k_out + (size_t)i * kP * D, p.v_out + (size_t)i * kP * D, D);
+    if (!level_ok(a.lv) || off < 0) return false;
+    a.blk = p.pool + off;
+    scales_behind(a.blk, a.lv, D, p.G, p.gv, a.klo, a.kstep, a.vlo, a.vstep);
+    a.k_out = p.k_out + (size_t)i * kP * D; a.v_out = p.v_out + (size_t)i * kP * D;
+    return true;
+}
+
+__device__ __forceinline__ float small_int_to_float(uint32_t c) {      // exact for c < 2^23
+    return __uint_as_float(0x4B000000u | c) - 8388608.0f;
+}
+
+template <int D, int LV>
+__device__ __forceinline__ void unpack_half(const uint8_t* __restrict__ half, const __half* __restrict__ lo,
+                                            const __half* __restrict__ step, bool values, int group, float* __restrict__ out) {
+    constexpr int QPR = D / 4, ROWS = kPackThreads / QPR, NI = kP / ROWS;
+    const int c4 = threadIdx.x % QPR, t0 = (threadIdx.x / QPR) * NI;
+    float4* o = reinterpret_cast<float4*>(out) + (size_t)t0 * QPR + c4;
+    if constexpr (LV == 1) {
+        const uint2 r = *reinterpret_cast<const uint2*>(half + 8 * c4);
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&r.y));
+#pragma unroll
+        for (int i = 0; i < NI; ++i) o[i * QPR] = make_float4(a.x, a.y, b.x, b.y);
+    } else if constexpr (LV == 16) {
+        uint2 r[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) r[i] = *reinterpret_cast<const uint2*>(half + (size_t)((t0 + i) * D + 4 * c4) * 2);
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+            o[i * QPR] = make_float4(__uint_as_float(r[i].x << 16), __uint_as_float(r[i].x & 0xffff0000u),
+                                     __uint_as_float(r[i].y << 16), __uint_as_float(r[i].y & 0xffff0000u));
+    } else {
+        uint32_t w[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const uint8_t* src = half + ((t0 + i) * D + 4 * c4) * LV / 8;
+            w[i] = LV == 8 ? *reinterpret_cast<const uint32_t*>(src) : LV == 4 ? *reinterpret_cast<const uint16_t*>(src) : *src;
+        }
+        float l[4], s[4];
+        const int vg = min(group, D), gv = D / vg, cg = 4 * c4 / vg;
+        if (!values) {
+            const size_t at = (size_t)(t0 / min(group, kP)) * D + 4 * c4;
+            const uint2 a = *reinterpret_cast<const uint2*>(lo + at), b = *reinterpret_cast<const uint2*>(step + at);
+            const float2 a0 = __half22float2(*reinterpret_cast<const __half2*>(&a.x)), a1 = __half22float2(*reinterpret_cast<const __half2*>(&a.y));
+            const float2 b0 = __half22float2(*reinterpret_cast<const __half2*>(&b.x)), b1 = __half22float2(*reinterpret_cast<const __half2*>(&b.y));
+            l[0] = a0.x; l[1] = a0.y; l[2] = a1.x; l[3] = a1.y;
+            s[0] = b0.x; s[1] = b0.y; s[2] = b1.x; s[3] = b1.y;
+        }
+        __half vl[NI], vs[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+            if (values) { vl[i] = lo[(t0 + i) * gv + cg]; vs[i] = step[(t0 + i) * gv + cg]; }
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            if (values) {
+                l[0] = l[1] = l[2] = l[3] = __half2float(vl[i]);
+                s[0] = s[1] = s[2] = s[3] = __half2float(vs[i]);
+            }
+            float x[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                x[c] = __fmaf_rn(small_int_to_float((w[i] >> (c * LV)) & ((1u << LV) - 1u)), s[c], l[c]);
+            o[i * QPR] = make_float4(x[0], x[1], x[2], x[3]);
+        }
+    }
+}
+
+template <int D, class P>
+__global__ void __launch_bounds__(kPackThreads) unpack_kernel(P p) {
+    UnpackAt a;
+    if (!locate<D>(p, (int)blockIdx.x, a)) return;
+    const bool values = blockIdx.y != 0;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(a.blk) | reinterpret_cast<uintptr_t>(a.klo) | reinterpret_cast<uintptr_t>(a.kstep) |
+                           reinterpret_cast<uintptr_t>(a.k_out) | reinterpret_cast<uintptr_t>(a.v_out);
+    if (bits & 15) {                                   // the CTA of the K half does both
+        if (!values)
+            dequant_block_to_tiles(a.blk, a.lv, D, p.group, p.gv, a.klo, a.kstep, a.vlo, a.vstep, a.k_out, a.v_out, D);
+        return;
+    }
+    const uint8_t* half = a.blk + (values ? half_bytes(a.lv, D) : 0);
+    const __half* lo = values ? a.vlo : a.klo;
+    const __half* step = values ? a.vstep : a.kstep;
+    float* out = values ? a.v_out : a.k_out;
+    if (a.lv == 16) unpack_half<D, 16>(half, lo, step, values, p.group, out);
+    else if (a.lv == 8) unpack_half<D, 8>(half, lo, step, values, p.group, out);
+    else if (a.lv == 4) unpack_half<D, 4>(half, lo, step, values, p.group, out);
+    else if (a.lv == 2) unpack_half<D, 2>(half, lo, step, values, p.group, out);
+    else unpack_half<D, 1>(half, lo, step, values, p.group, out);
+}
+
+template <class P>
+static int launch_unpack(const P& p, long n, cudaStream_t stream) {
+    if (n > 0x7fffffffL) return GKV_E_SHAPE;
+    if (p.D == 128) unpack_kernel<128, P><<<dim3((unsigned)n, 2), kPackThreads, 0, stream>>>(p);
+    else unpack_kernel<64, P><<<dim3((unsigned)n, 2), kPackThreads, 0, stream>>>(p);
+    GKV_LAUNCH_CHECK();
+    return GKV_OK;
 }
 
 
@@ -777,6 +895,8 @@ int gkv_unpack_blocks(const uint8_t* data, const int64_t* offs, const void* klo,
     p.level = level; p.k_out = k_out; p.v_out = v_out; p.nb = nb; p.D = D; p.group = group;
     p.G = (kP + group - 1) / group; p.gv = (D + group - 1) / group; p.per_row_meta = meta_rows != 1;
     p.stride_bh = stride_bh;
+    // the row form's planes are indexed with the caller's group; where it divides as the fast kernel assumes, that one runs
+    if (rq::shape_ok(D, group)) return launch_unpack(p, (long)rows * nb, (cudaStream_t)stream);
     unpack_blocks_kernel<<<dim3(nb, rows), kPackThreads, 0, (cudaStream_t)stream>>>(p);
     GKV_LAUNCH_CHECK();
     return GKV_OK;
@@ -832,9 +952,7 @@ int gkv_paged_unpack_blocks(const uint8_t* pool, const int64_t* offs, const int3
     PagedUnpackParams p;
     p.pool = pool; p.offs = offs; p.level = level; p.k_out = k_out; p.v_out = v_out; p.D = D; p.group = group;
     p.G = kP / min(group, kP); p.gv = D / min(group, D);
-    paged_unpack_kernel<<<n, kPackThreads, 0, (cudaStream_t)stream>>>(p);
-    GKV_LAUNCH_CHECK();
-    return GKV_OK;
+    return launch_unpack(p, n, (cudaStream_t)stream);
 }
 
 int gkv_paged_append_token(const void* k, const void* v, int src_dtype, uint8_t* pool, const int64_t* offs,
