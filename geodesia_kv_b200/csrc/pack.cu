@@ -178,6 +178,7 @@ __device__ void dequant_block_to_tiles(const uint8_t* __restrict__ blk, int lv, 
 }
 
 struct PackParams {
+    static constexpr bool kPacked = false, kMayRadii = false;
     const void* k; const void* v; int src_dtype;
     uint8_t* data; const int64_t* offs;
     __half* klo; __half* kstep; __half* vlo; __half* vstep;
@@ -249,6 +250,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_blocks_kernel(PackParams p)
 }
 
 struct DemoteParams {
+    static constexpr bool kPacked = true, kMayRadii = false;
     const uint8_t* data_old; const int64_t* offs_old; const int32_t* level_old;
     uint8_t* data_new; const int64_t* offs_new; const int32_t* level_new;
     __half* klo; __half* kstep; __half* vlo; __half* vstep;
@@ -309,6 +311,7 @@ __device__ __forceinline__ void scales_behind(const uint8_t* blk, int lv, int D,
 }
 
 struct PagedPackParams {
+    static constexpr bool kPacked = false, kMayRadii = true;
     const void* k; const void* v; int src_dtype;
     const int64_t* src_off; int64_t token_stride; const int32_t* nvalid;
     uint8_t* pool; const int64_t* dst_off; const int32_t* level;
@@ -317,6 +320,7 @@ struct PagedPackParams {
 };
 
 struct PagedDemoteParams {
+    static constexpr bool kPacked = true, kMayRadii = true;
     const uint8_t* pool_old; uint8_t* pool_new;
     const int64_t* off_old; const int32_t* level_old;
     const int64_t* off_new; const int32_t* level_new;
@@ -768,9 +772,10 @@ __global__ void __launch_bounds__(kStagedThreads, 2) staged_kernel(P p, int n, i
                 src.kind = 3;
                 src.v = st + half_bytes(d.old_level, D);
             }
+            src.k32 = s32(src.k); src.v32 = s32(src.v);
             src.klo = reinterpret_cast<const __half*>(st + kTileBytes); src.kstep = src.klo + G * D;
             src.vlo = src.kstep + G * D; src.vstep = src.vlo + kP * gv;
-            rq::requantise_staged<D>(src, j, sm.work);
+            rq::requantise_staged<D, P::kPacked, P::kMayRadii>(src, j, sm.work);
         }
         rq::work_sync();                               // every worker is done with the stage and the work area
         if (tid == 0) bar_arrive(&sm.empty[s]);
