@@ -46,6 +46,7 @@ SIGNATURES = {
     "gkv_paged_block_bytes": (_sz, [_i, _i, _i]),
     "gkv_paged_pack_blocks": (_i, [_vp, _vp, _i, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp] + [_i] * 4 + [_vp]),
     "gkv_paged_demote_blocks": (_i, [_vp] * 8 + [_i] * 4 + [_vp]),
+    "gkv_paged_plan_demotion": (_i, [_vp] * 5 + [_i64, C.POINTER(_f), C.c_double, _i, _i, _f, _f, _vp, _vp, _vp] + [_i] * 6 + [_vp]),
     "gkv_paged_unpack_blocks": (_i, [_vp] * 5 + [_i] * 4 + [_vp]),
     "gkv_paged_append_token": (_i, [_vp, _vp, _i] + [_vp] * 5 + [_i] * 4 + [_vp]),
     "gkv_paged_attn_decode": (_i, [_vp, _vp, _sz, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz] + [_i] * 7 + [_vp]),

@@ -10,6 +10,7 @@
 // available steps whose ratio is <= threshold, so a block that has already left rung 16
 // never moves again — the reference's behaviour, kept on purpose.
 #include "gkv_common.cuh"
+#include "requantise.cuh"
 
 namespace gkv {
 
@@ -30,92 +31,194 @@ struct AllocParams {
     float mass_power;
     int nb;
     const int32_t* nb_of;      // optional: blocks in use per problem (rows of a ragged batch); the rest keep their rung
+    // Table form (block tables of the paged pool): the ladder index, what must stay exact, the blocks in use and
+    // the budget follow from the row's rungs and its length, so idx, hot, nb_of and target_bits are not needed.
+    const int32_t* level; const int32_t* lens;
+    int64_t mass_stride, level_stride;
+    int sink_blocks, window_blocks;
+    double target_per_block;
 };
 
-template <typename T, typename Op>
-__device__ T block_reduce(T v, Op op, T* scratch) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    T r = scratch[0];
-    for (int w = 1; w < kAllocThreads / 32; ++w) r = op(r, scratch[w]);
-    return r;
+template <bool SMALL> struct SumOf { using type = double; };
+template <> struct SumOf<true> { using type = int; };
+
+// What the allocator has to know about block b of a problem.
+struct BlockState { int idx; bool hot; };
+template <bool TABLE>
+__device__ __forceinline__ BlockState block_state(const AllocParams& p, int prob, int b, int len) {
+    if (TABLE) {
+        const int lv = p.level[(size_t)prob * p.level_stride + b];
+        const int nbr = (len + kP - 1) / kP, open = len > 0 ? (len - 1) / kP : -1;
+        // sinks, the block being written and its predecessor, the recent window (policies.py:677-681)
+        const bool hot = (b < p.sink_blocks || b >= open - 1 || b >= nbr - p.window_blocks) && b < nbr;
+        return {(lv <= 8) + (lv <= 4) + (lv <= 2) + (lv <= 1), hot};
+    }
+    return {p.idx[(size_t)prob * p.nb + b], p.hot[(size_t)prob * p.nb + b] != 0};
 }
 
-// Ladder index a block lands on at threshold lam (the prefix rule).
-__device__ __forceinline__ int landing(const float* __restrict__ r4, int idx, bool hot, float lam) {
-    int pref = 0;
+// Marginal cost of every ladder step of a block: added damage per saved bit, `big` where the step is not open.
+__device__ __forceinline__ void step_ratios(const AllocParams& p, float mass, const float* __restrict__ E, const BlockState& st, float (&r)[4]) {
+    const float big = 3.4028234663852886e38f / 4.0f;
+    float mc = fmaxf(mass, 1e-12f);
+    if (p.mass_power != 1.0f) mc = powf(mc, p.mass_power);
+    float dmg[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) dmg[c] = __fmul_rn(mc, E[c]);
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
-        const bool ok = (r4[s] <= lam) && (s >= idx) && !hot;
-        if (ok && pref == s) pref = s + 1;
+        const float gain = fmaxf(__fsub_rn(p.bits[s], p.bits[s + 1]), 1e-9f);
+        const float cost = __fsub_rn(dmg[s + 1], dmg[s]);
+        r[s] = ((s >= st.idx) && !st.hot) ? __fdiv_rn(cost, gain) : big;
     }
-    return min(idx + pref, 4);
 }
 
-__global__ void __launch_bounds__(kAllocThreads) allocate_kernel(AllocParams p) {
-    __shared__ double sd[kAllocThreads / 32];
-    __shared__ uint32_t su[kAllocThreads / 32];
-    const int prob = blockIdx.x, tid = threadIdx.x;
-    const int nb_all = p.nb;
-    const int nb = p.nb_of ? max(0, min(nb_all, p.nb_of[prob])) : nb_all;
-    const float* mass = p.mass + (size_t)prob * nb_all;
+// Ladder index a block lands on at threshold lam: the prefix rule starts at step 0, so a block that has left rung
+// 16 (or must stay) does not move.
+__device__ __forceinline__ int landing(const float (&r)[4], const BlockState& st, float lam) {
+    if (st.idx != 0 || st.hot) return min(st.idx, 4);
+    int pref = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+        if (pref == s && r[s] <= lam) pref = s + 1;
+    return pref;
+}
+
+// Bound: latency — one CTA per row, and every candidate threshold is a sum over the row's blocks and a barrier.  So
+// several candidates are tried per round, the CTA has no more warps than the row has blocks, and rows of at most
+// 512 blocks (32k tokens) whose rungs cost whole numbers of bits (every ladder does) take SMALL: a block per
+// thread, its ratios in registers, and sums in integers, which one instruction adds up over a warp (seven candidates
+// per round: 11 rounds for fp32 keys).  Longer rows read the ratios back in every round and add doubles.
+template <bool SMALL, bool TABLE>
+__global__ void __launch_bounds__(kAllocThreads) allocate_kernel(const __grid_constant__ AllocParams p) {
+    constexpr int kCand = SMALL ? 7 : 3, kShift = SMALL ? 3 : 2;
+    using Sum = typename SumOf<SMALL>::type;
+    __shared__ Sum sums[2][kCand][kAllocThreads / 32];
+    __shared__ uint32_t su[2][kAllocThreads / 32];
+    const int prob = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+    const int nb_all = p.nb, len = TABLE ? p.lens[prob] : 0;
+    const int nb_row = TABLE ? (len + kP - 1) / kP : p.nb_of ? p.nb_of[prob] : nb_all;
+    const int nb = max(0, min(nb_all, nb_row));
+    const float* mass = p.mass + (size_t)prob * (TABLE ? p.mass_stride : (int64_t)nb_all);
     const float* E = p.E + (size_t)prob * nb_all * 5;
-    const int32_t* idx = p.idx + (size_t)prob * nb_all;
-    const uint8_t* hot = p.hot + (size_t)prob * nb_all;
-    float* ratio = p.ratio + (size_t)prob * nb_all * 4;
+    float* ratio = p.ratio ? p.ratio + (size_t)prob * nb_all * 4 : nullptr;
     int32_t* tgt = p.tgt + (size_t)prob * nb_all;
-    for (int b = nb + tid; b < nb_all; b += kAllocThreads) tgt[b] = idx[b];
-    const float big = 3.4028234663852886e38f / 4.0f;
+    for (int b = nb + tid; b < nb_all; b += blockDim.x) tgt[b] = block_state<TABLE>(p, prob, b, len).idx;
 
     uint32_t kmin = 0xffffffffu, kmax = 0u;
-    for (int b = tid; b < nb; b += kAllocThreads) {
-        float mc = fmaxf(mass[b], 1e-12f);
-        if (p.mass_power != 1.0f) mc = powf(mc, p.mass_power);
-        float dmg[5];
-#pragma unroll
-        for (int c = 0; c < 5; ++c) dmg[c] = __fmul_rn(mc, E[b * 5 + c]);
-        const int id = idx[b];
-        const bool h = hot[b] != 0;
+    float mine[4] = {0.f, 0.f, 0.f, 0.f};
+    BlockState my{4, true};
+    for (int b = tid; b < nb; b += blockDim.x) {
+        my = block_state<TABLE>(p, prob, b, len);
+        step_ratios(p, mass[b], E + b * 5, my, mine);
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const float gain = fmaxf(__fsub_rn(p.bits[s], p.bits[s + 1]), 1e-9f);
-            const float cost = __fsub_rn(dmg[s + 1], dmg[s]);
-            const float r = ((s >= id) && !h) ? __fdiv_rn(cost, gain) : big;
-            ratio[b * 4 + s] = r;
-            const uint32_t k = float_key(r);
+            if (ratio) ratio[b * 4 + s] = mine[s];
+            const uint32_t k = float_key(mine[s]);
             kmin = min(kmin, k);
             kmax = max(kmax, k);
         }
     }
-    kmin = block_reduce(kmin, [](uint32_t a, uint32_t b) { return a < b ? a : b; }, su);
-    kmax = block_reduce(kmax, [](uint32_t a, uint32_t b) { return a > b ? a : b; }, su);
-    __syncthreads();   // ratio[] written by this CTA is read back below
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if (lane == 0) { su[0][warp] = kmin; su[1][warp] = kmax; }
+    __syncthreads();                           // also: ratio[] written by this CTA is read back below
+    for (int w = 0; w < nwarp; ++w) { kmin = min(kmin, su[0][w]); kmax = max(kmax, su[1][w]); }
     if (nb == 0) return;
 
-    const float target = (float)p.target_bits[prob];   // fp32 comparison, as torch does
-    auto fits = [&](float lam) -> bool {
-        double tot = 0.0;
-        for (int b = tid; b < nb; b += kAllocThreads)
-            tot += (double)p.bits[landing(ratio + b * 4, idx[b], hot[b] != 0, lam)];
-        tot = block_reduce(tot, [](double a, double b) { return a + b; }, sd);
-        return !((float)tot > target);
+    const float target = TABLE ? (float)((double)nb_row * p.target_per_block) : (float)p.target_bits[prob];   // fp32 comparison, as torch does
+    const Sum bits[5] = {(Sum)p.bits[0], (Sum)p.bits[1], (Sum)p.bits[2], (Sum)p.bits[3], (Sum)p.bits[4]};
+    auto land = [&](int b, float lam) -> int {
+        if constexpr (SMALL) {
+            return landing(mine, my, lam);
+        } else {
+            float r[4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) r[s] = ratio[b * 4 + s];
+            return landing(r, block_state<TABLE>(p, prob, b, len), lam);
+        }
+    };
+    int par = 0;
+    auto fits = [&](const float (&lam)[kCand], bool (&ok)[kCand]) {
+        Sum tot[kCand];
+#pragma unroll
+        for (int c = 0; c < kCand; ++c) tot[c] = 0;
+        for (int b = tid; b < nb; b += blockDim.x) {
+#pragma unroll
+            for (int c = 0; c < kCand; ++c) {
+                const int l = land(b, lam[c]);
+                tot[c] += l == 0 ? bits[0] : l == 1 ? bits[1] : l == 2 ? bits[2] : l == 3 ? bits[3] : bits[4];
+            }
+        }
+        if constexpr (SMALL) {
+#pragma unroll
+            for (int c = 0; c < kCand; ++c) tot[c] = __reduce_add_sync(0xffffffffu, tot[c]);
+        } else {
+#pragma unroll
+            for (int o = 16; o; o >>= 1)
+#pragma unroll
+                for (int c = 0; c < kCand; ++c) tot[c] += __shfl_xor_sync(0xffffffffu, tot[c], o);
+        }
+        if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < kCand; ++c) sums[par][c][warp] = tot[c];
+        __syncthreads();                       // two buffers in turn: one barrier per round is enough
+#pragma unroll
+        for (int c = 0; c < kCand; ++c) {
+            Sum r = sums[par][c][0];
+            for (int w = 1; w < nwarp; ++w) r += sums[par][c][w];
+            ok[c] = !((float)r > target);
+        }
+        par ^= 1;
     };
 
     uint32_t lo = kmin, hi = kmax;
-    if (fits(key_float(kmax))) {
+    bool ok[kCand];
+    float lam[kCand];
+#pragma unroll
+    for (int c = 0; c < kCand; ++c) lam[c] = key_float(kmax);
+    fits(lam, ok);
+    if (ok[0]) {
         while (lo < hi) {
-            const uint32_t mid = lo + ((hi - lo) >> 1);
-            if (fits(key_float(mid))) hi = mid;
-            else lo = mid + 1;
+            uint32_t m[kCand];
+#pragma unroll
+            for (int c = 0; c < kCand; ++c) {
+                m[c] = lo + (uint32_t)(((unsigned long long)(hi - lo) * (unsigned)(c + 1)) >> kShift);
+                lam[c] = key_float(m[c]);
+            }
+            fits(lam, ok);
+            // the first candidate that fits and the last that does not close the interval
+            uint32_t nlo = lo, nhi = hi;
+#pragma unroll
+            for (int c = kCand - 1; c >= 0; --c)
+                if (ok[c]) nhi = m[c];
+#pragma unroll
+            for (int c = 0; c < kCand; ++c)
+                if (!ok[c]) nlo = m[c] + 1;
+            lo = nlo;
+            hi = nhi;
         }
     }
-    const float lam = key_float(hi);
-    for (int b = tid; b < nb; b += kAllocThreads)
-        tgt[b] = landing(ratio + b * 4, idx[b], hot[b] != 0, lam);
+    const float best = key_float(hi);
+    for (int b = tid; b < nb; b += blockDim.x) tgt[b] = land(b, best);
+}
+
+// Sums in integers are the doubles' sums when every rung costs a whole number of bits and 512 of them fit 31 bits.
+static bool whole_bits(const float (&bits)[5]) {
+    for (float b : bits)
+        if (!(b >= 0.f && b <= 4194303.f && b == (float)(int)b)) return false;
+    return true;
+}
+
+template <bool TABLE>
+static int launch_allocate(const AllocParams& p, int problems, cudaStream_t stream) {
+    if (p.nb <= kAllocThreads && whole_bits(p.bits)) {
+        const int threads = (p.nb + 31) & ~31;
+        allocate_kernel<true, TABLE><<<problems, threads, 0, stream>>>(p);
+    } else {
+        allocate_kernel<false, TABLE><<<problems, kAllocThreads, 0, stream>>>(p);
+    }
+    GKV_LAUNCH_CHECK();
+    return GKV_OK;
 }
 
 // ---- distortion table (policies.py:774-808) from rung-16 blocks of the packed cache ------
@@ -124,6 +227,7 @@ struct DistParams {
     int nb, D, group, per_row_meta;
     float value_weight;
     int64_t stride_bh;
+    int tab_stride;            // entries between the rows of offs and level (nb, or the width of a wider table)
 };
 
 constexpr int kDistThreads = 256;
@@ -146,7 +250,7 @@ __global__ void __launch_bounds__(kDistThreads) distortion_kernel(DistParams p) 
     float* ev = ek + 3 * G;              // [3][64]
     const int blk = blockIdx.x, row = blockIdx.y;
     const int mrow = p.per_row_meta ? row : 0;
-    const size_t mi = (size_t)mrow * p.nb + blk;
+    const size_t mi = (size_t)mrow * p.tab_stride + blk;
     float* Eo = p.E + ((size_t)row * p.nb + blk) * 5;
     if (p.level[mi] != 16) {
         if (tid < 5) Eo[tid] = 0.f;
@@ -235,6 +339,204 @@ __global__ void __launch_bounds__(kDistThreads) distortion_kernel(DistParams p) 
     }
 }
 
+// Head dims 64 and 128.  Every sum of the table is a serial fp32 chain in the reference's order (the allocator's
+// decisions hang on its last bit), so what bounds a block is the length of those chains, and what bounds the
+// launch is how many blocks an SM holds: the block stays in shared memory as the 16-bit rows it came as (17 KB),
+// three warps work on it, and ten CTAs fit an SM.  Columns first (a thread owns a channel pair: means, and the K
+// ranges by packed minimum and maximum, squared for the three rungs right away), then rows (a thread owns a token; rows are
+// padded by 16 bytes, so that eight lanes' 16-byte loads meet no bank twice) while the third warp adds up the
+// rungs' squares.  Square roots are monotonic and correctly rounded, so the maxima are taken over the sums.
+//
+// With value_weight = 0 the V half enters the table as 0 * b, which is 0 unless b is infinite or not a number;
+// b is finite if all |V| are below 2^40, so V is then only looked over, and worked through only if that fails.
+constexpr int kDistRowThreads = 96;
+template <int D>
+struct DistSmem {
+    static constexpr int LDB = 2 * D + 16;         // bytes per token row
+    static constexpr int LDQ = D + 4;              // floats per row of squares
+    alignas(16) uint8_t tile[kP * LDB];
+    alignas(16) float mean[D];
+    alignas(16) float sq[3 * 4 * LDQ];             // [rung][token group][channel]
+    uint32_t top[8];                               // K: largest sum per rung, of the centroid; V: the same
+    int v_large;
+};
+
+// Largest of the warp's non-negative sums into *top; one that is not a number counts as nothing, as in fmaxf.
+__device__ __forceinline__ void keep_max(uint32_t* top, float sum) {
+    const uint32_t u = __reduce_max_sync(0xffffffffu, sum == sum ? __float_as_uint(sum) : 0u);
+    if ((threadIdx.x & 31) == 0) atomicMax(top, u);
+}
+
+// Half a block on its way into the tile: asynchronous copies, so that they overlap with whatever follows up to
+// distortion_half (which waits for them).
+template <int D>
+__device__ __forceinline__ void distortion_load(const uint8_t* __restrict__ src, DistSmem<D>& sm) {
+    constexpr int LDB = DistSmem<D>::LDB, OPR = D / 8;
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+        const uint32_t tile = (uint32_t)__cvta_generic_to_shared(sm.tile);
+        for (int e = threadIdx.x; e < kP * OPR; e += kDistRowThreads)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tile + (uint32_t)((e / OPR) * LDB + (e % OPR) * 16)), "l"(src + 16 * e) : "memory");
+    } else {
+        for (int e = threadIdx.x; e < kP * D; e += kDistRowThreads)
+            reinterpret_cast<uint16_t*>(sm.tile + (e / D) * LDB)[e % D] = reinterpret_cast<const uint16_t*>(src)[e];
+    }
+}
+
+template <int D, bool VALUES>
+__device__ __forceinline__ void distortion_half(DistSmem<D>& sm, int kg, int vg) {
+    constexpr int LDB = DistSmem<D>::LDB, LDQ = DistSmem<D>::LDQ, OPR = D / 8;
+    const int tid = threadIdx.x, lane = tid & 31, G = kP / kg;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (tid < D / 2) {
+        float s0 = 0.f, s1 = 0.f;
+        const uint8_t* col = sm.tile + 4 * tid;
+        for (int tg = 0; tg < G; ++tg) {
+            uint32_t lo = 0x7F807F80u, hi = 0xFF80FF80u;       // +inf, -inf
+            for (int i0 = 0; i0 < kg; i0 += 16) {
+                uint32_t w[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) w[i] = *reinterpret_cast<const uint32_t*>(col + (tg * kg + i0 + i) * LDB);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    s0 = __fadd_rn(s0, __uint_as_float(w[i] << 16));
+                    s1 = __fadd_rn(s1, __uint_as_float(w[i] & 0xffff0000u));
+                    if (!VALUES) { lo = rq::min2<1>(lo, w[i]); hi = rq::max2<1>(hi, w[i]); }
+                }
+            }
+            if (!VALUES) {
+                const float r0 = __fsub_rn(__uint_as_float(hi << 16), __uint_as_float(lo << 16));
+                const float r1 = __fsub_rn(__uint_as_float(hi & 0xffff0000u), __uint_as_float(lo & 0xffff0000u));
+#pragma unroll
+                for (int li = 0; li < 3; ++li) {
+                    const float den = 2.0f * (float)((1 << (8 >> li)) - 1);
+                    const float a = __fdiv_rn(r0, den), b = __fdiv_rn(r1, den);
+                    *reinterpret_cast<float2*>(sm.sq + (li * G + tg) * LDQ + 2 * tid) = make_float2(__fmul_rn(a, a), __fmul_rn(b, b));
+                }
+            }
+        }
+        *reinterpret_cast<float2*>(sm.mean + 2 * tid) = make_float2(__fdiv_rn(s0, (float)kP), __fdiv_rn(s1, (float)kP));
+    }
+    __syncthreads();
+    if (tid < kP) {
+        const uint8_t* row = sm.tile + tid * LDB;
+        float s = 0.f, e[3] = {0.f, 0.f, 0.f};
+        uint32_t lo = 0x7F807F80u, hi = 0xFF80FF80u;
+#pragma unroll 2
+        for (int o = 0; o < OPR; ++o) {
+            const uint4 r = *reinterpret_cast<const uint4*>(row + 16 * o);
+            const float4 m0 = *reinterpret_cast<const float4*>(sm.mean + 8 * o), m1 = *reinterpret_cast<const float4*>(sm.mean + 8 * o + 4);
+            const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+            const float mu[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float x0 = __fsub_rn(__uint_as_float(w[c] << 16), mu[2 * c]);
+                const float x1 = __fsub_rn(__uint_as_float(w[c] & 0xffff0000u), mu[2 * c + 1]);
+                s = __fadd_rn(s, __fmul_rn(x0, x0));
+                s = __fadd_rn(s, __fmul_rn(x1, x1));
+                if (VALUES) { lo = rq::min2<1>(lo, w[c]); hi = rq::max2<1>(hi, w[c]); }
+            }
+            if (VALUES && (8 * o + 8) % vg == 0) {             // the end of a channel group
+                const float h = fmaxf(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u));
+                const float l = fminf(__uint_as_float(lo << 16), __uint_as_float(lo & 0xffff0000u));
+                const float range = __fsub_rn(h, l);
+#pragma unroll
+                for (int li = 0; li < 3; ++li) {
+                    const float x = __fdiv_rn(range, 2.0f * (float)((1 << (8 >> li)) - 1));
+                    e[li] = __fadd_rn(e[li], __fmul_rn(__fmul_rn(x, x), (float)vg));
+                }
+                lo = 0x7F807F80u; hi = 0xFF80FF80u;
+            }
+        }
+        keep_max(&sm.top[VALUES ? 7 : 3], s);
+        if (VALUES)
+#pragma unroll
+            for (int li = 0; li < 3; ++li) keep_max(&sm.top[4 + li], e[li]);
+    } else if (!VALUES) {                                      // the third warp: one lane per (rung, token group)
+        float s = 0.f;
+        if (lane < 3 * G) {
+            const float4* q = reinterpret_cast<const float4*>(sm.sq + lane * LDQ);
+#pragma unroll 8
+            for (int d = 0; d < D / 4; ++d) {
+                const float4 v = q[d];
+                s = __fadd_rn(s, v.x); s = __fadd_rn(s, v.y); s = __fadd_rn(s, v.z); s = __fadd_rn(s, v.w);
+            }
+        }
+#pragma unroll
+        for (int li = 0; li < 3; ++li) keep_max(&sm.top[li], lane / G == li ? s : 0.f);
+    }
+    __syncthreads();
+}
+
+template <int D>
+__global__ void __launch_bounds__(kDistRowThreads) distortion_rows_kernel(DistParams p) {
+    __shared__ DistSmem<D> sm;
+    const int tid = threadIdx.x;
+    const int kg = min(p.group, kP), vg = min(p.group, D);
+    const int blk = blockIdx.x, row = blockIdx.y;
+    const size_t mi = (size_t)(p.per_row_meta ? row : 0) * p.tab_stride + blk;
+    float* Eo = p.E + ((size_t)row * p.nb + blk) * 5;
+    if (p.level[mi] != 16) {
+        if (tid < 5) Eo[tid] = 0.f;
+        return;
+    }
+    const uint8_t* kb = p.data + (size_t)row * p.stride_bh + p.offs[mi];
+    const uint8_t* vb = kb + kP * D * 2;
+    if (tid < 8) sm.top[tid] = 0u;
+    if (tid == 0) sm.v_large = 0;
+    bool need_v = p.value_weight != 0.f;
+    distortion_load<D>(kb, sm);
+    if (!need_v) {
+        uint32_t big = 0u;
+        if ((reinterpret_cast<uintptr_t>(vb) & 15) == 0) {
+#pragma unroll 11
+            for (int e = tid; e < kP * D / 8; e += kDistRowThreads) {
+                const uint4 r = reinterpret_cast<const uint4*>(vb)[e];
+                big = __vmaxu2(__vmaxu2(__vmaxu2(big, r.x & 0x7fff7fffu), __vmaxu2(r.y & 0x7fff7fffu, r.z & 0x7fff7fffu)), r.w & 0x7fff7fffu);
+            }
+        } else {
+            for (int e = tid; e < kP * D; e += kDistRowThreads) big = max(big, (uint32_t)reinterpret_cast<const uint16_t*>(vb)[e] & 0x7fffu);
+        }
+        __syncthreads();
+        constexpr uint32_t k2p40 = (127u + 40u) << 7;          // 2^40 as bf16
+        if ((big & 0xffffu) >= k2p40 || (big >> 16) >= k2p40) sm.v_large = 1;
+    }
+    distortion_half<D, false>(sm, kg, vg);                     // its barriers also publish v_large
+    need_v = need_v || sm.v_large != 0;
+    if (need_v) {
+        distortion_load<D>(vb, sm);
+        distortion_half<D, true>(sm, kg, vg);
+    }
+    if (tid < 5) {
+        float a = 0.f, b = 0.f;
+        if (tid > 0) {
+            a = __fsqrt_rn(__uint_as_float(sm.top[tid - 1]));
+            b = need_v ? __fsqrt_rn(__uint_as_float(sm.top[3 + tid])) : 0.f;
+        }
+        Eo[tid] = __fadd_rn(a, __fmul_rn(p.value_weight, b));
+    }
+}
+
+static int launch_distortion(const DistParams& p, int rows, cudaStream_t stream) {
+    const int nb = p.nb, D = p.D;
+    const int kg = min(p.group, kP), vg = min(p.group, D);
+    const int G = kP / kg, gv = D / vg;
+    if (rq::shape_ok(D, p.group)) {
+        if (p.D == 128) distortion_rows_kernel<128><<<dim3(nb, rows), kDistRowThreads, 0, stream>>>(p);
+        else distortion_rows_kernel<64><<<dim3(nb, rows), kDistRowThreads, 0, stream>>>(p);
+        GKV_LAUNCH_CHECK();
+        return GKV_OK;
+    }
+    const size_t smem = sizeof(float) * ((size_t)2 * kP * (D + 1) + (size_t)G * D + (size_t)kP * gv + 2 * D + 2 * kP + 3 * G + 3 * kP);
+    const size_t smem_max = sizeof(float) * ((size_t)2 * kP * (kMaxD + 1) + (size_t)kP * kMaxD + (size_t)kP * kMaxD + 2 * kMaxD + 2 * kP + 3 * kP + 3 * kP);
+    GKV_CUDA_TRY(cudaFuncSetAttribute(distortion_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(smem_max > 227 * 1024 ? 227 * 1024 : smem_max)));
+    if (smem > 227 * 1024) return GKV_E_SHAPE;
+    distortion_kernel<<<dim3(nb, rows), kDistThreads, smem, stream>>>(p);
+    GKV_LAUNCH_CHECK();
+    return GKV_OK;
+}
+
 }  // namespace gkv
 
 extern "C" {
@@ -258,9 +560,9 @@ int gkv_allocate_ragged(const float* mass, const float* E, const int32_t* idx, c
     p.mass = mass; p.E = E; p.idx = idx; p.hot = hot; p.target_bits = target_bits; p.ratio = ratio;
     p.tgt = tgt_idx; p.mass_power = mass_power; p.nb = nb; p.nb_of = nb_of;
     for (int i = 0; i < 5; ++i) p.bits[i] = bits_host[i];
-    allocate_kernel<<<problems, kAllocThreads, 0, (cudaStream_t)stream>>>(p);
-    GKV_LAUNCH_CHECK();
-    return GKV_OK;
+    p.level = nullptr; p.lens = nullptr; p.mass_stride = p.level_stride = nb;
+    p.sink_blocks = p.window_blocks = 0; p.target_per_block = 0.0;
+    return launch_allocate<false>(p, problems, (cudaStream_t)stream);
 }
 
 int gkv_block_distortion(const uint8_t* data, const int64_t* offs, const int32_t* level, float* E, int rows,
@@ -274,17 +576,34 @@ int gkv_block_distortion(const uint8_t* data, const int64_t* offs, const int32_t
     if (!data || !offs || !level || !E) return GKV_E_NULL;
     DistParams p;
     p.data = data; p.offs = offs; p.level = level; p.E = E; p.nb = nb; p.D = D; p.group = group;
-    p.per_row_meta = meta_rows != 1; p.value_weight = value_weight; p.stride_bh = stride_bh;
-    const int kg = min(group, kP), vg = min(group, D);
-    const int G = kP / kg, gv = D / vg;
-    const size_t smem = sizeof(float) * ((size_t)2 * kP * (D + 1) + (size_t)G * D + (size_t)kP * gv + 2 * D + 2 * kP + 3 * G + 3 * kP);
-    const size_t smem_max = sizeof(float) * ((size_t)2 * kP * (kMaxD + 1) + (size_t)kP * kMaxD + (size_t)kP * kMaxD + 2 * kMaxD + 2 * kP + 3 * kP + 3 * kP);
-    GKV_CUDA_TRY(cudaFuncSetAttribute(distortion_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(smem_max > 227 * 1024 ? 227 * 1024 : smem_max)));
-    if (smem > 227 * 1024) return GKV_E_SHAPE;
-    distortion_kernel<<<dim3(nb, rows), kDistThreads, smem, (cudaStream_t)stream>>>(p);
-    GKV_LAUNCH_CHECK();
-    return GKV_OK;
+    p.per_row_meta = meta_rows != 1; p.value_weight = value_weight; p.stride_bh = stride_bh; p.tab_stride = nb;
+    return launch_distortion(p, rows, (cudaStream_t)stream);
+}
+
+int gkv_paged_plan_demotion(const uint8_t* pool, const int64_t* offs, const int32_t* level, const int32_t* lens,
+                            const float* mass, int64_t mass_stride, const float* bits_host, double target_per_block,
+                            int sink_blocks, int window_blocks, float mass_power, float value_weight, float* E,
+                            float* ratio, int32_t* tgt_idx, int rows, int nb, int cap, int D, int block, int group,
+                            void* stream) {
+    using namespace gkv;
+    if (block != kP) return GKV_E_BLOCK;
+    if (rows <= 0 || nb < 0 || cap < nb || !rq::shape_ok(D, group)) return GKV_E_SHAPE;
+    if (nb == 0) return GKV_OK;
+    if (mass_stride < nb) return GKV_E_ARG;
+    if (!pool || !offs || !level || !lens || !mass || !bits_host || !E || !tgt_idx) return GKV_E_NULL;
+    DistParams d;
+    d.data = pool; d.offs = offs; d.level = level; d.E = E; d.nb = nb; d.D = D; d.group = group;
+    d.per_row_meta = 1; d.value_weight = value_weight; d.stride_bh = 0; d.tab_stride = cap;
+    if (const int rc = launch_distortion(d, rows, (cudaStream_t)stream)) return rc;
+    AllocParams p;
+    p.mass = mass; p.E = E; p.idx = nullptr; p.hot = nullptr; p.target_bits = nullptr;
+    p.ratio = ratio; p.tgt = tgt_idx; p.mass_power = mass_power; p.nb = nb; p.nb_of = nullptr;
+    for (int i = 0; i < 5; ++i) p.bits[i] = bits_host[i];
+    if (nb <= kAllocThreads && whole_bits(p.bits)) p.ratio = nullptr;      // the kernel that keeps ratios in registers
+    else if (!ratio) return GKV_E_NULL;
+    p.level = level; p.lens = lens; p.mass_stride = mass_stride; p.level_stride = cap;
+    p.sink_blocks = sink_blocks; p.window_blocks = window_blocks; p.target_per_block = target_per_block;
+    return launch_allocate<true>(p, rows, (cudaStream_t)stream);
 }
 
 }  // extern "C"

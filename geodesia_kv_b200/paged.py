@@ -378,25 +378,21 @@ class PagedLayerCache:
         (rows, nb) int32 ON THE DEVICE (nothing is read back here)."""
         from .policies import ladder_bits
         nb, dev, rows, D = self.nb, self.device, self.rows, self.D
-        offs, level = self.offs[:, :nb].contiguous(), self.level[:, :nb].contiguous()
+        m = self.mass if mass is None else mass
+        if m.dtype != torch.float32 or m.stride(-1) != 1 or m.stride(0) < nb or m.shape[0] != rows or m.shape[1] < nb:
+            m = m.expand(rows, nb).to(torch.float32).contiguous()
         E = torch.empty(rows, nb, 5, dtype=torch.float32, device=dev)
-        m = (self.mass[:, :nb] if mass is None else mass).contiguous()
-        idx = ((level <= 8).to(torch.int32) + (level <= 4).to(torch.int32) + (level <= 2).to(torch.int32)
-               + (level <= 1).to(torch.int32)).contiguous()
-        hot = self.hot_blocks(nb, sinks, window)
-        nb_of = ((self.lens + (BLOCK - 1)) // BLOCK).to(torch.int32).contiguous()
-        target = (nb_of.to(torch.float64) * (budget_bits * 2.0 * BLOCK * D)).contiguous()
-        ratio = torch.empty(rows, nb, 4, dtype=torch.float32, device=dev)
+        ratio = torch.empty(rows, nb, 4, dtype=torch.float32, device=dev) if nb > 512 else None     # longer rows keep them in memory
         tgt = torch.empty(rows, nb, dtype=torch.int32, device=dev)
         bits = (C.c_float * 5)(*ladder_bits(BLOCK, D, self.group))
         with torch.cuda.device(dev):
-            rc = self.lib.gkv_block_distortion(self.pool.data.data_ptr(), offs.data_ptr(), level.data_ptr(), E.data_ptr(),
-                                               rows, nb, D, BLOCK, self.group, float(value_weight), 0, rows, _stream(dev))
-            _lib.check(rc, "gkv_block_distortion")
-            rc = self.lib.gkv_allocate_ragged(m.data_ptr(), E.data_ptr(), idx.data_ptr(), hot.data_ptr(), bits,
-                                              target.data_ptr(), float(mass_power), ratio.data_ptr(), tgt.data_ptr(),
-                                              nb_of.data_ptr(), rows, nb, _stream(dev))
-            _lib.check(rc, "gkv_allocate_ragged")
+            rc = self.lib.gkv_paged_plan_demotion(self.pool.data.data_ptr(), self.offs.data_ptr(), self.level.data_ptr(),
+                                                  self.lens.data_ptr(), m.data_ptr(), m.stride(0), bits,
+                                                  float(budget_bits * 2.0 * BLOCK * D), max(1, (sinks + BLOCK - 1) // BLOCK),
+                                                  max(1, (window + BLOCK - 1) // BLOCK), float(mass_power), float(value_weight),
+                                                  E.data_ptr(), ratio.data_ptr() if nb > 512 else None, tgt.data_ptr(), rows, nb,
+                                                  self.cap, D, BLOCK, self.group, _stream(dev))
+        _lib.check(rc, "gkv_paged_plan_demotion")
         return tgt
 
     def apply_demotion(self, tgt_idx_host: np.ndarray) -> int:

@@ -295,6 +295,19 @@ int gkv_paged_demote_blocks(const uint8_t *pool_old, const int64_t *off_old, con
                             uint8_t *pool_new, const int64_t *off_new, const int32_t *level_new,
                             float *ek, float *ev, int n, int D, int block, int group, void *stream);
 
+/* Distortion table and rung allocation (gkv_block_distortion, gkv_allocate_ragged) straight from a block
+ * table: the ladder index follows from level, the blocks in use and what must stay exact (the first
+ * sink_blocks, the open block, its predecessor, the last window_blocks; policies.py:677-681) from lens, the
+ * budget of a row is target_per_block bits times its blocks in use.  mass: rows mass_stride floats apart.
+ * E (rows, nb, 5) and ratio (rows, nb, 4) are scratch (ratio may be NULL for nb <= 512 and whole bits);
+ * tgt_idx (rows, nb) int32.                                                                            */
+int gkv_paged_plan_demotion(const uint8_t *pool, const int64_t *offs, const int32_t *level,
+                            const int32_t *lens, const float *mass, int64_t mass_stride,
+                            const float *bits_host, double target_per_block, int sink_blocks,
+                            int window_blocks, float mass_power, float value_weight, float *E,
+                            float *ratio, int32_t *tgt_idx, int rows, int nb, int cap, int D, int block,
+                            int group, void *stream);
+
 /* Exact dequantisation of n pool blocks -> fp32 k_out, v_out (n, 64, D) (tests, debugging).   */
 int gkv_paged_unpack_blocks(const uint8_t *pool, const int64_t *offs, const int32_t *level,
                             float *k_out, float *v_out, int n, int D, int block, int group,

@@ -76,3 +76,79 @@ def test_pack_awkward_values(oracle, D, group, dtype):
         for key in ("klo", "kstep", "vlo", "vstep"):
             got, ref = (a.view(np.float16) for a in (getattr(cache, key).cpu().view(torch.int16).numpy().view(np.uint16)[0, 0], want[key]))
             assert np.array_equal(got, ref, equal_nan=True), (kind, key)
+
+
+@pytest.mark.parametrize("D,group", [(128, 32), (128, 16), (128, 64), (64, 16), (64, 64), (96, 32)])
+@pytest.mark.parametrize("value_weight", [0.0, 0.5])
+def test_distortion_edges(oracle, D, group, value_weight):
+    """The V half enters with weight 0 unless one of its values is too large for that to be 0."""
+    from geodesia_kv_b200 import policies
+    from geodesia_kv_b200.pack_layout import pack_cache
+    nb = 6
+    k = torch.from_numpy(awkward(1, (nb, 64, D), 1)).bfloat16()
+    v = torch.from_numpy(awkward(2, (nb, 64, D), 1)).bfloat16()
+    v[1, 3, 5] = 2.0 ** 41
+    v[2, 60, D - 1] = float("inf")
+    v[3, 0, 0] = float("nan")
+    k[4, 7, 9] = float("inf")
+    level = torch.full((1, 1, nb), 16, dtype=torch.int32, device="cuda")
+    cache = pack_cache(k.cuda().view(1, 1, -1, D), v.cuda().view(1, 1, -1, D), level, group)
+    E = policies.block_distortion(cache, value_weight).cpu().numpy()[0, 0]
+    want = oracle.distortion(k.float().numpy(), v.float().numpy(), group, value_weight)
+    assert np.array_equal(E, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("nb", [1, 32, 33, 100, 512, 513])
+@pytest.mark.parametrize("whole", [True, False])
+def test_allocate_sizes(oracle, nb, whole):
+    """A block per thread up to 512, several above; rungs that cost whole bits are added as integers."""
+    import ctypes as C
+    from geodesia_kv_b200 import _lib
+    lib, rows = _lib.load(), 5
+    rng = np.random.default_rng(nb)
+    E = ((np.abs(rng.standard_normal((rows, nb, 1))) + 0.5) * np.array([0.0, 0.02, 0.3, 1.5, 6.0])).astype(np.float32)
+    mass = rng.random((rows, nb), dtype=np.float32)
+    idx = np.maximum(rng.integers(-4, 5, (rows, nb)), 0).astype(np.int32)
+    hot = (rng.random((rows, nb)) < 0.1).astype(np.uint8)
+    bits = np.array([262144, 147456, 81920, 49152, 4096], np.float32) + (0 if whole else 0.25)
+    budget = np.array([0.1, 2.5, 4.0, 7.0, 50.0]) * 2 * 64 * 128 * nb
+    cu = [torch.from_numpy(a).cuda() for a in (mass, E, idx, hot, budget)]
+    ratio, tgt = torch.empty(rows, nb, 4, device="cuda"), torch.empty(rows, nb, dtype=torch.int32, device="cuda")
+    rc = lib.gkv_allocate(cu[0].data_ptr(), cu[1].data_ptr(), cu[2].data_ptr(), cu[3].data_ptr(), (C.c_float * 5)(*bits), cu[4].data_ptr(),
+                          1.0, ratio.data_ptr(), tgt.data_ptr(), rows, nb, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    for r in range(rows):
+        want, ref = oracle.allocate(mass[r], E[r], idx[r], hot[r], bits, budget[r])
+        assert np.array_equal(tgt[r].cpu().numpy(), want), (r, nb)
+        assert np.array_equal(ratio[r].cpu().numpy(), ref)
+
+
+def test_table_form_plans_as_the_array_form():
+    """The allocator's inputs derived from a ragged block table, against the same inputs spelled out."""
+    import ctypes as C
+    from geodesia_kv_b200 import _lib, policies
+    from geodesia_kv_b200.paged import PagedLayerCache, PagedPool
+    lib, D, group, B, Hkv = _lib.load(), 128, 32, 5, 2
+    lengths = [1, 64, 65, 640, 1999]
+    layer = PagedLayerCache(PagedPool(64 << 20, D, group), B, Hkv)
+    k = torch.randn(B, Hkv, max(lengths), D, device="cuda", dtype=torch.bfloat16)
+    layer.prefill(k, k, lengths)
+    mass = torch.rand(layer.rows, layer.nb + 3, device="cuda")                # wider than the table is used
+    stream = torch.cuda.current_stream().cuda_stream
+    for step in range(2):                                                     # the second time some blocks have moved
+        nb, rows = layer.nb, layer.rows
+        got = layer.plan_demotion(4.0, mass=mass)
+        level = layer.level[:, :nb].contiguous()
+        idx = ((level <= 8).int() + (level <= 4).int() + (level <= 2).int() + (level <= 1).int()).contiguous()
+        E = torch.empty(rows, nb, 5, device="cuda")
+        offs, m, hot = layer.offs[:, :nb].contiguous(), mass[:, :nb].contiguous(), layer.hot_blocks(nb)
+        assert lib.gkv_block_distortion(layer.pool.data.data_ptr(), offs.data_ptr(), level.data_ptr(), E.data_ptr(),
+                                        rows, nb, D, 64, group, 0.0, 0, rows, stream) == 0
+        nb_of = ((layer.lens + 63) // 64).int().contiguous()
+        target = nb_of.double() * (4.0 * 2.0 * 64 * D)
+        ratio, want = torch.empty(rows, nb, 4, device="cuda"), torch.empty(rows, nb, dtype=torch.int32, device="cuda")
+        bits = (C.c_float * 5)(*policies.ladder_bits(64, D, group))
+        assert lib.gkv_allocate_ragged(m.data_ptr(), E.data_ptr(), idx.data_ptr(), hot.data_ptr(), bits,
+                                       target.data_ptr(), 1.0, ratio.data_ptr(), want.data_ptr(), nb_of.data_ptr(), rows, nb, stream) == 0
+        assert torch.equal(got, want), step
+        assert step or layer.apply_demotion(got.cpu().numpy()) > 0
