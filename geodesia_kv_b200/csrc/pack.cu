@@ -310,6 +310,18 @@ __device__ __forceinline__ void scales_behind(const uint8_t* blk, int lv, int D,
     klo = base; kstep = klo + G * D; vlo = kstep + G * D; vstep = vlo + kP * gv;
 }
 
+// Block table of the pool's rows, brought up to date by the kernel that moves the blocks (block i of the launch is
+// entry flat[i] of the (rows, cap) tables), so that entering and demoting blocks needs no launch per table.  Null
+// `flat`: the caller keeps the table itself.
+struct TableRef {
+    const int64_t* flat;
+    int64_t* offs; int32_t* level; int32_t* valid;
+    float* mass; float* ek; float* ev;     // pack: cleared when given
+    int32_t* lens; const int32_t* row_len; // pack: lens[row] = row_len[i] when given ...
+    int len_add, per_row;                  // ... or lens[row] += len_add once per row of `per_row` consecutive blocks
+    int cap;
+};
+
 struct PagedPackParams {
     static constexpr bool kPacked = false, kMayRadii = true;
     const void* k; const void* v; int src_dtype;
@@ -317,6 +329,7 @@ struct PagedPackParams {
     uint8_t* pool; const int64_t* dst_off; const int32_t* level;
     float* ek; float* ev;
     int group, G, gv;
+    TableRef tab;
 };
 
 struct PagedDemoteParams {
@@ -324,8 +337,9 @@ struct PagedDemoteParams {
     const uint8_t* pool_old; uint8_t* pool_new;
     const int64_t* off_old; const int32_t* level_old;
     const int64_t* off_new; const int32_t* level_new;
-    float* ek; float* ev;
+    float* ek; float* ev;      // entry i, or with a table entry flat[i]
     int group, G, gv;
+    TableRef tab;
 };
 
 struct PagedUnpackParams {
@@ -495,6 +509,26 @@ __global__ void paged_append_kernel(AppendParams p) {
 }
 
 
+// Entries of rung-16 slots that rows are about to grow into (their tokens arrive by paged_append_kernel).
+__global__ void open_blocks_kernel(const int64_t* flat, const int64_t* offs, int n, int64_t* tab_offs, int32_t* tab_level,
+                                   float* tab_mass, float* tab_ek, float* tab_ev) {
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    const int64_t f = flat[i];
+    tab_offs[f] = offs[i];
+    tab_level[f] = 16;
+    tab_mass[f] = 0.f; tab_ek[f] = 0.f; tab_ev[f] = 0.f;
+}
+
+// A block table as it is before the first block enters.
+__global__ void clear_table_kernel(int64_t* offs, int32_t* level, int32_t* valid, float* mass, int32_t* lens, size_t n, int rows) {
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (size_t i = first; i < n; i += step) { offs[i] = -1; level[i] = 0; valid[i] = 0; mass[i] = 0.f; }
+    for (size_t i = first; i < (size_t)rows; i += step) lens[i] = 0;
+}
+
+
 // ---- persistent, bulk-copy-fed kernels ---------------------------------------------------------------
 // The kernels above start a CTA per block: the CTA reads the block's table entries, then its bytes, then
 // computes, then stores — a chain of dependent memory round trips that two resident CTAs per SM cannot
@@ -635,11 +669,35 @@ __device__ void describe(const PagedDemoteParams& p, int i, Desc& d) {
     d.src_kind = 3; d.old_level = lo; d.old_blk = p.pool_old + oo;
     scales_behind(d.old_blk, lo, D, p.G, p.gv, d.oklo, d.okstep, d.ovlo, d.ovstep);
     d.dst = p.pool_new + on; d.level = ln;
-    d.ek = p.ek ? p.ek + i : nullptr; d.ev = p.ev ? p.ev + i : nullptr;
+    const int64_t at = p.tab.flat ? p.tab.flat[i] : (int64_t)i;
+    d.ek = p.ek ? p.ek + at : nullptr; d.ev = p.ev ? p.ev + at : nullptr;
     const __half *a, *b, *c, *e;
     scales_behind(d.dst, ln, D, p.G, p.gv, a, b, c, e);
     d.klo = const_cast<__half*>(a); d.kstep = const_cast<__half*>(b);
     d.vlo = const_cast<__half*>(c); d.vstep = const_cast<__half*>(e);
+}
+
+// Block i's entries of the table, by one thread.
+template <class P>
+__device__ __forceinline__ void commit(const P&, int) {}
+template <>
+__device__ __forceinline__ void commit(const PagedPackParams& p, int i) {
+    if (!p.tab.flat) return;
+    const int64_t f = p.tab.flat[i];
+    p.tab.offs[f] = p.dst_off[i];
+    p.tab.level[f] = p.level[i];
+    p.tab.valid[f] = p.nvalid ? p.nvalid[i] : kP;
+    if (p.tab.mass) { p.tab.mass[f] = 0.f; p.tab.ek[f] = 0.f; p.tab.ev[f] = 0.f; }
+    const int row = (int)(f / p.tab.cap);
+    if (p.tab.row_len) p.tab.lens[row] = p.tab.row_len[i];             // the same value from every block of the row
+    else if (p.tab.per_row > 0 && i % p.tab.per_row == 0) p.tab.lens[row] += p.tab.len_add;
+}
+template <>
+__device__ __forceinline__ void commit(const PagedDemoteParams& p, int i) {
+    if (!p.tab.flat) return;
+    const int64_t f = p.tab.flat[i];
+    p.tab.offs[f] = p.off_new[i];
+    p.tab.level[f] = p.level_new[i];
 }
 
 // The producer lane: look block i up and start its copies into a stage; a source the copy engine cannot take
@@ -777,6 +835,7 @@ __global__ void __launch_bounds__(kStagedThreads, 2) staged_kernel(P p, int n, i
             src.vlo = src.kstep + G * D; src.vstep = src.vlo + kP * gv;
             rq::requantise_staged<D, P::kPacked, P::kMayRadii>(src, j, sm.work);
         }
+        if (tid == 128) commit(p, (int)blockIdx.x + it * (int)gridDim.x);
         rq::work_sync();                               // every worker is done with the stage and the work area
         if (tid == 0) bar_arrive(&sm.empty[s]);
     }
@@ -788,6 +847,7 @@ __global__ void __launch_bounds__(rq::kThreads, 2) direct_kernel(P p, int group)
     __shared__ rq::Shared sm;
     Desc d;
     describe<D>(p, (int)blockIdx.x, d);
+    if (threadIdx.x == 0) commit(p, (int)blockIdx.x);
     if (d.skip) return;
     rq::Job j;
     j.src_kind = d.src_kind; j.ksrc = d.ksrc; j.vsrc = d.vsrc; j.src_stride = d.src_stride; j.nvalid = d.nvalid;
@@ -928,6 +988,28 @@ int gkv_paged_pack_blocks(const void* k, const void* v, int src_dtype, const int
     p.k = k; p.v = v; p.src_dtype = src_dtype; p.src_off = src_off; p.token_stride = token_stride; p.nvalid = nvalid;
     p.pool = pool; p.dst_off = dst_off; p.level = level; p.ek = ek; p.ev = ev; p.group = group;
     p.G = kP / min(group, kP); p.gv = D / min(group, D);
+    p.tab = TableRef{};
+    return st::launch_d(p, n, D, group, src_dtype == 0, (cudaStream_t)stream);
+}
+
+int gkv_paged_enter_blocks(const void* k, const void* v, int src_dtype, const int64_t* src_off, int64_t token_stride,
+                           const int32_t* nvalid, uint8_t* pool, const int64_t* dst_off, const int32_t* level,
+                           const int64_t* flat, int64_t* tab_offs, int32_t* tab_level, int32_t* tab_valid,
+                           float* tab_mass, float* tab_ek, float* tab_ev, int32_t* lens, const int32_t* row_len,
+                           int len_add, int per_row, int cap, int n, int D, int block, int group, void* stream) {
+    using namespace gkv;
+    if (block != kP) return GKV_E_BLOCK;
+    if (n < 0 || cap <= 0 || !rq::shape_ok(D, group) || token_stride < D) return GKV_E_SHAPE;
+    if (src_dtype < 0 || src_dtype > 2 || per_row < 0) return GKV_E_ARG;
+    if ((tab_mass == nullptr) != (tab_ek == nullptr) || (tab_ek == nullptr) != (tab_ev == nullptr)) return GKV_E_ARG;
+    if (n == 0) return GKV_OK;
+    if (!k || !v || !src_off || !pool || !dst_off || !level || !flat || !tab_offs || !tab_level || !tab_valid) return GKV_E_NULL;
+    if ((row_len || per_row > 0) && !lens) return GKV_E_NULL;
+    PagedPackParams p;
+    p.k = k; p.v = v; p.src_dtype = src_dtype; p.src_off = src_off; p.token_stride = token_stride; p.nvalid = nvalid;
+    p.pool = pool; p.dst_off = dst_off; p.level = level; p.ek = nullptr; p.ev = nullptr; p.group = group;
+    p.G = kP / min(group, kP); p.gv = D / min(group, D);
+    p.tab = TableRef{flat, tab_offs, tab_level, tab_valid, tab_mass, tab_ek, tab_ev, lens, row_len, len_add, per_row, cap};
     return st::launch_d(p, n, D, group, src_dtype == 0, (cudaStream_t)stream);
 }
 
@@ -944,7 +1026,51 @@ int gkv_paged_demote_blocks(const uint8_t* pool_old, const int64_t* off_old, con
     p.pool_old = pool_old; p.pool_new = pool_new; p.off_old = off_old; p.level_old = level_old;
     p.off_new = off_new; p.level_new = level_new; p.ek = ek; p.ev = ev; p.group = group;
     p.G = kP / min(group, kP); p.gv = D / min(group, D);
+    p.tab = TableRef{};
     return st::launch_d(p, n, D, group, false, (cudaStream_t)stream);
+}
+
+int gkv_paged_demote_entries(uint8_t* pool, const int64_t* off_old, const int32_t* level_old, const int64_t* off_new,
+                             const int32_t* level_new, const int64_t* flat, int64_t* tab_offs, int32_t* tab_level,
+                             float* tab_ek, float* tab_ev, int n, int D, int block, int group, void* stream) {
+    using namespace gkv;
+    if (block != kP) return GKV_E_BLOCK;
+    if (n < 0 || !rq::shape_ok(D, group)) return GKV_E_SHAPE;
+    if (n == 0) return GKV_OK;
+    if (!pool || !off_old || !level_old || !off_new || !level_new || !flat || !tab_offs || !tab_level || !tab_ek || !tab_ev)
+        return GKV_E_NULL;
+    PagedDemoteParams p;
+    p.pool_old = pool; p.pool_new = pool; p.off_old = off_old; p.level_old = level_old;
+    p.off_new = off_new; p.level_new = level_new; p.ek = tab_ek; p.ev = tab_ev; p.group = group;
+    p.G = kP / min(group, kP); p.gv = D / min(group, D);
+    p.tab = TableRef{};
+    p.tab.flat = flat; p.tab.offs = tab_offs; p.tab.level = tab_level;
+    return st::launch_d(p, n, D, group, false, (cudaStream_t)stream);
+}
+
+int gkv_paged_open_blocks(const int64_t* flat, const int64_t* offs, int n, int64_t* tab_offs, int32_t* tab_level,
+                          float* tab_mass, float* tab_ek, float* tab_ev, void* stream) {
+    using namespace gkv;
+    if (n < 0) return GKV_E_SHAPE;
+    if (n == 0) return GKV_OK;
+    if (!flat || !offs || !tab_offs || !tab_level || !tab_mass || !tab_ek || !tab_ev) return GKV_E_NULL;
+    open_blocks_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(flat, offs, n, tab_offs, tab_level, tab_mass, tab_ek, tab_ev);
+    GKV_LAUNCH_CHECK();
+    return GKV_OK;
+}
+
+int gkv_paged_clear_table(int64_t* offs, int32_t* level, int32_t* valid, float* mass, int32_t* lens, int rows, int cap,
+                          void* stream) {
+    using namespace gkv;
+    if (rows < 0 || cap < 0) return GKV_E_SHAPE;
+    if (rows == 0) return GKV_OK;
+    if (!lens || (cap > 0 && (!offs || !level || !valid || !mass))) return GKV_E_NULL;
+    const size_t n = (size_t)rows * cap > (size_t)rows ? (size_t)rows * cap : (size_t)rows;
+    const size_t want = (n + 255) / 256;
+    clear_table_kernel<<<(unsigned)(want < 4096 ? want : 4096), 256, 0, (cudaStream_t)stream>>>(offs, level, valid, mass, lens,
+                                                                                               (size_t)rows * cap, rows);
+    GKV_LAUNCH_CHECK();
+    return GKV_OK;
 }
 
 int gkv_paged_unpack_blocks(const uint8_t* pool, const int64_t* offs, const int32_t* level, float* k_out,

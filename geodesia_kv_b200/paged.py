@@ -192,12 +192,19 @@ class PagedLayerCache:
     def _row_blocks(self) -> np.ndarray:
         return np.repeat(self.blocks_per_seq(), self.Hkv)
 
-    def _put(self, table: torch.Tensor, flat_idx: np.ndarray, values: np.ndarray) -> None:
-        if flat_idx.size == 0:
-            return
-        idx = torch.from_numpy(flat_idx.astype(np.int64)).to(self.device, non_blocking=True)
-        val = torch.from_numpy(np.ascontiguousarray(values)).to(self.device, non_blocking=True).to(table.dtype)
-        table.view(-1).index_put_((idx,), val)
+    def _upload(self, *arrays: np.ndarray):
+        """Host arrays -> (device buffer, their addresses in it), all in ONE copy, each 8-byte aligned.  The caller
+        holds the buffer until its kernel is launched; after that the stream order of the allocator protects it."""
+        starts, end = [], 0
+        for a in arrays:
+            starts.append(end)
+            end += (a.nbytes + 7) // 8 * 8
+        buf = np.empty(end, dtype=np.uint8)
+        for a, at in zip(arrays, starts):
+            buf[at:at + a.nbytes] = np.ascontiguousarray(a).view(np.uint8)
+        staged = torch.from_numpy(buf).to(self.device, non_blocking=True)
+        base = staged.data_ptr()
+        return staged, [base + at for at in starts]
 
     # -- growth ---------------------------------------------------------------------------------
     def prefill(self, k: torch.Tensor, v: torch.Tensor, lengths: Sequence[int] | None = None) -> None:
@@ -225,12 +232,27 @@ class PagedLayerCache:
         self.offs_h[row_of, blk_of] = slots
         self.level_h[row_of, blk_of] = 16
         self.len_h[:] = lengths
-        flat = row_of * self.cap + blk_of
-        self._put(self.offs, flat, slots)
-        self._put(self.valid, flat, nvalid)
-        self._put(self.level, flat, np.full(total, 16, dtype=np.int32))
-        self.lens.copy_(torch.from_numpy(np.repeat(lengths, Hkv).astype(np.int32)), non_blocking=True)
-        self.pack_blocks(k, v, src_off, D, nvalid, slots, np.full(total, 16, dtype=np.int32))
+        self._enter(k, v, src_off, nvalid, slots, row_of * self.cap + blk_of, fresh=False,
+                    row_len=lengths[rows_b[row_of]].astype(np.int32))
+
+    def _enter(self, k, v, src_off, nvalid, slots, flat, fresh: bool, row_len=None, len_add: int = 0, per_row: int = 0) -> None:
+        """Pack blocks into rung-16 slots and enter them into the table: one upload, one kernel.  ``fresh``
+        clears the entries' mass and radii; the row lengths are set from ``row_len`` (per block) or advanced
+        by ``len_add`` (rows of ``per_row`` consecutive blocks)."""
+        n, dev = int(flat.size), self.device
+        arrays = [src_off.astype(np.int64, copy=False), slots, flat.astype(np.int64, copy=False),
+                  np.ascontiguousarray(nvalid, dtype=np.int32), np.full(n, 16, dtype=np.int32)]
+        if row_len is not None:
+            arrays.append(row_len)
+        with torch.cuda.device(dev):
+            staged, (src, dst, at, nv, lv, *rl) = self._upload(*arrays)
+            rc = self.lib.gkv_paged_enter_blocks(k.data_ptr(), v.data_ptr(), _DT[k.dtype], src, int(self.D), nv,
+                                                 self.pool.data.data_ptr(), dst, lv, at, self.offs.data_ptr(),
+                                                 self.level.data_ptr(), self.valid.data_ptr(),
+                                                 self.mass.data_ptr() if fresh else None, self.ek.data_ptr() if fresh else None,
+                                                 self.ev.data_ptr() if fresh else None, self.lens.data_ptr(), rl[0] if rl else None,
+                                                 len_add, per_row, self.cap, n, self.D, BLOCK, self.group, _stream(dev))
+        _lib.check(rc, "gkv_paged_enter_blocks")
 
     def extend(self, k: torch.Tensor, v: torch.Tensor) -> None:
         """Append whole blocks to EVERY sequence: k, v (B, Hkv, n*64, D) dense; all sequences must
@@ -251,16 +273,9 @@ class PagedLayerCache:
         slots[fresh] = self.pool.alloc(16, fresh.size)
         self.offs_h[row_of, blk_of] = slots
         self.level_h[row_of, blk_of] = 16
-        flat = row_of * self.cap + blk_of
-        self._put(self.offs, flat, slots)
-        self._put(self.level, flat, np.full(flat.size, 16, dtype=np.int32))
-        self._put(self.valid, flat, np.full(flat.size, BLOCK, dtype=np.int32))
-        for t in (self.mass, self.ek, self.ev):
-            self._put(t, flat, np.zeros(flat.size, dtype=np.float32))
         self.len_h += T
-        self.lens += T
-        self.pack_blocks(k, v, (row_of * T + blk_in * BLOCK) * D, D, np.full(flat.size, BLOCK, np.int32), slots,
-                         np.full(flat.size, 16, dtype=np.int32))
+        self._enter(k, v, (row_of * T + blk_in * BLOCK) * D, np.full(slots.size, BLOCK, np.int32), slots,
+                    row_of * self.cap + blk_of, fresh=True, len_add=T, per_row=n)
 
     def pack_blocks(self, k, v, src_off, token_stride, nvalid, slots, levels, radii: bool = False):
         """Quantise blocks from dense rows into given slots (element offsets into k and v)."""
@@ -304,11 +319,12 @@ class PagedLayerCache:
         slots = self.pool.alloc(16, rows.size)
         self.offs_h[rows, blks] = slots
         self.level_h[rows, blks] = 16
-        flat = rows * self.cap + blks
-        self._put(self.offs, flat, slots)
-        self._put(self.level, flat, np.full(rows.size, 16, dtype=np.int32))
-        for t in (self.mass, self.ek, self.ev):
-            self._put(t, flat, np.zeros(rows.size, dtype=np.float32))
+        flat, dev = rows * self.cap + blks, self.device
+        with torch.cuda.device(dev):
+            staged, (at, so) = self._upload(flat.astype(np.int64, copy=False), slots)
+            rc = self.lib.gkv_paged_open_blocks(at, so, int(flat.size), self.offs.data_ptr(), self.level.data_ptr(),
+                                                self.mass.data_ptr(), self.ek.data_ptr(), self.ev.data_ptr(), _stream(dev))
+        _lib.check(rc, "gkv_paged_open_blocks")
 
     def sync_lengths(self) -> None:
         """Re-read the row lengths from the device (after append_device calls the host did not count)."""
@@ -414,21 +430,12 @@ class PagedLayerCache:
             if sel.size:
                 off_new[sel] = self.pool.alloc(rung, sel.size)
         dev = self.device
-        up = lambda a, dt: torch.from_numpy(np.ascontiguousarray(a)).to(dev, non_blocking=True).to(dt)
-        oo, lo, on, ln = up(off_old, torch.int64), up(lv_old, torch.int32), up(off_new, torch.int64), up(lv_new, torch.int32)
-        ek = torch.zeros(n, dtype=torch.float32, device=dev)
-        ev = torch.zeros(n, dtype=torch.float32, device=dev)
-        pool = self.pool.data
         with torch.cuda.device(dev):
-            rc = self.lib.gkv_paged_demote_blocks(pool.data_ptr(), oo.data_ptr(), lo.data_ptr(), pool.data_ptr(),
-                                                  on.data_ptr(), ln.data_ptr(), ek.data_ptr(), ev.data_ptr(), n, self.D,
-                                                  BLOCK, self.group, _stream(dev))
-        _lib.check(rc, "gkv_paged_demote_blocks")
-        flat = torch.from_numpy((r * self.cap + b).astype(np.int64)).to(dev, non_blocking=True)
-        self.offs.view(-1).index_put_((flat,), on)
-        self.level.view(-1).index_put_((flat,), ln)
-        self.ek.view(-1).index_put_((flat,), ek, accumulate=True)
-        self.ev.view(-1).index_put_((flat,), ev, accumulate=True)
+            staged, (old, new, at, lo, ln) = self._upload(off_old, off_new, r * self.cap + b, lv_old, lv_new)
+            rc = self.lib.gkv_paged_demote_entries(self.pool.data.data_ptr(), old, lo, new, ln, at, self.offs.data_ptr(),
+                                                   self.level.data_ptr(), self.ek.data_ptr(), self.ev.data_ptr(), n, self.D,
+                                                   BLOCK, self.group, _stream(dev))
+        _lib.check(rc, "gkv_paged_demote_entries")
         self.offs_h[r, b] = off_new
         self.level_h[r, b] = lv_new
         # the old slots are free for whatever is launched after the demotion kernel on this stream
@@ -467,11 +474,11 @@ class PagedLayerCache:
         self.offs_h[:] = -1
         self.level_h[:] = 0
         self.len_h[:] = 0
-        self.offs.fill_(-1)
-        self.level.fill_(0)
-        self.valid.zero_()
-        self.mass.zero_()
-        self.lens.zero_()
+        dev = self.device
+        with torch.cuda.device(dev):
+            rc = self.lib.gkv_paged_clear_table(self.offs.data_ptr(), self.level.data_ptr(), self.valid.data_ptr(),
+                                                self.mass.data_ptr(), self.lens.data_ptr(), self.rows, self.cap, _stream(dev))
+        _lib.check(rc, "gkv_paged_clear_table")
 
     def dequantise(self):
         """Exact fp32 K, V (rows, nb*64, D) of the cached tokens (tests, debugging); padding is zero."""

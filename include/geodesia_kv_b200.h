@@ -295,6 +295,33 @@ int gkv_paged_demote_blocks(const uint8_t *pool_old, const int64_t *off_old, con
                             uint8_t *pool_new, const int64_t *off_new, const int32_t *level_new,
                             float *ek, float *ev, int n, int D, int block, int group, void *stream);
 
+/* The same two operations on blocks that belong to a block table of (rows, cap) entries, which the
+ * launch brings up to date itself: block i is entry flat[i] = row * cap + block of the tables.
+ *
+ * enter_blocks: as pack_blocks, then offs, level and valid of the entry become dst_off[i], level[i] and
+ * nvalid[i]; mass, ek, ev (all or none) are cleared; lens[row] becomes row_len[i] (NULL: left alone), or,
+ * with per_row > 0 and row_len NULL, grows by len_add once per row (rows of per_row consecutive i).
+ * demote_entries: as demote_blocks within one pool, then offs and level become off_new[i], level_new[i];
+ * the radii are added to ek[flat[i]], ev[flat[i]].  Entries must be distinct.                      */
+int gkv_paged_enter_blocks(const void *k, const void *v, int src_dtype, const int64_t *src_off,
+                           int64_t token_stride, const int32_t *nvalid, uint8_t *pool,
+                           const int64_t *dst_off, const int32_t *level, const int64_t *flat,
+                           int64_t *tab_offs, int32_t *tab_level, int32_t *tab_valid, float *tab_mass,
+                           float *tab_ek, float *tab_ev, int32_t *lens, const int32_t *row_len, int len_add,
+                           int per_row, int cap, int n, int D, int block, int group, void *stream);
+int gkv_paged_demote_entries(uint8_t *pool, const int64_t *off_old, const int32_t *level_old,
+                             const int64_t *off_new, const int32_t *level_new, const int64_t *flat,
+                             int64_t *tab_offs, int32_t *tab_level, float *tab_ek, float *tab_ev, int n,
+                             int D, int block, int group, void *stream);
+
+/* n entries get empty rung-16 slots (offs[i]); their mass and radii are cleared. */
+int gkv_paged_open_blocks(const int64_t *flat, const int64_t *offs, int n, int64_t *tab_offs,
+                          int32_t *tab_level, float *tab_mass, float *tab_ek, float *tab_ev, void *stream);
+
+/* A table without blocks: offs -1, level, valid, mass and the row lengths 0. */
+int gkv_paged_clear_table(int64_t *offs, int32_t *level, int32_t *valid, float *mass, int32_t *lens,
+                          int rows, int cap, void *stream);
+
 /* Distortion table and rung allocation (gkv_block_distortion, gkv_allocate_ragged) straight from a block
  * table: the ladder index follows from level, the blocks in use and what must stay exact (the first
  * sink_blocks, the open block, its predecessor, the last window_blocks; policies.py:677-681) from lens, the
