@@ -40,6 +40,8 @@ SIGNATURES = {
                                        [C.POINTER(_vp), _i, _i, _vp, _vp, _vp]),
     "gkv_combine_partials": (_i, [_vp, _vp, _i, _i, _i, _vp]),
     "gkv_pack_blocks": (_i, [_vp, _vp, _i, _vp, _vp] + [_vp] * 4 + [_vp, _vp] + [_i] * 7 + [_i64, _i, _vp]),
+    "gkv_layout_rows": (_i, [_vp] * 4 + [_i64] + [_i] * 4 + [_vp]),
+    "gkv_pack_rows": (_i, [_vp, _vp, _i, _i64, _vp, _vp] + [_vp] * 4 + [_vp] * 3 + [_i] * 5 + [_i64, _vp]),
     "gkv_demote_blocks": (_i, [_vp] * 6 + [_vp] * 4 + [_i] * 5 + [_i64, _i64, _i, _vp]),
     "gkv_unpack_blocks": (_i, [_vp] * 7 + [_vp, _vp] + [_i] * 5 + [_i64, _i, _vp]),
     "gkv_maintenance_status": (_i, [C.POINTER(_i)]),

@@ -186,6 +186,7 @@ struct PackParams {
     int nb, b_lo, D, group, G, gv, per_row_meta;
     int64_t stride_bh;
     int nbx;                // blocks per row handled by this launch (b_hi - b_lo)
+    int64_t T;              // token rows between the cache rows of k and v (nb * 64, or fewer: `valid` then ends the last block)
 };
 
 __device__ __forceinline__ float load_src(const void* p, int dtype, size_t i) {
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_blocks_kernel(PackParams p)
     if (!level_ok(lv)) return;
     int nvalid = p.valid ? p.valid[(size_t)mrow * p.nb + blk] : kP;
     nvalid = max(1, min(nvalid, kP));
-    const size_t src0 = ((size_t)row * p.nb + blk) * kP * D;
+    const size_t src0 = ((size_t)row * p.T + (size_t)blk * kP) * D;
     const bool vec16 = p.src_dtype != 0 && ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0;
     if (vec16) {
         // eight 16-bit elements per load (D % 8 == 0, so a load never straddles a row)
@@ -611,7 +612,7 @@ __device__ void describe(const PackParams& p, int i, Desc& d) {
     const size_t mi = (size_t)mrow * p.nb + blk;
     const int lv = p.level[mi];
     if (!level_ok(lv)) { d.skip = 1; return; }
-    const size_t src0 = ((size_t)row * p.nb + blk) * kP * D, esz = p.src_dtype == 0 ? 4 : 2;
+    const size_t src0 = ((size_t)row * p.T + (size_t)blk * kP) * D, esz = p.src_dtype == 0 ? 4 : 2;
     d.src_kind = p.src_dtype; d.src_stride = D;
     d.nvalid = max(1, min(p.valid ? p.valid[mi] : kP, kP));
     d.ksrc = static_cast<const uint8_t*>(p.k) + src0 * esz;
@@ -888,14 +889,65 @@ static int set_smem(const void* fn, size_t bytes) {
     return GKV_OK;
 }
 
+// ---- where the blocks of packed rows go ----------------------------------------------------------------
+// One CTA per cache row: an exclusive scan of the block sizes (a running offset over chunks of one block per
+// thread), and the valid counts of a row of T tokens.
+__global__ void __launch_bounds__(1024) layout_rows_kernel(const int32_t* __restrict__ level, int64_t* __restrict__ offs,
+                                                           int32_t* __restrict__ valid, int64_t* __restrict__ row_bytes,
+                                                           int64_t T, int nb, int D) {
+    __shared__ int sums[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+    const size_t row0 = (size_t)blockIdx.x * nb;
+    int64_t run = 0;
+    for (int b0 = 0; b0 < nb; b0 += blockDim.x) {
+        const int b = b0 + tid;
+        int size = 0;
+        if (b < nb) {
+            const int lv = level[row0 + b];
+            size = level_ok(lv) ? 2 * half_bytes(lv, D) : 0;
+        }
+        int incl = size;                                // at most 1024 blocks of 64 KB: fits 32 bits
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) sums[warp] = incl;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < nwarp; ++w) { const int x = sums[w]; before += w < warp ? x : 0; all += x; }
+        if (b < nb) {
+            offs[row0 + b] = run + before + incl - size;
+            const int64_t left = T - (int64_t)b * kP;
+            valid[row0 + b] = left < kP ? (int)left : kP;
+        }
+        run += all;
+        __syncthreads();
+    }
+    if (tid == 0) row_bytes[blockIdx.x] = run;
+}
+
+// Rows are as wide as the longest: what lies behind a row's last block reads as zeros.
+__global__ void zero_tails_kernel(uint8_t* data, const int64_t* row_bytes, int64_t stride, int rows) {
+    for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+        uint8_t* d = data + (size_t)row * stride;
+        const int64_t lo = row_bytes[row], mid = (lo + 15) & ~(int64_t)15;
+        if (((reinterpret_cast<uintptr_t>(d) | (uintptr_t)stride) & 15) == 0) {
+            for (int64_t i = lo + threadIdx.x; i < mid && i < stride; i += blockDim.x) d[i] = 0;
+            for (int64_t i = mid + 16 * (int64_t)threadIdx.x; i < stride; i += 16 * (int64_t)blockDim.x)
+                *reinterpret_cast<uint4*>(d + i) = make_uint4(0, 0, 0, 0);
+        } else {
+            for (int64_t i = lo + threadIdx.x; i < stride; i += blockDim.x) d[i] = 0;
+        }
+    }
+}
+
 }  // namespace gkv
 
-extern "C" {
-
-int gkv_pack_blocks(const void* k, const void* v, int src_dtype, uint8_t* data, const int64_t* offs,
-                    void* klo, void* kstep, void* vlo, void* vstep, const int32_t* level,
-                    const int32_t* valid, int rows, int nb, int b_lo, int b_hi, int D, int block,
-                    int group, int64_t stride_bh, int meta_rows, void* stream) {
+static int pack_impl(const void* k, const void* v, int src_dtype, int64_t T, uint8_t* data, const int64_t* offs,
+                     void* klo, void* kstep, void* vlo, void* vstep, const int32_t* level,
+                     const int32_t* valid, int rows, int nb, int b_lo, int b_hi, int D, int block,
+                     int group, int64_t stride_bh, int meta_rows, void* stream) {
     using namespace gkv;
     if (block != kP) return GKV_E_BLOCK;
     if (rows <= 0 || nb <= 0 || D <= 0 || D > kMaxD || D % 8 || group <= 0) return GKV_E_SHAPE;
@@ -910,11 +962,47 @@ int gkv_pack_blocks(const void* k, const void* v, int src_dtype, uint8_t* data, 
     p.level = level; p.valid = valid; p.nb = nb; p.b_lo = b_lo; p.D = D; p.group = group;
     p.G = (kP + group - 1) / group; p.gv = (D + group - 1) / group; p.per_row_meta = meta_rows != 1;
     p.stride_bh = stride_bh;
-    p.nbx = b_hi - b_lo;
+    p.nbx = b_hi - b_lo; p.T = T;
     if (rq::shape_ok(D, group)) return st::launch_d(p, rows * (b_hi - b_lo), D, group, src_dtype == 0, (cudaStream_t)stream);
     int rc = set_smem((const void*)pack_blocks_kernel, tile_smem(kMaxD));
     if (rc) return rc;
     pack_blocks_kernel<<<dim3(b_hi - b_lo, rows), kPackThreads, tile_smem(D), (cudaStream_t)stream>>>(p);
+    GKV_LAUNCH_CHECK();
+    return GKV_OK;
+}
+
+extern "C" {
+
+int gkv_pack_blocks(const void* k, const void* v, int src_dtype, uint8_t* data, const int64_t* offs,
+                    void* klo, void* kstep, void* vlo, void* vstep, const int32_t* level,
+                    const int32_t* valid, int rows, int nb, int b_lo, int b_hi, int D, int block,
+                    int group, int64_t stride_bh, int meta_rows, void* stream) {
+    return pack_impl(k, v, src_dtype, (int64_t)nb * gkv::kP, data, offs, klo, kstep, vlo, vstep, level, valid, rows, nb, b_lo,
+                     b_hi, D, block, group, stride_bh, meta_rows, stream);
+}
+
+int gkv_pack_rows(const void* k, const void* v, int src_dtype, int64_t T, uint8_t* data, const int64_t* offs, void* klo,
+                  void* kstep, void* vlo, void* vstep, const int32_t* level, const int32_t* valid,
+                  const int64_t* row_bytes, int rows, int nb, int D, int block, int group, int64_t stride_bh,
+                  void* stream) {
+    using namespace gkv;
+    if (T <= 0 || (T + kP - 1) / kP != nb || rows <= 0 || stride_bh < 0) return GKV_E_SHAPE;
+    if (!valid || !row_bytes || !data) return GKV_E_NULL;
+    zero_tails_kernel<<<rows < 65535 ? rows : 65535, 128, 0, (cudaStream_t)stream>>>(data, row_bytes, stride_bh, rows);
+    GKV_LAUNCH_CHECK();
+    return pack_impl(k, v, src_dtype, T, data, offs, klo, kstep, vlo, vstep, level, valid, rows, nb, 0, nb, D, block, group,
+                     stride_bh, rows, stream);
+}
+
+int gkv_layout_rows(const int32_t* level, int64_t* offs, int32_t* valid, int64_t* row_bytes, int64_t T, int rows, int nb,
+                    int D, int block, void* stream) {
+    using namespace gkv;
+    if (block != kP) return GKV_E_BLOCK;
+    if (rows <= 0 || nb <= 0 || D <= 0 || D > kMaxD || (T + kP - 1) / kP != nb) return GKV_E_SHAPE;
+    if (!level || !offs || !valid || !row_bytes) return GKV_E_NULL;
+    int threads = (nb + 31) & ~31;
+    threads = threads > 1024 ? 1024 : threads;
+    layout_rows_kernel<<<rows, threads, 0, (cudaStream_t)stream>>>(level, offs, valid, row_bytes, T, nb, D);
     GKV_LAUNCH_CHECK();
     return GKV_OK;
 }

@@ -114,32 +114,33 @@ def pack_cache(k: torch.Tensor, v: torch.Tensor, level: torch.Tensor, group: int
     B, Hkv, T, D = k.shape
     nb = (T + BLOCK - 1) // BLOCK
     level = level.to(device=k.device, dtype=torch.int32).expand(B, Hkv, nb).contiguous()
-    if valid is None:
-        valid = torch.full((B, Hkv, nb), BLOCK, dtype=torch.int32, device=k.device)
-        if T % BLOCK:
-            valid[..., -1] = T % BLOCK
-    valid = valid.to(device=k.device, dtype=torch.int32).expand(B, Hkv, nb).contiguous()
-    if T != nb * BLOCK:                       # the kernel indexes whole blocks
-        pad = nb * BLOCK - T
-        k = torch.nn.functional.pad(k, (0, 0, 0, pad))
-        v = torch.nn.functional.pad(v, (0, 0, 0, pad))
+    if valid is not None:
+        valid = valid.to(device=k.device, dtype=torch.int32).expand(B, Hkv, nb).contiguous()
+        if T != nb * BLOCK:                   # the caller's counts may reach into the padding: it has to exist
+            k, v = (torch.nn.functional.pad(t, (0, 0, 0, nb * BLOCK - T)) for t in (k, v))
+            T = nb * BLOCK
     dt = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[k.dtype]
     k, v = k.contiguous(), v.contiguous()
-    offs, row_bytes = layout_offsets(level, D)
-    stride = int(row_bytes.max().item()) if nb else 0
-    stride = (stride + 255) // 256 * 256
     G, gv = (BLOCK + group - 1) // group, (D + group - 1) // group
-    dev = k.device
-    data = torch.zeros(B, Hkv, stride, dtype=torch.uint8, device=dev)
+    dev, rows = k.device, B * Hkv
+    lib = _lib.load()
+    offs = torch.empty(B, Hkv, nb, dtype=torch.int64, device=dev)
+    counts = torch.empty(B, Hkv, nb, dtype=torch.int32, device=dev)
+    row_bytes = torch.empty(rows, dtype=torch.int64, device=dev)
     planes = [torch.empty(B, Hkv, nb, *s, dtype=torch.float16, device=dev)
               for s in ((G, D), (G, D), (BLOCK, gv), (BLOCK, gv))]
-    lib = _lib.load()
     with torch.cuda.device(dev):
-        rc = lib.gkv_pack_blocks(k.data_ptr(), v.data_ptr(), dt, data.data_ptr(), offs.data_ptr(),
-                                 *(p.data_ptr() for p in planes), level.data_ptr(), valid.data_ptr(),
-                                 B * Hkv, nb, 0, nb, D, BLOCK, group, stride, B * Hkv,
-                                 torch.cuda.current_stream(dev).cuda_stream)
-    _lib.check(rc, "gkv_pack_blocks")
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        rc = lib.gkv_layout_rows(level.data_ptr(), offs.data_ptr(), counts.data_ptr(), row_bytes.data_ptr(), T, rows, nb, D,
+                                 BLOCK, stream)
+        _lib.check(rc, "gkv_layout_rows")
+        valid = counts if valid is None else valid
+        stride = (int(row_bytes.cpu().max()) + 255) // 256 * 256          # the width of the allocation: the one read-back
+        data = torch.empty(B, Hkv, stride, dtype=torch.uint8, device=dev)
+        rc = lib.gkv_pack_rows(k.data_ptr(), v.data_ptr(), dt, T, data.data_ptr(), offs.data_ptr(),
+                               *(p.data_ptr() for p in planes), level.data_ptr(), valid.data_ptr(), row_bytes.data_ptr(),
+                               rows, nb, D, BLOCK, group, stride, stream)
+    _lib.check(rc, "gkv_pack_rows")
     return PackedCache(data, offs, *planes, level, valid, group, D)
 
 

@@ -234,6 +234,19 @@ int gkv_pack_blocks(const void *k, const void *v, int src_dtype, uint8_t *data, 
                     const int32_t *valid, int rows, int nb, int b_lo, int b_hi, int D, int block,
                     int group, int64_t stride_bh, int meta_rows, void *stream);
 
+/* Contiguous placement of rows of nb blocks at rungs level (rows, nb): offs (rows, nb), the bytes of every
+ * row (rows), and the valid counts of rows of T tokens (nb = ceil(T / 64)).                              */
+int gkv_layout_rows(const int32_t *level, int64_t *offs, int32_t *valid, int64_t *row_bytes, int64_t T,
+                    int rows, int nb, int D, int block, void *stream);
+
+/* gkv_pack_blocks for whole rows of T tokens, which need not fill their last block (k, v: (rows, T, D);
+ * valid says where a row's last block ends), laid out by gkv_layout_rows; bytes from row_bytes[r] to the
+ * row stride are set to zero.                                                                          */
+int gkv_pack_rows(const void *k, const void *v, int src_dtype, int64_t T, uint8_t *data, const int64_t *offs,
+                  void *klo, void *kstep, void *vlo, void *vstep, const int32_t *level, const int32_t *valid,
+                  const int64_t *row_bytes, int rows, int nb, int D, int block, int group, int64_t stride_bh,
+                  void *stream);
+
 /* Demotion without a dense copy: block b of a row is read at rung level_old[b]
  * from offs_old[b], re-quantised from its CURRENT reconstruction to level_new[b]
  * (the batched demotion of geodesia_kv/policies.py:869-908) and written at

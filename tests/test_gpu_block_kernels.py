@@ -78,6 +78,21 @@ def test_pack_awkward_values(oracle, D, group, dtype):
             assert np.array_equal(got, ref, equal_nan=True), (kind, key)
 
 
+@pytest.mark.parametrize("nb", [1, 63, 64, 65, 200])
+def test_layout_of_rows(nb):
+    from geodesia_kv_b200.pack_layout import layout_offsets, pack_cache
+    rng = np.random.default_rng(nb)
+    for T in (nb * 64, nb * 64 - 63):
+        level = torch.from_numpy(LADDER[rng.integers(0, 5, (2, 2, nb))]).cuda()
+        k = torch.randn(2, 2, T, 64, device="cuda", dtype=torch.bfloat16)
+        cache = pack_cache(k, k, level, 32)
+        offs, row_bytes = layout_offsets(level, 64)
+        assert torch.equal(cache.offs, offs) and cache.data.shape[-1] == -(-int(row_bytes.max()) // 256) * 256
+        assert cache.valid[..., -1].eq(64 - (nb * 64 - T)).all() and cache.valid[..., :-1].eq(64).all()
+        behind = torch.arange(cache.data.shape[-1], device="cuda") >= row_bytes[..., None]
+        assert not cache.data[behind].any()
+
+
 @pytest.mark.parametrize("D,group", [(128, 32), (128, 16), (128, 64), (64, 16), (64, 64), (96, 32)])
 @pytest.mark.parametrize("value_weight", [0.0, 0.5])
 def test_distortion_edges(oracle, D, group, value_weight):
