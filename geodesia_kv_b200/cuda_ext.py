@@ -31,6 +31,7 @@ from typing import Any, Optional
 import torch
 
 from . import _lib
+from ._cuda import on, stream as _stream
 
 _EXT: Any = None
 _TRIED = False
@@ -38,10 +39,6 @@ _TRIED = False
 
 def _ptr(t: Optional[torch.Tensor]) -> int:
     return 0 if t is None or t.numel() == 0 else t.data_ptr()
-
-
-def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
 
 
 class _Extension:
@@ -71,7 +68,7 @@ class _Extension:
             return 0
         import ctypes
         word = ctypes.c_int(0)
-        with torch.cuda.device(dev):
+        with on(dev):
             _lib.check(self.lib.gkv_decode_status(ws.data_ptr(), ctypes.byref(word), _stream(dev)), "gkv_decode_status")
         return int(word.value)
 
@@ -135,7 +132,7 @@ class _Extension:
         partials = partials.contiguous()
         parts, B, Hq, D2 = partials.shape
         out = torch.empty(B, Hq, D2 - 2, dtype=torch.float32, device=partials.device)
-        with torch.cuda.device(partials.device):
+        with on(partials.device):
             rc = self.lib.gkv_combine_partials(partials.data_ptr(), out.data_ptr(), parts, B * Hq, D2 - 2,
                                                _stream(partials.device))
         _lib.check(rc, "gkv_combine_partials")
@@ -171,7 +168,7 @@ class _Extension:
         q, data, offs, level, valid = (t.contiguous() for t in (q, data, offs, level, valid))
         klo, kstep, vlo, vstep = (t.contiguous() for t in (klo, kstep, vlo, vstep))
         if mass:
-            with torch.cuda.device(dev):
+            with on(dev):
                 need = self.lib.gkv_decode_mass_workspace_bytes(B, Hq, Hkv, D, nb, int(group))
                 ws = self._workspace(dev, need)
                 plan = self._plan(offs, level, valid, meta_rows, nb)
@@ -187,7 +184,7 @@ class _Extension:
                     out.zero_()
             _lib.check(rc, "gkv_mixed_attn_decode_mass")
             return out, bm
-        with torch.cuda.device(dev):
+        with on(dev):
             need = self.lib.gkv_decode_workspace_bytes(B, Hq, Hkv, D, nb)
             ws = self._workspace(dev, need)
             plan = self._plan(offs, level, valid, meta_rows, nb)

@@ -13,6 +13,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib
+from ._cuda import on, stream as _stream
 from .packed import pack_bits
 
 BLOCK = 64
@@ -129,8 +130,8 @@ def pack_cache(k: torch.Tensor, v: torch.Tensor, level: torch.Tensor, group: int
     row_bytes = torch.empty(rows, dtype=torch.int64, device=dev)
     planes = [torch.empty(B, Hkv, nb, *s, dtype=torch.float16, device=dev)
               for s in ((G, D), (G, D), (BLOCK, gv), (BLOCK, gv))]
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with on(dev):
+        stream = _stream(dev)
         rc = lib.gkv_layout_rows(level.data_ptr(), offs.data_ptr(), counts.data_ptr(), row_bytes.data_ptr(), T, rows, nb, D,
                                  BLOCK, stream)
         _lib.check(rc, "gkv_layout_rows")
@@ -151,10 +152,10 @@ def unpack_cache(c: PackedCache):
     k = torch.empty(B, Hkv, nb * BLOCK, c.D, dtype=torch.float32, device=dev)
     v = torch.empty_like(k)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with on(dev):
         rc = lib.gkv_unpack_blocks(c.data.data_ptr(), c.offs.data_ptr(), c.klo.data_ptr(), c.kstep.data_ptr(),
                                    c.vlo.data_ptr(), c.vstep.data_ptr(), c.level.data_ptr(), k.data_ptr(),
                                    v.data_ptr(), B * Hkv, nb, c.D, BLOCK, c.group, c.data.size(-1), B * Hkv,
-                                   torch.cuda.current_stream(dev).cuda_stream)
+                                   _stream(dev))
     _lib.check(rc, "gkv_unpack_blocks")
     return k, v

@@ -31,15 +31,12 @@ import numpy as np
 import torch
 
 from . import _lib
+from ._cuda import on, stream as _stream
 
 BLOCK = 64
 LADDER = (16, 8, 4, 2, 1)
 _LADDER_NP = np.array(LADDER, dtype=np.int32)
 _DT = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
-
-
-def _stream(dev):
-    return torch.cuda.current_stream(dev).cuda_stream
 
 
 def ladder_index_np(level: np.ndarray) -> np.ndarray:
@@ -106,18 +103,21 @@ class PagedPool:
             return np.empty(0, dtype=np.int64)
         size = self.slot[rung]
         per_slab = self.slab_bytes // size
-        while self._top[rung] < n:
-            if not self._free_slabs:
+        need = max(0, -(-(n - self._top[rung]) // per_slab))
+        if need:
+            took = [self._free_slabs.pop() for _ in range(min(need, len(self._free_slabs)))]
+            if took:
+                s = np.array(took, dtype=np.int64)
+                self._slab_rung[s] = rung
+                # pushed high to low, so low addresses are handed out first
+                self._push(rung, (s[:, None] * self.slab_bytes + np.arange(per_slab - 1, -1, -1, dtype=np.int64) * size).reshape(-1))
+            if len(took) < need:
                 raise PoolExhausted(f"pool of {self.capacity_bytes} bytes exhausted asking for {n} slots of rung {rung} "
                                     f"({self.bytes_in_use} bytes in use)")
-            s = self._free_slabs.pop()
-            self._slab_rung[s] = rung
-            # pushed high to low, so low addresses are handed out first
-            self._push(rung, s * self.slab_bytes + np.arange(per_slab - 1, -1, -1, dtype=np.int64) * size)
         top = self._top[rung]
         out = self._stack[rung][top - n:top][::-1].copy()
         self._top[rung] = top - n
-        np.add.at(self._slab_live, out // self.slab_bytes, 1)
+        self._slab_live += np.bincount(out // self.slab_bytes, minlength=self.n_slabs)
         self.bytes_in_use += n * size
         self.peak_bytes_in_use = max(self.peak_bytes_in_use, self.bytes_in_use)
         return out
@@ -130,19 +130,21 @@ class PagedPool:
         slabs = offs // self.slab_bytes
         if np.any(self._slab_rung[slabs] != rung):
             raise ValueError("a freed offset does not belong to a slab of that rung")
-        np.subtract.at(self._slab_live, slabs, 1)
+        gone = np.bincount(slabs, minlength=self.n_slabs)
+        self._slab_live -= gone
         self.bytes_in_use -= offs.size * self.slot[rung]
         self._push(rung, offs)
-        touched = np.unique(slabs)
-        empty = touched[self._slab_live[touched] == 0]
+        empty = np.nonzero((gone > 0) & (self._slab_live == 0))[0]
         if empty.size:
             top = self._top[rung]
             st = self._stack[rung][:top]
-            keep = st[~np.isin(st // self.slab_bytes, empty)]
+            idle = np.zeros(self.n_slabs, dtype=bool)
+            idle[empty] = True
+            keep = st[~idle[st // self.slab_bytes]]
             self._stack[rung][:keep.size] = keep
             self._top[rung] = keep.size
             self._slab_rung[empty] = 0
-            self._free_slabs.extend(int(s) for s in empty[::-1])
+            self._free_slabs.extend(empty[::-1].tolist())
 
 
 class PagedLayerCache:
@@ -244,7 +246,7 @@ class PagedLayerCache:
                   np.ascontiguousarray(nvalid, dtype=np.int32), np.full(n, 16, dtype=np.int32)]
         if row_len is not None:
             arrays.append(row_len)
-        with torch.cuda.device(dev):
+        with on(dev):
             staged, (src, dst, at, nv, lv, *rl) = self._upload(*arrays)
             rc = self.lib.gkv_paged_enter_blocks(k.data_ptr(), v.data_ptr(), _DT[k.dtype], src, int(self.D), nv,
                                                  self.pool.data.data_ptr(), dst, lv, at, self.offs.data_ptr(),
@@ -285,7 +287,7 @@ class PagedLayerCache:
         so, nv, sl, lv = up(src_off, torch.int64), up(nvalid, torch.int32), up(slots, torch.int64), up(levels, torch.int32)
         ek = torch.zeros(n, dtype=torch.float32, device=dev) if radii else None
         ev = torch.zeros(n, dtype=torch.float32, device=dev) if radii else None
-        with torch.cuda.device(dev):
+        with on(dev):
             rc = self.lib.gkv_paged_pack_blocks(k.data_ptr(), v.data_ptr(), _DT[k.dtype], so.data_ptr(), int(token_stride),
                                                 nv.data_ptr(), self.pool.data.data_ptr(), sl.data_ptr(), lv.data_ptr(),
                                                 ek.data_ptr() if radii else None, ev.data_ptr() if radii else None,
@@ -320,7 +322,7 @@ class PagedLayerCache:
         self.offs_h[rows, blks] = slots
         self.level_h[rows, blks] = 16
         flat, dev = rows * self.cap + blks, self.device
-        with torch.cuda.device(dev):
+        with on(dev):
             staged, (at, so) = self._upload(flat.astype(np.int64, copy=False), slots)
             rc = self.lib.gkv_paged_open_blocks(at, so, int(flat.size), self.offs.data_ptr(), self.level.data_ptr(),
                                                 self.mass.data_ptr(), self.ek.data_ptr(), self.ev.data_ptr(), _stream(dev))
@@ -337,7 +339,7 @@ class PagedLayerCache:
         if not (k_new.is_contiguous() and v_new.is_contiguous()):
             k_new, v_new = k_new.contiguous(), v_new.contiguous()
         dev = self.device
-        with torch.cuda.device(dev):
+        with on(dev):
             rc = self.lib.gkv_paged_append_token(k_new.data_ptr(), v_new.data_ptr(), _DT[k_new.dtype],
                                                  self.pool.data.data_ptr(), self.offs.data_ptr(), self.valid.data_ptr(),
                                                  self.lens.data_ptr(), self.status.data_ptr(), self.rows, self.cap,
@@ -359,7 +361,7 @@ class PagedLayerCache:
         if nb != self.cap:                                           # the kernel wants tables of width nb
             offs, level, valid = offs[:, :nb].contiguous(), level[:, :nb].contiguous(), valid[:, :nb].contiguous()
         lib = self.lib
-        with torch.cuda.device(dev):
+        with on(dev):
             need = (lib.gkv_decode_mass_workspace_bytes(B, Hq, self.Hkv, D, nb, self.group) if want_mass
                     else lib.gkv_decode_workspace_bytes(B, Hq, self.Hkv, D, nb))
             ws = ext._workspace(dev, need)
@@ -401,7 +403,7 @@ class PagedLayerCache:
         ratio = torch.empty(rows, nb, 4, dtype=torch.float32, device=dev) if nb > 512 else None     # longer rows keep them in memory
         tgt = torch.empty(rows, nb, dtype=torch.int32, device=dev)
         bits = (C.c_float * 5)(*ladder_bits(BLOCK, D, self.group))
-        with torch.cuda.device(dev):
+        with on(dev):
             rc = self.lib.gkv_paged_plan_demotion(self.pool.data.data_ptr(), self.offs.data_ptr(), self.level.data_ptr(),
                                                   self.lens.data_ptr(), m.data_ptr(), m.stride(0), bits,
                                                   float(budget_bits * 2.0 * BLOCK * D), max(1, (sinks + BLOCK - 1) // BLOCK),
@@ -430,7 +432,7 @@ class PagedLayerCache:
             if sel.size:
                 off_new[sel] = self.pool.alloc(rung, sel.size)
         dev = self.device
-        with torch.cuda.device(dev):
+        with on(dev):
             staged, (old, new, at, lo, ln) = self._upload(off_old, off_new, r * self.cap + b, lv_old, lv_new)
             rc = self.lib.gkv_paged_demote_entries(self.pool.data.data_ptr(), old, lo, new, ln, at, self.offs.data_ptr(),
                                                    self.level.data_ptr(), self.ek.data_ptr(), self.ev.data_ptr(), n, self.D,
@@ -475,7 +477,7 @@ class PagedLayerCache:
         self.level_h[:] = 0
         self.len_h[:] = 0
         dev = self.device
-        with torch.cuda.device(dev):
+        with on(dev):
             rc = self.lib.gkv_paged_clear_table(self.offs.data_ptr(), self.level.data_ptr(), self.valid.data_ptr(),
                                                 self.mass.data_ptr(), self.lens.data_ptr(), self.rows, self.cap, _stream(dev))
         _lib.check(rc, "gkv_paged_clear_table")
@@ -486,7 +488,7 @@ class PagedLayerCache:
         k = torch.zeros(self.rows, nb, BLOCK, self.D, dtype=torch.float32, device=dev)
         v = torch.zeros_like(k)
         offs, level = self.offs[:, :nb].contiguous(), self.level[:, :nb].contiguous()
-        with torch.cuda.device(dev):
+        with on(dev):
             rc = self.lib.gkv_paged_unpack_blocks(self.pool.data.data_ptr(), offs.data_ptr(), level.data_ptr(),
                                                   k.data_ptr(), v.data_ptr(), self.rows * nb, self.D, BLOCK, self.group,
                                                   _stream(dev))
