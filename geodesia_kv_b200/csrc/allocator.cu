@@ -39,9 +39,6 @@ struct AllocParams {
     double target_per_block;
 };
 
-template <bool SMALL> struct SumOf { using type = double; };
-template <> struct SumOf<true> { using type = int; };
-
 // What the allocator has to know about block b of a problem.
 struct BlockState { int idx; bool hot; };
 template <bool TABLE>
@@ -83,37 +80,158 @@ __device__ __forceinline__ int landing(const float (&r)[4], const BlockState& st
     return pref;
 }
 
-// Bound: latency — one CTA per row, and every candidate threshold is a sum over the row's blocks and a barrier.  So
-// several candidates are tried per round, the CTA has no more warps than the row has blocks, and rows of at most
-// 512 blocks (32k tokens) whose rungs cost whole numbers of bits (every ladder does) take SMALL: a block per
-// thread, its ratios in registers, and sums in integers, which one instruction adds up over a warp (seven candidates
-// per round: 11 rounds for fp32 keys).  Longer rows read the ratios back in every round and add doubles.
-template <bool SMALL, bool TABLE>
-__global__ void __launch_bounds__(kAllocThreads) allocate_kernel(const __grid_constant__ AllocParams p) {
-    constexpr int kCand = SMALL ? 7 : 3, kShift = SMALL ? 3 : 2;
-    using Sum = typename SumOf<SMALL>::type;
-    __shared__ Sum sums[2][kCand][kAllocThreads / 32];
+// The interval of keys [lo, hi] after N thresholds m (ascending) were tried: the first that fits and the last that
+// does not close it.
+template <int N>
+__device__ __forceinline__ void split_points(uint32_t lo, uint32_t hi, uint32_t (&m)[N]) {
+#pragma unroll
+    for (int c = 0; c < N; ++c) m[c] = lo + (uint32_t)(((unsigned long long)(hi - lo) * (unsigned)(c + 1)) / (unsigned)(N + 1));
+}
+template <int N>
+__device__ __forceinline__ void narrow(const uint32_t (&m)[N], const bool (&ok)[N], uint32_t& lo, uint32_t& hi) {
+#pragma unroll
+    for (int c = N - 1; c >= 0; --c)
+        if (ok[c]) hi = m[c];
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+        if (!ok[c]) lo = m[c] + 1;
+}
+__device__ __forceinline__ const float* mass_row(const AllocParams& p, int prob, bool table) {
+    return p.mass + (size_t)prob * (table ? p.mass_stride : (int64_t)p.nb);
+}
+template <bool TABLE>
+__device__ __forceinline__ float target_of(const AllocParams& p, int prob, int nb_row) {      // fp32 comparison, as torch does
+    return TABLE ? (float)((double)nb_row * p.target_per_block) : (float)p.target_bits[prob];
+}
+
+// Rows of at most 512 blocks (32k tokens) whose rungs cost whole numbers of bits (every ladder does): one block per
+// thread.  Bound: the length of one warp's instruction stream (a row is one CTA with no more warps than it has blocks,
+// and nothing else runs on its SM), so a candidate has to be cheap: a block's four ratios become ascending keys once
+// (the prefix rule: step s is taken below its own threshold and those before it), a candidate is four compares whose
+// votes are counted, and the bits follow from the counts.  64 rows of 128 blocks: 25 -> 8.6 us against seven candidates
+// per round with selected bits and a reduction each, 20 us with one candidate in doubles.
+template <bool TABLE>
+__global__ void __launch_bounds__(kAllocThreads) allocate_small_kernel(const __grid_constant__ AllocParams p) {
+    constexpr int kCand = 3;
+    __shared__ int sums[2][kCand][kAllocThreads / 32];
     __shared__ uint32_t su[2][kAllocThreads / 32];
-    const int prob = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+    __shared__ int s0[kAllocThreads / 32];
+    const int prob = blockIdx.x, b = threadIdx.x, lane = b & 31, warp = b >> 5, nwarp = blockDim.x >> 5;
     const int nb_all = p.nb, len = TABLE ? p.lens[prob] : 0;
     const int nb_row = TABLE ? (len + kP - 1) / kP : p.nb_of ? p.nb_of[prob] : nb_all;
     const int nb = max(0, min(nb_all, nb_row));
-    const float* mass = p.mass + (size_t)prob * (TABLE ? p.mass_stride : (int64_t)nb_all);
-    const float* E = p.E + (size_t)prob * nb_all * 5;
-    float* ratio = p.ratio ? p.ratio + (size_t)prob * nb_all * 4 : nullptr;
     int32_t* tgt = p.tgt + (size_t)prob * nb_all;
-    for (int b = nb + tid; b < nb_all; b += blockDim.x) tgt[b] = block_state<TABLE>(p, prob, b, len).idx;
-
-    uint32_t kmin = 0xffffffffu, kmax = 0u;
-    float mine[4] = {0.f, 0.f, 0.f, 0.f};
     BlockState my{4, true};
-    for (int b = tid; b < nb; b += blockDim.x) {
-        my = block_state<TABLE>(p, prob, b, len);
-        step_ratios(p, mass[b], E + b * 5, my, mine);
+    uint32_t kmin = 0xffffffffu, kmax = 0u, key[4] = {~0u, ~0u, ~0u, ~0u};
+    const int bits[5] = {(int)p.bits[0], (int)p.bits[1], (int)p.bits[2], (int)p.bits[3], (int)p.bits[4]};
+    int mine = 0;                               // bits of this thread's block where it stands
+    if (b < nb_all) my = block_state<TABLE>(p, prob, b, len);
+    if (b < nb) {
+        float r[4];
+        step_ratios(p, mass_row(p, prob, TABLE)[b], p.E + ((size_t)prob * nb_all + b) * 5, my, r);
+        float* ratio = p.ratio ? p.ratio + ((size_t)prob * nb_all + b) * 4 : nullptr;
+        uint32_t top = 0u;
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            if (ratio) ratio[b * 4 + s] = mine[s];
-            const uint32_t k = float_key(mine[s]);
+            if (ratio) ratio[s] = r[s];
+            const uint32_t k = float_key(r[s]);
+            kmin = min(kmin, k);
+            kmax = max(kmax, k);
+            // -0 and +0 are the same threshold; a ratio that is not a number is below none
+            top = max(top, r[s] == r[s] ? float_key(r[s] + 0.f) : ~0u);
+            key[s] = (my.idx == 0 && !my.hot) ? top : ~0u;
+        }
+        const int id = min(my.idx, 4);
+        mine = id == 0 ? bits[0] : id == 1 ? bits[1] : id == 2 ? bits[2] : id == 3 ? bits[3] : bits[4];
+    } else if (b < nb_all) {
+        tgt[b] = my.idx;
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (nwarp > 1) {
+        if (lane == 0) { su[0][warp] = kmin; su[1][warp] = kmax; s0[warp] = mine; }
+        __syncthreads();
+        kmin = __reduce_min_sync(0xffffffffu, lane < nwarp ? su[0][lane] : ~0u);
+        kmax = __reduce_max_sync(0xffffffffu, lane < nwarp ? su[1][lane] : 0u);
+        mine = __reduce_add_sync(0xffffffffu, lane < nwarp ? s0[lane] : 0);
+    }
+    if (nb == 0) return;
+
+    const float target = target_of<TABLE>(p, prob, nb_row);
+    const int gain[4] = {bits[0] - bits[1], bits[1] - bits[2], bits[2] - bits[3], bits[3] - bits[4]};
+    int par = 0;
+    auto fits = [&](const uint32_t (&m)[kCand], bool (&ok)[kCand]) {
+        int tot[kCand];
+#pragma unroll
+        for (int c = 0; c < kCand; ++c) {
+            // a threshold that is not a number takes no step (it compares with nothing)
+            const uint32_t at = key_float(m[c]) == key_float(m[c]) ? (m[c] == 0x7fffffffu ? 0x80000000u : m[c]) : 0u;
+            tot[c] = 0;
+#pragma unroll
+            for (int s = 0; s < 4; ++s) tot[c] += __popc(__ballot_sync(0xffffffffu, key[s] <= at && key[s] != ~0u)) * gain[s];
+        }
+        if (nwarp > 1) {
+            if (lane == 0)
+#pragma unroll
+                for (int c = 0; c < kCand; ++c) sums[par][c][warp] = tot[c];
+            __syncthreads();                    // two buffers in turn: one barrier per round is enough
+#pragma unroll
+            for (int c = 0; c < kCand; ++c) tot[c] = __reduce_add_sync(0xffffffffu, lane < nwarp ? sums[par][c][lane] : 0);
+            par ^= 1;
+        }
+#pragma unroll
+        for (int c = 0; c < kCand; ++c) ok[c] = !((float)(mine - tot[c]) > target);
+    };
+    uint32_t lo = kmin, hi = kmax, m[kCand] = {kmax, kmax, kmax};
+    bool ok[kCand];
+    fits(m, ok);
+    if (ok[0]) {
+        while (lo < hi) {
+            split_points(lo, hi, m);
+            fits(m, ok);
+            narrow(m, ok, lo, hi);
+        }
+    }
+    if (b < nb) {
+        const float lam = key_float(hi);
+        const uint32_t at = lam == lam ? (hi == 0x7fffffffu ? 0x80000000u : hi) : 0u;
+        int l = min(my.idx, 4);
+        if (my.idx == 0 && !my.hot) {
+            l = 0;
+#pragma unroll
+            for (int s = 0; s < 4; ++s) l += key[s] <= at && key[s] != ~0u;
+        }
+        tgt[b] = l;
+    }
+}
+
+// Longer rows: the ratios go to memory and are read back in every round, several blocks per thread, sums in doubles (in an
+// order that does not depend on the data).
+template <bool TABLE>
+__global__ void __launch_bounds__(kAllocThreads) allocate_kernel(const __grid_constant__ AllocParams p) {
+    constexpr int kCand = 3;
+    __shared__ double sums[2][kCand][kAllocThreads / 32];
+    __shared__ uint32_t su[2][kAllocThreads / 32];
+    const int prob = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int nwarp = kAllocThreads / 32;
+    const int nb_all = p.nb, len = TABLE ? p.lens[prob] : 0;
+    const int nb_row = TABLE ? (len + kP - 1) / kP : p.nb_of ? p.nb_of[prob] : nb_all;
+    const int nb = max(0, min(nb_all, nb_row));
+    const float* mass = mass_row(p, prob, TABLE);
+    const float* E = p.E + (size_t)prob * nb_all * 5;
+    float* ratio = p.ratio + (size_t)prob * nb_all * 4;
+    int32_t* tgt = p.tgt + (size_t)prob * nb_all;
+    for (int b = nb + tid; b < nb_all; b += kAllocThreads) tgt[b] = block_state<TABLE>(p, prob, b, len).idx;
+
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
+    for (int b = tid; b < nb; b += kAllocThreads) {
+        float r[4];
+        step_ratios(p, mass[b], E + b * 5, block_state<TABLE>(p, prob, b, len), r);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            ratio[b * 4 + s] = r[s];
+            const uint32_t k = float_key(r[s]);
             kmin = min(kmin, k);
             kmax = max(kmax, k);
         }
@@ -125,81 +243,50 @@ __global__ void __launch_bounds__(kAllocThreads) allocate_kernel(const __grid_co
     for (int w = 0; w < nwarp; ++w) { kmin = min(kmin, su[0][w]); kmax = max(kmax, su[1][w]); }
     if (nb == 0) return;
 
-    const float target = TABLE ? (float)((double)nb_row * p.target_per_block) : (float)p.target_bits[prob];   // fp32 comparison, as torch does
-    const Sum bits[5] = {(Sum)p.bits[0], (Sum)p.bits[1], (Sum)p.bits[2], (Sum)p.bits[3], (Sum)p.bits[4]};
+    const float target = target_of<TABLE>(p, prob, nb_row);
     auto land = [&](int b, float lam) -> int {
-        if constexpr (SMALL) {
-            return landing(mine, my, lam);
-        } else {
-            float r[4];
+        float r[4];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) r[s] = ratio[b * 4 + s];
-            return landing(r, block_state<TABLE>(p, prob, b, len), lam);
-        }
+        for (int s = 0; s < 4; ++s) r[s] = ratio[b * 4 + s];
+        return landing(r, block_state<TABLE>(p, prob, b, len), lam);
     };
     int par = 0;
-    auto fits = [&](const float (&lam)[kCand], bool (&ok)[kCand]) {
-        Sum tot[kCand];
-#pragma unroll
-        for (int c = 0; c < kCand; ++c) tot[c] = 0;
-        for (int b = tid; b < nb; b += blockDim.x) {
+    auto fits = [&](const uint32_t (&m)[kCand], bool (&ok)[kCand]) {
+        double tot[kCand] = {0.0, 0.0, 0.0};
+        for (int b = tid; b < nb; b += kAllocThreads)
 #pragma unroll
             for (int c = 0; c < kCand; ++c) {
-                const int l = land(b, lam[c]);
-                tot[c] += l == 0 ? bits[0] : l == 1 ? bits[1] : l == 2 ? bits[2] : l == 3 ? bits[3] : bits[4];
+                const int l = land(b, key_float(m[c]));
+                tot[c] += (double)(l == 0 ? p.bits[0] : l == 1 ? p.bits[1] : l == 2 ? p.bits[2] : l == 3 ? p.bits[3] : p.bits[4]);
             }
-        }
-        if constexpr (SMALL) {
 #pragma unroll
-            for (int c = 0; c < kCand; ++c) tot[c] = __reduce_add_sync(0xffffffffu, tot[c]);
-        } else {
+        for (int o = 16; o; o >>= 1)
 #pragma unroll
-            for (int o = 16; o; o >>= 1)
-#pragma unroll
-                for (int c = 0; c < kCand; ++c) tot[c] += __shfl_xor_sync(0xffffffffu, tot[c], o);
-        }
+            for (int c = 0; c < kCand; ++c) tot[c] += __shfl_xor_sync(0xffffffffu, tot[c], o);
         if (lane == 0)
 #pragma unroll
             for (int c = 0; c < kCand; ++c) sums[par][c][warp] = tot[c];
         __syncthreads();                       // two buffers in turn: one barrier per round is enough
 #pragma unroll
         for (int c = 0; c < kCand; ++c) {
-            Sum r = sums[par][c][0];
+            double r = sums[par][c][0];
             for (int w = 1; w < nwarp; ++w) r += sums[par][c][w];
             ok[c] = !((float)r > target);
         }
         par ^= 1;
     };
-
-    uint32_t lo = kmin, hi = kmax;
+    uint32_t lo = kmin, hi = kmax, m[kCand] = {kmax, kmax, kmax};
     bool ok[kCand];
-    float lam[kCand];
-#pragma unroll
-    for (int c = 0; c < kCand; ++c) lam[c] = key_float(kmax);
-    fits(lam, ok);
+    fits(m, ok);
     if (ok[0]) {
         while (lo < hi) {
-            uint32_t m[kCand];
-#pragma unroll
-            for (int c = 0; c < kCand; ++c) {
-                m[c] = lo + (uint32_t)(((unsigned long long)(hi - lo) * (unsigned)(c + 1)) >> kShift);
-                lam[c] = key_float(m[c]);
-            }
-            fits(lam, ok);
-            // the first candidate that fits and the last that does not close the interval
-            uint32_t nlo = lo, nhi = hi;
-#pragma unroll
-            for (int c = kCand - 1; c >= 0; --c)
-                if (ok[c]) nhi = m[c];
-#pragma unroll
-            for (int c = 0; c < kCand; ++c)
-                if (!ok[c]) nlo = m[c] + 1;
-            lo = nlo;
-            hi = nhi;
+            split_points(lo, hi, m);
+            fits(m, ok);
+            narrow(m, ok, lo, hi);
         }
     }
-    const float best = key_float(hi);
-    for (int b = tid; b < nb; b += blockDim.x) tgt[b] = land(b, best);
+    const float lam = key_float(hi);
+    for (int b = tid; b < nb; b += kAllocThreads) tgt[b] = land(b, lam);
 }
 
 // Sums in integers are the doubles' sums when every rung costs a whole number of bits and 512 of them fit 31 bits.
@@ -213,9 +300,9 @@ template <bool TABLE>
 static int launch_allocate(const AllocParams& p, int problems, cudaStream_t stream) {
     if (p.nb <= kAllocThreads && whole_bits(p.bits)) {
         const int threads = (p.nb + 31) & ~31;
-        allocate_kernel<true, TABLE><<<problems, threads, 0, stream>>>(p);
+        allocate_small_kernel<TABLE><<<problems, threads, 0, stream>>>(p);
     } else {
-        allocate_kernel<false, TABLE><<<problems, kAllocThreads, 0, stream>>>(p);
+        allocate_kernel<TABLE><<<problems, kAllocThreads, 0, stream>>>(p);
     }
     GKV_LAUNCH_CHECK();
     return GKV_OK;
