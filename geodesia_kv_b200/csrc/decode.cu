@@ -2,6 +2,8 @@
 
 #include <string.h>
 
+#include <utility>
+
 #include "decode_generic.cuh"
 #include "decode_mma.cuh"
 
@@ -50,8 +52,6 @@ constexpr int kCombineThreads = 256;
 // One CTA per output row.  The records of a row are shared out over the NW warps (record s goes
 // to warp s mod NW, whose lanes read it coalesced), each warp keeps a running (m, l, o) of its
 // records, and the NW states are merged through shared memory — the same recurrence at both levels.
-// NW = 8 normally; 32 for rows with a few hundred records, which one wide CTA merges faster than
-// two launches of narrow ones (the single-sequence case, where the call is launch-bound).
 // KPER = channels per lane (D <= 32 * KPER): head dims up to 128 take the instantiation with half the
 // registers, which lets half as many more CTAs sit on an SM (the kernel is bound by the latency of its few
 // loads per warp, i.e. by how many CTAs are resident).
@@ -70,6 +70,8 @@ __global__ void __launch_bounds__(NW * 32) combine_kernel(CombineParams p) {
         base = p.rec + (size_t)orow * (D + 2);
         stride = p.stride_s;
     }
+    mma::grid_release();
+    mma::grid_wait();
     const float poison = (p.status && *p.status) ? __int_as_float(0x7fc00000) : 0.f;
     constexpr int kPer = KPER;                        // channels per lane
     float m = -INFINITY, l = 0.f, o[kPer];
@@ -98,16 +100,25 @@ __global__ void __launch_bounds__(NW * 32) combine_kernel(CombineParams p) {
                 v[b][i] = d < D ? rec[2 + d] : 0.f;
             }
         }
+        // one reference for the batch: its exponentials are independent of one another, where a running
+        // reference makes a chain of two per record
+        float mn = m;
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) mn = fmaxf(mn, ms[b]);
+        if (!(mn > -INFINITY)) continue;                 // nothing but empty slices so far (warp-uniform)
+        const float a = expf(m - mn);                    // 0 while m = -inf
+        l *= a;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) o[i] *= a;
 #pragma unroll
         for (int b = 0; b < kBatch; ++b) {
-            if (!(ms[b] > -INFINITY)) continue;          // empty slice (warp-uniform)
-            const float mn = fmaxf(m, ms[b]);
-            const float a = expf(m - mn), bb = expf(ms[b] - mn);   // a = 0 while m = -inf
-            l = l * a + ls[b] * bb;
+            if (!(ms[b] > -INFINITY)) continue;          // empty slice (warp-uniform): its words may hold anything
+            const float w = expf(ms[b] - mn);
+            l = fmaf(ls[b], w, l);
 #pragma unroll
-            for (int i = 0; i < kPer; ++i) o[i] = o[i] * a + v[b][i] * bb;
-            m = mn;
+            for (int i = 0; i < kPer; ++i) o[i] = fmaf(v[b][i], w, o[i]);
         }
+        m = mn;
     }
     if (lane == 0) { sm_m[warp] = m; sm_l[warp] = l; }
 #pragma unroll
@@ -145,27 +156,35 @@ __global__ void __launch_bounds__(NW * 32) combine_kernel(CombineParams p) {
 // quantity geodesia_kv/policies.py:1497-1509 obtains from a dense softmax over the keys.  Here it is put
 // together from what the decode kernel reported per block half and head — the reference m it was using
 // and the sum of exp(s - m) — and the final (M, L) of every head: weight = exp(m - M) * sum / L.
+//
+// Eight lanes per block, one head each (the tensor-core kernel takes at most eight heads per row): all reports of a
+// block are in flight at once and a warp's loads are contiguous; with a thread per block they were a chain of
+// dependent loads and uncoalesced.
 __global__ void block_mass_kernel(const float2* __restrict__ part, const float2* __restrict__ ml,
                                   const int32_t* __restrict__ level, const int32_t* __restrict__ valid,
                                   float* __restrict__ mass, int rows, int nb, int rep, int upb, int per_row_meta) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)rows * nb) return;
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int h = threadIdx.x & 7;
+    if (i >= (size_t)rows * nb) return;                     // whole groups of eight lanes
+    mma::grid_wait();
+    const unsigned group = 0xffu << (threadIdx.x & 24);
     const int row = (int)(i / nb), b = (int)(i % nb);
     const size_t mi = (size_t)(per_row_meta ? row : 0) * nb + b;
+    const bool live = valid[mi] > 0 && level_ok(level[mi]);
     float acc = 0.f;
-    if (valid[mi] > 0 && level_ok(level[mi])) {
-        for (int h = 0; h < rep; ++h) {
-            const float2 f = ml[(size_t)row * rep + h];
-            float w = 0.f;
-            for (int u = 0; u < upb; ++u) {
-                const float2 pr = part[(i * upb + u) * rep + h];
-                if (pr.x > -INFINITY) w += expf(pr.x - f.x) * pr.y;
-            }
-            acc += w / fmaxf(f.y, 1e-20f);
+    if (live && h < rep) {
+        const float2 f = ml[(size_t)row * rep + h];
+        float w = 0.f;
+#pragma unroll 4
+        for (int u = 0; u < upb; ++u) {
+            const float2 pr = part[(i * upb + u) * rep + h];
+            if (pr.x > -INFINITY) w += expf(pr.x - f.x) * pr.y;
         }
-        acc /= (float)rep;
+        acc = w / fmaxf(f.y, 1e-20f);
     }
-    mass[i] = acc;
+#pragma unroll
+    for (int o = 4; o; o >>= 1) acc += __shfl_xor_sync(group, acc, o);
+    if (h == 0) mass[i] = acc / (float)rep;
 }
 
 // ---- final merge of a sequence that is split over several GPUs ------------------------------------
@@ -336,15 +355,12 @@ struct Plan {
     int parts;            // records per cache row and query head (the tensor-core kernel writes one per consumer warp)
     int segs;             // > 1: the merge runs in two levels, `segs` partial merges per output row first
     bool mma;             // tensor-core kernel (persistent, work items of `bps` blocks)
-    bool wide = false;    // one merge level by a CTA of 32 warps (a few hundred records per row)
     int grid;
 };
 
 constexpr size_t kHeaderBytes = 256;   // work counter + status word in front of the records
 constexpr int kAutoItemBlocks = 64;     // largest work item the planner picks by itself
 constexpr int kCombineDirect = 256;    // up to this many records per output row one CTA merges them all
-constexpr int kCombineWide = 256;      // up to this many, one CTA of 32 warps would (measured slower than two levels on the
-                                       // single-sequence case, 34.8 against 28.7 us per call: not used, same as kCombineDirect)
 constexpr int kCombineSegs = 32;       // above it: this many CTAs per row merge a slice each, then one merges those
 
 static bool mma_shape_ok(int D, int group, int rep) {
@@ -407,8 +423,7 @@ static Plan make_plan(int rows, int nb, int D, int group, int rep, bool allow_mm
         const int cmin = chunk < mma::kMaxCentroidItemBlocks ? chunk : mma::kMaxCentroidItemBlocks;
         pl.nsplit = (nb + cmin - 1) / cmin + 4;
         pl.parts = pl.nsplit * mma::kConsumerWarps;
-        pl.wide = pl.parts > kCombineDirect && pl.parts <= kCombineWide;
-        pl.segs = pl.parts > kCombineWide ? (pl.parts / 64 < kCombineSegs ? pl.parts / 64 : kCombineSegs) : 1;
+        pl.segs = pl.parts > kCombineDirect ? (pl.parts / 64 < kCombineSegs ? pl.parts / 64 : kCombineSegs) : 1;
         return pl;
     }
     // generic kernel: enough slices for ~4 CTAs per SM
@@ -514,13 +529,25 @@ static void make_tensor_maps(mma::TensorMaps& tm, const uint8_t* data, size_t to
     tm.usable = ok ? 1 : 0;
 }
 
+// Launch that may start before the stream's previous kernel has ended (see mma::grid_wait).
+template <class... KArgs, class... Args>
+static int launch_overlapped(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    GKV_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
+    return GKV_OK;
+}
+
 template <int D, int G, bool DUP, bool MASS>
 static int launch_mma3(const mma::Params& p, const mma::TensorMaps& tm, int grid, cudaStream_t stream) {
     static unsigned char done[kMaxDevices] = {0};
     if (const int rc = opt_in_smem(mma::decode_mma_kernel<D, G, DUP, MASS>, done, mma::Cfg<D, G>::SMEM)) return rc;
-    mma::decode_mma_kernel<D, G, DUP, MASS><<<grid, mma::kThreads, mma::Cfg<D, G>::SMEM, stream>>>(p, tm);
-    GKV_LAUNCH_CHECK();
-    return GKV_OK;
+    return launch_overlapped(mma::decode_mma_kernel<D, G, DUP, MASS>, dim3((unsigned)grid), mma::kThreads, mma::Cfg<D, G>::SMEM,
+                             stream, p, tm);
 }
 
 template <int D, int G, bool DUP>
@@ -545,6 +572,11 @@ static int launch_plan(const int32_t* level, const int32_t* valid, const int64_t
                                                             header ? (int)(kHeaderBytes / 4) : 0);
     GKV_LAUNCH_CHECK();
     return GKV_OK;
+}
+
+static int launch_combine(const CombineParams& c, dim3 grid, cudaStream_t stream) {
+    return c.D <= 128 ? launch_overlapped(combine_kernel<8, 4>, grid, kCombineThreads, 0, stream, c)
+                      : launch_overlapped(combine_kernel<8>, grid, kCombineThreads, 0, stream, c);
 }
 
 static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs, const void* klo,
@@ -585,7 +617,8 @@ static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs,
         if (plan) {
             // the caller keeps the block lists (they change only with level/valid/offs): only the
             // work counter and the status word have to start at zero
-            GKV_CUDA_TRY(cudaMemsetAsync(header, 0, kHeaderBytes, stream));
+            mma::reset_kernel<<<1, (int)(kHeaderBytes / 4), 0, stream>>>(header, (int)(kHeaderBytes / 4));
+            GKV_LAUNCH_CHECK();
         } else {
             // the block lists sit at the end of the workspace, behind the records of either kernel
             uint4* mine = reinterpret_cast<uint4*>(static_cast<uint8_t*>(workspace) + need - perm_bytes(meta_rows, nb));
@@ -648,23 +681,19 @@ static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs,
         // level 1: (rows, parts, rep, D+2) -> (segs, B*Hq, D+2) behind the records
         float* mid = records + (size_t)B * Hq * pl.parts * (D + 2);
         c.out = mid; c.normalise = 0; c.segs = pl.segs; c.per_seg = (pl.parts + pl.segs - 1) / pl.segs;
-        if (D <= 128) combine_kernel<8, 4><<<dim3(B * Hq, pl.segs), kCombineThreads, 0, stream>>>(c);
-        else combine_kernel<8><<<dim3(B * Hq, pl.segs), kCombineThreads, 0, stream>>>(c);
-        GKV_LAUNCH_CHECK();
+        if (const int rc = launch_combine(c, dim3(B * Hq, pl.segs), stream)) return rc;
         c.rec = mid; c.out = out; c.parts = pl.segs; c.rep = 0; c.nsplit = 0; c.plan_tab = nullptr;
         c.stride_s = (int64_t)B * Hq * (D + 2); c.normalise = normalise; c.segs = 1; c.per_seg = 0;
     }
     c.ml_out = mass_ml;
     if (xch) exchange_combine_kernel<<<B * Hq, kCombineThreads, 0, stream>>>(c, *xch);
-    else if (pl.wide && pl.segs <= 1) combine_kernel<32><<<B * Hq, 1024, 0, stream>>>(c);
-    else if (D <= 128) combine_kernel<8, 4><<<B * Hq, kCombineThreads, 0, stream>>>(c);
-    else combine_kernel<8><<<B * Hq, kCombineThreads, 0, stream>>>(c);
+    else if (const int rc = launch_combine(c, dim3(B * Hq), stream)) return rc;
     GKV_LAUNCH_CHECK();
     if (mass_out) {
-        const size_t n = (size_t)rows * nb;
-        block_mass_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(mass_part, mass_ml, level, valid, mass_out, rows, nb,
-                                                                       rep, kP / group, meta_rows != 1);
-        GKV_LAUNCH_CHECK();
+        const size_t n = (size_t)rows * nb * 8;
+        if (const int rc = launch_overlapped(block_mass_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, (const float2*)mass_part,
+                                             (const float2*)mass_ml, level, valid, mass_out, rows, nb, rep, kP / group, (int)(meta_rows != 1)))
+            return rc;
     }
     return GKV_OK;
 }
@@ -699,9 +728,10 @@ size_t gkv_decode_workspace_bytes(int B, int Hq, int Hkv, int D, int nb) {
 int gkv_decode_launch_count(int B, int Hq, int Hkv, int D, int nb, int group, int planned) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || D <= 0 || nb < 0 || group <= 0) return 0;
     const gkv::Plan pl = gkv::make_plan(B * Hkv, nb, D, group, Hq / Hkv, nb > 0);
-    // tensor-core path: block lists (unless the caller keeps them), split kernel, one or two merge
-    // levels; generic path: split kernel, merge
-    return pl.mma ? (planned ? 1 : 2) + (pl.segs > 1 ? 2 : 1) : 2;
+    // tensor-core path: block lists (or, where the caller keeps them, the reset of the call's counter), split kernel,
+    // one or two merge levels; generic path: split kernel, merge
+    (void)planned;
+    return pl.mma ? 2 + (pl.segs > 1 ? 2 : 1) : 2;
 }
 
 int gkv_decode_kernel_launches(int B, int Hq, int Hkv, int D, int nb, int group) {
@@ -844,6 +874,7 @@ int gkv_combine_partials(const float* partials, float* out, int parts, int rows,
     c.rec = partials; c.out = out; c.parts = parts; c.D = D; c.rep = 0; c.nsplit = 0;
     c.stride_s = (int64_t)rows * (D + 2); c.normalise = 1; c.status = nullptr; c.segs = 1; c.per_seg = 0; c.ml_out = nullptr;
     c.plan_tab = nullptr; c.chunk = 1; c.tab_per_row = 0; c.warps_per_item = 1;
+    // the records come from anywhere in the stream: launched the ordinary way
     if (D <= 128) gkv::combine_kernel<8, 4><<<rows, gkv::kCombineThreads, 0, static_cast<cudaStream_t>(stream)>>>(c);
     else gkv::combine_kernel<8><<<rows, gkv::kCombineThreads, 0, static_cast<cudaStream_t>(stream)>>>(c);
     GKV_LAUNCH_CHECK();
