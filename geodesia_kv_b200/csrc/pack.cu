@@ -533,7 +533,7 @@ __global__ void clear_table_kernel(int64_t* offs, int32_t* level, int32_t* valid
 // ---- persistent, bulk-copy-fed kernels ---------------------------------------------------------------
 // The kernels above start a CTA per block: the CTA reads the block's table entries, then its bytes, then
 // computes, then stores — a chain of dependent memory round trips that two resident CTAs per SM cannot
-// hide.  Here CTAs are persistent (two per SM) and hold a ninth warp, the producer: it looks up block
+// hide.  Here CTAs are persistent (three per SM) and hold a ninth warp, the producer: it looks up block
 // i + grid (table entries: two dependent global loads) and starts ONE bulk copy per contiguous piece of
 // its source (K rows, V rows; or the packed block and its scale planes) into a two-stage ring in shared
 // memory while the 256 working threads are on block i out of the other stage, so every global-memory
@@ -544,8 +544,12 @@ namespace st {
 
 constexpr int kStages = 2;
 constexpr int kTileBytes = 2 * kP * 128 * 2;          // the largest block: rung 16 at D = 128
-constexpr int kScaleBytes = 4 * 4 * 128 * 2;          // four planes of at most (4, 128) fp16
-constexpr int kStageBytes = kTileBytes + kScaleBytes;
+constexpr int kStageBytes = kTileBytes;
+// A packed block of a quantised rung is at most half a tile long: its four scale planes (at most (4, 128) fp16 each) and the
+// partial K ranges of its re-quantisation stand behind it in the stage.
+constexpr int kScalesAt = kTileBytes / 2, kRangesAt = kScalesAt + 4 * 4 * 128 * 2;
+static_assert(kRangesAt + 2 * 8 * 128 * 4 <= kStageBytes, "room behind a packed block");
+constexpr int kCtasPerSM = 3;                         // 72 registers and 75 KB of shared memory each
 constexpr unsigned long long kWaitNs = 2000000000ull; // a copy that has not landed after 2 s never will
 
 struct Desc {
@@ -556,7 +560,7 @@ struct Desc {
 };
 
 struct __align__(128) Smem {
-    rq::Shared work;
+    rq::Work work;
     Desc desc[kStages];
     unsigned long long full[kStages];
     unsigned long long empty[kStages];
@@ -729,7 +733,7 @@ __device__ void fetch(const P& p, int i, int n, Smem& sm, int s, int G, int gv) 
                 bar_expect(&sm.full[s], bytes + (q ? 2 * ks + 2 * vs : 0u));
                 bulk(st, d.old_blk, bytes, &sm.full[s]);
                 if (q) {
-                    uint8_t* sc = st + kTileBytes;
+                    uint8_t* sc = st + kScalesAt;
                     bulk(sc, d.oklo, ks, &sm.full[s]);
                     bulk(sc + ks, d.okstep, ks, &sm.full[s]);
                     bulk(sc + 2 * ks, d.ovlo, vs, &sm.full[s]);
@@ -762,7 +766,7 @@ __device__ void copy_by_hand(const Desc& d, uint8_t* st, int G, int gv) {
     const int bytes = 2 * half_bytes(d.old_level, D);
     for (int e = tid; e < bytes; e += rq::kThreads) st[e] = d.old_blk[e];
     if (d.old_level == 8 || d.old_level == 4 || d.old_level == 2) {
-        __half* sc = reinterpret_cast<__half*>(st + kTileBytes);
+        __half* sc = reinterpret_cast<__half*>(st + kScalesAt);
         for (int e = tid; e < G * D; e += rq::kThreads) { sc[e] = d.oklo[e]; sc[G * D + e] = d.okstep[e]; }
         for (int e = tid; e < kP * gv; e += rq::kThreads) { sc[2 * G * D + e] = d.ovlo[e]; sc[2 * G * D + kP * gv + e] = d.ovstep[e]; }
     }
@@ -771,7 +775,7 @@ __device__ void copy_by_hand(const Desc& d, uint8_t* st, int G, int gv) {
 constexpr int kStagedThreads = rq::kThreads + 32;      // 256 working threads + the producer warp
 
 template <int D, class P>
-__global__ void __launch_bounds__(kStagedThreads, 2) staged_kernel(P p, int n, int group) {
+__global__ void __launch_bounds__(kStagedThreads, kCtasPerSM) staged_kernel(P p, int n, int group) {
     extern __shared__ __align__(128) uint8_t raw[];
     Smem& sm = *reinterpret_cast<Smem*>(raw);
     const int tid = threadIdx.x;
@@ -832,7 +836,8 @@ __global__ void __launch_bounds__(kStagedThreads, 2) staged_kernel(P p, int n, i
                 src.v = st + half_bytes(d.old_level, D);
             }
             src.k32 = s32(src.k); src.v32 = s32(src.v);
-            src.klo = reinterpret_cast<const __half*>(st + kTileBytes); src.kstep = src.klo + G * D;
+            src.fpart = reinterpret_cast<float*>(st + kRangesAt);
+            src.klo = reinterpret_cast<const __half*>(st + kScalesAt); src.kstep = src.klo + G * D;
             src.vlo = src.kstep + G * D; src.vstep = src.vlo + kP * gv;
             rq::requantise_staged<D, P::kPacked, P::kMayRadii>(src, j, sm.work);
         }
@@ -869,7 +874,7 @@ static int launch(const P& p, int n, int group, bool fp32_rows, cudaStream_t str
     GKV_CUDA_TRY(cudaGetDevice(&dev));
     GKV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     GKV_CUDA_TRY(cudaFuncSetAttribute(staged_kernel<D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
-    const int grid = n < 2 * sms ? n : 2 * sms;
+    const int grid = n < kCtasPerSM * sms ? n : kCtasPerSM * sms;
     staged_kernel<D, P><<<grid, kStagedThreads, sizeof(Smem), stream>>>(p, n, group);
     GKV_LAUNCH_CHECK();
     return GKV_OK;

@@ -44,10 +44,8 @@ struct Job {
 };
 
 struct __align__(16) Shared {
-    union {
-        struct { uint32_t kmin[4 * 128], kmax[4 * 128]; };      // [G][D] order-preserving keys (requantise)
-        float part[2 * 8 * 128];                                // [min, max][warp][D] K ranges of eight tokens (quantise_staged)
-    };
+    uint32_t kmin[4 * 128];     // [G][D] order-preserving keys
+    uint32_t kmax[4 * 128];
     float4 ks[4 * 128];         // [G][D] (lo16, step16, 1 / step16) as fp32
     uint32_t err[2];            // max error norms (bits of non-negative floats)
     float csum[2][kP];          // centroid target: per-token squared error sums
@@ -461,11 +459,20 @@ __device__ void requantise(const Job& j, Shared& sm) {
 // warp that feeds the stages), which must not be part of these barriers.
 __device__ __forceinline__ void work_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
+// Work area of a CTA beside its stages.  Small on purpose: with two 32 KB stages it decides whether three CTAs fit an SM.
+struct __align__(16) Work {
+    uint16_t part[2 * 8 * 128];  // [min, max][warp][D]: K ranges of eight tokens (16-bit sources); centroid: the means as floats
+    float2 lr[4 * 128];          // [G][D] low end and code factor of the K groups
+    __half s[4 * 128];           // [G][D] step of the K groups
+    uint32_t err[2];             // max error norms (bits of non-negative floats)
+};
+
 struct StagedSrc {
     const uint8_t* k; const uint8_t* v;     // dense tiles (kind 1 bf16, 2 fp16), or the halves of the packed block (kind 3)
     int kind, nvalid, level;                // level: rung of a packed source (8, 4 or 2)
     const __half* klo; const __half* kstep; const __half* vlo; const __half* vstep;
     int kgs, vgs;                           // log2 of the K token group and of the V channel group (both powers of two)
+    float* fpart;                           // packed sources: room for [min, max][warp][D] fp32 K ranges (a free part of the stage)
     uint32_t k32, v32;                      // k and v as shared-memory addresses: plain 32-bit arithmetic, LDS instead of generic loads
 };
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
@@ -584,9 +591,10 @@ __device__ __forceinline__ Scale scale_of(float lo, float hi) {
 // multiply-add rounds to nearest-even and leaves the integer in the low 16 bits (two's complement; quotients
 // stay below 30000, see scale_of), where pairs are clamped by one instruction.  Returns the octet's squared
 // reconstruction error when RADII.
-// NS = 8: a scale per channel; 1: one for the octet.
-template <int LV, bool RADII, int NS>
-__device__ __forceinline__ float codes8(const float (&x)[8], const float (&l)[NS], const float (&s)[NS], const float (&r)[NS], uint32_t (&w)[LV == 8 ? 2 : 1]) {
+// NS = 8: a scale per channel; 1: one for the octet.  step_of(c): the step of channel c, which only the exact division
+// and the radii need.
+template <int LV, bool RADII, int NS, class Step>
+__device__ __forceinline__ float codes8(const float (&x)[8], const float (&l)[NS], const float (&r)[NS], const Step& step_of, uint32_t (&w)[LV == 8 ? 2 : 1]) {
     constexpr float kMagic = 12582912.0f, qmax = (float)((1 << LV) - 1), tie = 0.5f - (qmax + 1.0f) * 2.5e-7f;
     float m[8];
     bool redo = false;                         // some quotient is near a tie, or not a number
@@ -609,11 +617,11 @@ __device__ __forceinline__ float codes8(const float (&x)[8], const float (&l)[NS
         while (todo) {
             const int at = __ffs((int)todo) - 1;
             todo &= todo - 1u;
-            float xa = x[0], la = l[0], sa = s[0];
+            float xa = x[0], la = l[0];
 #pragma unroll
             for (int c = 1; c < 8; ++c)
-                if (at == c) { xa = x[c]; la = l[c % NS]; sa = s[c % NS]; }
-            const float q = rintf(__fdiv_rn(__fsub_rn(xa, la), sa));
+                if (at == c) { xa = x[c]; la = l[c % NS]; }
+            const float q = rintf(__fdiv_rn(__fsub_rn(xa, la), step_of(at)));
             const float ma = kMagic + ((q != q) ? 0.f : fminf(fmaxf(q, 0.f), qmax));
 #pragma unroll
             for (int c = 0; c < 8; ++c)
@@ -640,7 +648,7 @@ __device__ __forceinline__ float codes8(const float (&x)[8], const float (&l)[NS
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             const float q = fminf(fmaxf(__fsub_rn(m[c], kMagic), 0.f), qmax);
-            const float e = x[c] - __fmaf_rn(q, s[c % NS], l[c % NS]);
+            const float e = x[c] - __fmaf_rn(q, step_of(c), l[c % NS]);
             e2 += e * e;
         }
     }
@@ -675,8 +683,10 @@ __device__ __forceinline__ void store_octet(uint8_t* out, const uint32_t (&w)[LV
 // Measured, 4096 blocks per launch, bf16 in, D = 128, g = 32, ns per block of the whole chip, with one body for all
 // that found K ranges by shared-memory atomics and took every quotient apart from the others' -> so: 8-bit 29.6 -> 19.0,
 // 4-bit 29.2 -> 16.1, 2-bit 29.1 -> 16.1, centroid 9.2 -> 8.0, the mix 35.6 -> 16.4.
+// With three CTAs of 72 registers per SM instead of two of 96: 8-bit 16.8, 4-bit 15.2, 2-bit 15.2, centroid 7.1, mix 15.8
+// (three CTAs with one stage each: 19.5, 17.6, 17.6, 8.9, 17.8).
 template <int D, int LV, int SRC, bool RADII>
-__device__ __forceinline__ void quantise_staged(const StagedSrc& src, const Job& j, Shared& sm) {
+__device__ __forceinline__ void quantise_staged(const StagedSrc& src, const Job& j, Work& sm) {
     constexpr int OPR = D / 8, NI = kP * OPR / kThreads;       // octets per row; tokens of K per thread
     constexpr bool T16 = SRC != 3;
     constexpr uint32_t PINF = SRC == 2 ? 0x7C007C00u : 0x7F807F80u, NINF = SRC == 2 ? 0xFC00FC00u : 0xFF80FF80u;
@@ -706,7 +716,7 @@ __device__ __forceinline__ void quantise_staged(const StagedSrc& src, const Job&
                 lo[c] = min2<SRC>(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
                 hi[c] = max2<SRC>(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
             }
-        uint16_t* part = reinterpret_cast<uint16_t*>(sm.part);             // [2][8 warps][D]
+        uint16_t* part = sm.part;                                          // [2][8 warps][D]
         if (lane < OPR) *reinterpret_cast<uint4*>(part + warp * D + 8 * c8) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         else if (lane < 2 * OPR) *reinterpret_cast<uint4*>(part + (8 + warp) * D + 8 * c8) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     } else {
@@ -728,10 +738,10 @@ __device__ __forceinline__ void quantise_staged(const StagedSrc& src, const Job&
                 hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
             }
         if (lane < OPR) {
-            float4* part = reinterpret_cast<float4*>(sm.part + (size_t)warp * D + 8 * c8);
+            float4* part = reinterpret_cast<float4*>(src.fpart + warp * D + 8 * c8);
             part[0] = make_float4(lo[0], lo[1], lo[2], lo[3]); part[1] = make_float4(lo[4], lo[5], lo[6], lo[7]);
         } else if (lane < 2 * OPR) {
-            float4* part = reinterpret_cast<float4*>(sm.part + (size_t)(8 + warp) * D + 8 * c8);
+            float4* part = reinterpret_cast<float4*>(src.fpart + (8 + warp) * D + 8 * c8);
             part[0] = make_float4(hi[0], hi[1], hi[2], hi[3]); part[1] = make_float4(hi[4], hi[5], hi[6], hi[7]);
         }
     }
@@ -801,9 +811,10 @@ __device__ __forceinline__ void quantise_staged(const StagedSrc& src, const Job&
             float x[8];
             staged_octet<D, SRC>(src, 1, t, q4 * NO + (o ^ f), x);
             const bool second = NSET == 2 && o >= OS;
-            const float l[1] = {second ? sc[NSET - 1].l : sc[0].l}, s[1] = {second ? sc[NSET - 1].s : sc[0].s}, r[1] = {second ? sc[NSET - 1].r : sc[0].r};
+            const float l[1] = {second ? sc[NSET - 1].l : sc[0].l}, r[1] = {second ? sc[NSET - 1].r : sc[0].r};
+            const float step = second ? sc[NSET - 1].s : sc[0].s;
             uint32_t w[NW];
-            const float e = codes8<LV, RADII, 1>(x, l, s, r, w);
+            const float e = codes8<LV, RADII, 1>(x, l, r, [&](int) { return step; }, w);
             store_octet<LV>(vdst + (o ^ f) * LV, w, aligned);
             if constexpr (RADII) {
                 pair = (o & 1) ? pair + e : e;
@@ -824,34 +835,36 @@ __device__ __forceinline__ void quantise_staged(const StagedSrc& src, const Job&
         float lo = INFINITY, hi = -INFINITY;
         for (int w = w0; w < w1; ++w) {
             if constexpr (T16) {
-                const uint16_t* part = reinterpret_cast<const uint16_t*>(sm.part);
-                lo = fminf(lo, widen<SRC>(part[w * D + d]));
-                hi = fmaxf(hi, widen<SRC>(part[(8 + w) * D + d]));
+                lo = fminf(lo, widen<SRC>(sm.part[w * D + d]));
+                hi = fmaxf(hi, widen<SRC>(sm.part[(8 + w) * D + d]));
             } else {
-                lo = fminf(lo, sm.part[w * D + d]);
-                hi = fmaxf(hi, sm.part[(8 + w) * D + d]);
+                lo = fminf(lo, src.fpart[w * D + d]);
+                hi = fmaxf(hi, src.fpart[(8 + w) * D + d]);
             }
         }
         const Scale k = scale_of<LV>(lo, hi);
         j.klo[u] = k.l16; j.kstep[u] = k.s16;
-        // a thread reads the entries of its eight channels: the lanes of a token row read consecutive 16-byte slots
-        sm.ks[(tg * 8 + (d & 7)) * OPR + (d >> 3)] = make_float4(k.l, k.s, k.r, 0.f);
+        // a thread reads the entries of its eight channels: the lanes of a token row read consecutive slots
+        const int at = (tg * 8 + (d & 7)) * OPR + (d >> 3);
+        sm.lr[at] = make_float2(k.l, k.r);
+        sm.s[at] = k.s16;
     }
     work_sync();                               // also: every source byte has been read before the first K code is stored
 
     // ---- K codes ---------------------------------------------------------------------------
     {
-        const float4* sc = sm.ks + (t0 >> kgs) * 8 * OPR + c8;
-        float l[8], s[8], r[8];
+        const int at = (t0 >> kgs) * 8 * OPR + c8;
+        float l[8], r[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) { const float4 k = sc[c * OPR]; l[c] = k.x; s[c] = k.y; r[c] = k.z; }
+        for (int c = 0; c < 8; ++c) { const float2 k = sm.lr[at + c * OPR]; l[c] = k.x; r[c] = k.y; }
+        auto step_of = [&](int c) { return __half2float(sm.s[at + c * OPR]); };
         uint8_t* kdst = j.dst + (t0 * D + 8 * c8) * LV / 8;
 #pragma unroll 1
         for (int i = 0; i < NI; ++i) {
             float x[8];
             staged_octet<D, SRC>(src, 0, t0 + i, c8, x);
             uint32_t w[NW];
-            float e2 = codes8<LV, RADII, 8>(x, l, s, r, w);
+            float e2 = codes8<LV, RADII, 8>(x, l, r, step_of, w);
             store_octet<LV>(kdst + i * (D * LV / 8), w, aligned);
             if constexpr (RADII) {
 #pragma unroll
@@ -879,10 +892,10 @@ __device__ __forceinline__ void quantise_staged(const StagedSrc& src, const Job&
 // costs it one 4-byte load, two widenings and two additions; what bounds it is the chain of 64 additions.  Radii:
 // a thread adds up a quarter of a token's row, as in the V half of the quantised rungs.
 template <int D, int SRC, bool RADII>
-__device__ __forceinline__ void centroid_staged(const StagedSrc& src, const Job& j, Shared& sm) {
+__device__ __forceinline__ void centroid_staged(const StagedSrc& src, const Job& j, Work& sm) {
     constexpr int E = D / 4, NO = E / 8;
     const int tid = threadIdx.x, lane = tid & 31;
-    float* mean = sm.part;                                 // [2][D], fp16-rounded
+    float* mean = reinterpret_cast<float*>(sm.part);       // [2][D], fp16-rounded
     if constexpr (SRC != 3) {
         if (tid < D) {
             const int which = tid / (D / 2), c = 2 * (tid % (D / 2));
@@ -960,7 +973,7 @@ __device__ __forceinline__ void centroid_staged(const StagedSrc& src, const Job&
 // The rungs of a source kind: PACKED launches demote (bf16 tiles of a rung-16 block, or a quantised block, which
 // only moves further down), the others pack dense bf16 / fp16 rows.  MAY_RADII: the launch may ask for error radii.
 template <int D, int SRC, bool RADII>
-__device__ __forceinline__ void quantise_rung(const StagedSrc& src, const Job& j, Shared& sm) {
+__device__ __forceinline__ void quantise_rung(const StagedSrc& src, const Job& j, Work& sm) {
     if (j.level == 1) { centroid_staged<D, SRC, RADII>(src, j, sm); return; }
     // one body per rung, so that every shift, mask and byte offset is a constant
     if constexpr (SRC != 3) {
@@ -970,7 +983,7 @@ __device__ __forceinline__ void quantise_rung(const StagedSrc& src, const Job& j
     else quantise_staged<D, 2, SRC, RADII>(src, j, sm);
 }
 template <int D, int SRC, bool MAY_RADII>
-__device__ __forceinline__ void quantise_src(const StagedSrc& src, const Job& j, Shared& sm) {
+__device__ __forceinline__ void quantise_src(const StagedSrc& src, const Job& j, Work& sm) {
     if constexpr (MAY_RADII) {
         if (j.ek != nullptr) { quantise_rung<D, SRC, true>(src, j, sm); return; }
     }
@@ -978,7 +991,7 @@ __device__ __forceinline__ void quantise_src(const StagedSrc& src, const Job& j,
 }
 
 template <int D, bool PACKED, bool MAY_RADII>
-__device__ void requantise_staged(const StagedSrc& src, const Job& j, Shared& sm) {
+__device__ void requantise_staged(const StagedSrc& src, const Job& j, Work& sm) {
     constexpr int OPR = D / 8, ROWS = kThreads / OPR, NI = kP / ROWS;
     const int tid = threadIdx.x;
     const int c8 = tid % OPR, tr = tid / OPR;
