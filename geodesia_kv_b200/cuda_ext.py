@@ -173,7 +173,7 @@ class _Extension:
                 ws = self._workspace(dev, need)
                 plan = self._plan(offs, level, valid, meta_rows, nb)
                 out = torch.empty((B, Hq, D), dtype=torch.float32, device=dev)
-                bm = torch.zeros((B, Hkv, nb), dtype=torch.float32, device=dev)
+                bm = torch.empty((B, Hkv, nb), dtype=torch.float32, device=dev)       # every entry is written
                 rc = 0
                 if nb:
                     rc = self.lib.gkv_mixed_attn_decode_mass(
