@@ -74,7 +74,8 @@ size_t gkv_decode_workspace_bytes(int B, int Hq, int Hkv, int D, int nb);
 /* Number of kernels one decode call of this shape launches (host arithmetic only; for callers
  * that account for launches, e.g. a benchmark).  Assumes 16-byte aligned scale planes, which is
  * what selects the tensor-core kernel.  `planned` != 0: the caller passes prebuilt block lists
- * (gkv_mixed_attn_decode_planned), which saves one kernel.  No counterpart in the reference.   */
+ * (gkv_mixed_attn_decode_planned); a one-CTA reset of the call's counter then stands in for the
+ * block-list kernel, so the count is the same.  No counterpart in the reference.               */
 int gkv_decode_kernel_launches(int B, int Hq, int Hkv, int D, int nb, int group);
 int gkv_decode_launch_count(int B, int Hq, int Hkv, int D, int nb, int group, int planned);
 
