@@ -167,3 +167,32 @@ def test_table_form_plans_as_the_array_form():
                                        target.data_ptr(), 1.0, ratio.data_ptr(), want.data_ptr(), nb_of.data_ptr(), rows, nb, stream) == 0
         assert torch.equal(got, want), step
         assert step or layer.apply_demotion(got.cpu().numpy()) > 0
+
+
+@pytest.mark.parametrize("B,Hq,Hkv", [(1, 7, 1), (200, 8, 8), (120, 8, 2), (64, 64, 8), (3, 12, 4)])
+def test_merge_widths_and_mass(oracle, B, Hq, Hkv):
+    """From 7 to 4096 output rows the merge runs with 8, 2, 4, 1 and 8 warps per row; the mass takes 1 to 8 heads per cache row.
+
+    Both are sums of fp32 products whose operands carry 22 bits: 5e-5 absolute is what the kernel states for outputs of
+    order one, masses are sums of weights that add up to one."""
+    from geodesia_kv_b200.cuda_ext import get_ext
+    from geodesia_kv_b200.pack_layout import pack_cache
+    nb, D, group = 9, 64, 32
+    gen = torch.Generator(device="cuda").manual_seed(B + Hq)
+    k, v = (torch.randn(B, Hkv, nb * 64 - 5, D, device="cuda", generator=gen) for _ in range(2))
+    level = torch.from_numpy(LADDER).cuda()[torch.randint(0, 5, (B, Hkv, nb), device="cuda", generator=gen)]
+    cache = pack_cache(k, v, level, group)
+    q = torch.randn(B, Hq, D, device="cuda", generator=gen) * D ** -0.5
+    ext = get_ext()
+    out, mass = ext.mixed_attn_decode_with_mass(q, *cache.kernel_args())
+    plain = ext.mixed_attn_decode(q, *cache.kernel_args())
+    ext.set_decode_kernel("generic")
+    try:
+        want = ext.mixed_attn_decode(q, *cache.kernel_args())
+    finally:
+        ext.set_decode_kernel("auto")
+    assert (out - want).abs().max() < 5e-5 and (plain - want).abs().max() < 5e-5
+    assert (mass.sum(-1) - 1).abs().max() < 1e-5
+    one = [t[:1].contiguous().cpu() for t in (q, cache.data, cache.offs, cache.klo, cache.kstep, cache.vlo, cache.vstep, cache.level, cache.valid)]
+    arrays = [t.view(torch.int16).numpy().view(np.uint16) if t.dtype == torch.float16 else t.numpy() for t in one]
+    assert np.abs(mass[:1].cpu().numpy() - oracle.block_mass(*arrays, 64, group)).max() < 1e-5
