@@ -599,6 +599,9 @@ __device__ __forceinline__ void bulk(void* dst, const void* src, uint32_t bytes,
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(s32(dst)), "l"(src), "r"(bytes), "r"(s32(b)) : "memory");
 }
+// Orders this thread's ordinary accesses to shared memory before copies of the asynchronous proxy that follow a
+// synchronisation with the thread that starts them: barriers alone order accesses of one proxy only.
+__device__ __forceinline__ void fence_before_copies() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ---- what block i of each kind of launch is ----------------------------------------------------------
@@ -840,6 +843,8 @@ __global__ void __launch_bounds__(kStagedThreads, kCtasPerSM) staged_kernel(P p,
             src.klo = reinterpret_cast<const __half*>(st + kScalesAt); src.kstep = src.klo + G * D;
             src.vlo = src.kstep + G * D; src.vstep = src.vlo + kP * gv;
             rq::requantise_staged<D, P::kPacked, P::kMayRadii>(src, j, sm.work);
+            // the stage's next block may be copied over what was stored here by hand or as partial ranges
+            if (!d.staged || src.kind == 3) fence_before_copies();
         }
         if (tid == 128) commit(p, (int)blockIdx.x + it * (int)gridDim.x);
         rq::work_sync();                               // every worker is done with the stage and the work area

@@ -196,3 +196,69 @@ def test_merge_widths_and_mass(oracle, B, Hq, Hkv):
     one = [t[:1].contiguous().cpu() for t in (q, cache.data, cache.offs, cache.klo, cache.kstep, cache.vlo, cache.vstep, cache.level, cache.valid)]
     arrays = [t.view(torch.int16).numpy().view(np.uint16) if t.dtype == torch.float16 else t.numpy() for t in one]
     assert np.abs(mass[:1].cpu().numpy() - oracle.block_mass(*arrays, 64, group)).max() < 1e-5
+
+
+def _pool_blocks(rng, D, group, levels, slot):
+    """Packed blocks with values and scales of every size, `slot` bytes apart; the bytes behind a block stay as they are."""
+    n, G, gv = levels.size, 64 // min(group, 64), D // min(group, D)
+    pool = rng.integers(0, 256, (n, slot), dtype=np.uint8)
+    for i, lv in enumerate(levels):
+        nbytes = 4 * 64 * D if lv == 16 else 64 * D * int(lv) // 4
+        if lv == 16:
+            x = torch.from_numpy(rng.standard_normal(2 * 64 * D).astype(np.float32)).bfloat16()
+            pool[i, :nbytes] = x.view(torch.int16).numpy().view(np.uint8)
+        else:
+            scales = (rng.random(2 * (G * D + 64 * gv)).astype(np.float16) + np.float16(0.01)).view(np.uint8)
+            pool[i, nbytes:nbytes + scales.size] = scales
+    return pool
+
+
+@pytest.mark.parametrize("D,group", [(128, 32), (64, 16)])
+def test_stages_shared_by_packed_and_exact_blocks(D, group):
+    """A stage of the ring holds blocks of every source rung in turn, copied in or brought in by hand (the pool that
+    starts 8 bytes off), and a packed block's partial ranges in between: the same bytes as when no stage is used twice."""
+    from geodesia_kv_b200 import _lib
+    lib, slot, n = _lib.load(), 512 * D, 4000                   # a CTA has four blocks or more, two per stage
+    rng = np.random.default_rng(D)
+    old = np.array([8, 16, 4, 16, 8, 16, 16], np.int32)[np.arange(n) % 7]
+    new = np.array([4, 4, 2, 1, 2, 8, 2], np.int32)[np.arange(n) % 7]
+    pool = torch.from_numpy(_pool_blocks(rng, D, group, old, slot)).cuda()
+    off = torch.arange(n, device="cuda") * slot
+    lo, ln = torch.from_numpy(old).cuda(), torch.from_numpy(new).cuda()
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def demote(shift, per_launch):
+        src = torch.zeros(n * slot + 16, dtype=torch.uint8, device="cuda")
+        src[shift:shift + n * slot] = pool.view(-1)
+        dst, ek, ev = torch.zeros(n * slot, dtype=torch.uint8, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+        for i in range(0, n, per_launch):
+            m = min(per_launch, n - i)
+            assert lib.gkv_paged_demote_blocks(src.data_ptr() + shift, off[i:].data_ptr(), lo[i:].data_ptr(), dst.data_ptr(), off[i:].data_ptr(),
+                                               ln[i:].data_ptr(), ek[i:].data_ptr(), ev[i:].data_ptr(), m, D, 64, group, stream) == 0
+        return dst, ek, ev
+
+    want = demote(0, 64)                                         # every CTA has one block
+    for shift in (0, 8):
+        for got, ref in zip(demote(shift, n), want):
+            assert torch.equal(got, ref), shift
+
+
+def test_stages_shared_by_rows_copied_and_rows_brought_by_hand():
+    """Every second block's rows start at an address that a copy cannot take."""
+    from geodesia_kv_b200 import _lib
+    lib, D, group, n = _lib.load(), 128, 32, 4000
+    k, v = (torch.randn(n * 64 * D + 8, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    src = torch.arange(n, device="cuda") * (64 * D) + (torch.arange(n, device="cuda") % 2) * 3
+    level = torch.tensor([8, 4, 2, 1, 16], dtype=torch.int32, device="cuda")[torch.arange(n, device="cuda") % 5].contiguous()
+    slots = torch.arange(n, device="cuda") * (256 * D)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def pack(per_launch):
+        pool = torch.zeros(n * 256 * D, dtype=torch.uint8, device="cuda")
+        for i in range(0, n, per_launch):
+            m = min(per_launch, n - i)
+            assert lib.gkv_paged_pack_blocks(k.data_ptr(), v.data_ptr(), 1, src[i:].data_ptr(), D, None, pool.data_ptr(), slots[i:].data_ptr(),
+                                             level[i:].data_ptr(), None, None, m, D, 64, group, stream) == 0
+        return pool
+
+    assert torch.equal(pack(n), pack(64))
