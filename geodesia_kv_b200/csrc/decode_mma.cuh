@@ -205,6 +205,10 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
+// Orders ordinary accesses to shared memory (among them cp.async) before bulk copies that follow, in this thread or
+// after a synchronisation with another: barriers alone order accesses of one proxy only.
+__device__ __forceinline__ void fence_before_bulk() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -621,6 +625,11 @@ __device__ __forceinline__ bool produce_item(const Params& p, const TensorMaps& 
             ps.head = head;
             ps.used = used;
         }
+        // The copies below may land on scale planes and blocks that this warp's lanes once stored in the ring.  One fence
+        // per batch here, not one per block in the warps that release the slots: 32 x 16k tokens 221.6 against 222.4 us,
+        // one sequence of 1M tokens 208.3 against 211.7.
+        fence_before_bulk();
+        __syncwarp();
         const int my_seq = ps.seq_alloc + lane;
         const int my_slot = my_seq % kNSlot;
         uint4 cur = make_uint4(0, 0, 0, 0);
@@ -1342,6 +1351,7 @@ __device__ __forceinline__ void clear_invalid_tail(uint8_t* blk, int level, int 
         uint16_t* lo = reinterpret_cast<uint16_t*>(blk + 2 * kP * RB + 2 * C::KSCALE);
         for (int i = nvalid * C::GV + lane; i < kP * C::GV; i += 32) { lo[i] = 0; lo[C::VSCALE / 2 + i] = 0; }
     }
+    fence_before_bulk();        // the next copy into these bytes comes from the producer, after the pair has released them
     __syncwarp();
 }
 

@@ -262,3 +262,30 @@ def test_stages_shared_by_rows_copied_and_rows_brought_by_hand():
         return pool
 
     assert torch.equal(pack(n), pack(64))
+
+
+@pytest.mark.parametrize("D,group,Hq", [(128, 32, 8), (64, 16, 2)])
+def test_decode_ring_of_short_and_hand_copied_blocks(oracle, D, group, Hq):
+    """Every region of the byte rings holds copied blocks, blocks at odd addresses brought in by hand, scale planes, and
+    short blocks whose tails are cleared in place, one after the other.
+
+    5e-5: the kernel's stated error for outputs of order one (operands carry 22 bits)."""
+    from geodesia_kv_b200.cuda_ext import get_ext
+    from helpers import kernel_args, oracle_args
+    Hkv, nb = 2, 700
+    c = oracle_cache(oracle, 900 + D, 1, Hkv, nb, D, group, probs=(0.2, 0.25, 0.25, 0.2, 0.1))
+    rng = np.random.default_rng(D)
+    c["valid"][:] = np.where(rng.random(c["valid"].shape) < 0.5, rng.integers(1, 65, c["valid"].shape), 64)
+    sizes = np.array([[oracle.block_bytes(int(lv), 64, D) for lv in c["level"][0, h]] for h in range(Hkv)])
+    moved = np.where(np.arange(nb) % 3 == 0, 4, 0)[None] + 16 * np.arange(nb)[None] + c["offs"][0]      # every third at an odd address
+    data = np.zeros((1, Hkv, int((moved + sizes).max()) + 64), np.uint8)
+    for h in range(Hkv):
+        for i in range(nb):
+            o, m, n = int(c["offs"][0, h, i]), int(moved[h, i]), int(sizes[h, i])
+            data[0, h, m:m + n] = c["data"][0, h, o:o + n]
+    c["data"], c["offs"] = data[..., :data.shape[-1] // 16 * 16].copy(), moved[None].astype(np.int64)
+    t = to_torch(c, "cuda")
+    q = rng.standard_normal((1, Hq, D), dtype=np.float32) * np.float32(D ** -0.5)
+    got = get_ext().mixed_attn_decode(torch.from_numpy(q).cuda(), *kernel_args(t, c)).cpu().numpy()
+    assert np.abs(got - oracle.mixed_attn_decode(q, *oracle_args(c))).max() < 5e-5
+    assert get_ext().decode_status() == 0
