@@ -522,10 +522,11 @@ __global__ void open_blocks_kernel(const int64_t* flat, const int64_t* offs, int
 }
 
 // A block table as it is before the first block enters.
-__global__ void clear_table_kernel(int64_t* offs, int32_t* level, int32_t* valid, float* mass, int32_t* lens, size_t n, int rows) {
+__global__ void clear_table_kernel(int64_t* offs, int32_t* level, int32_t* valid, float* mass, float* ek, float* ev, int32_t* lens,
+                                   size_t n, int rows) {
     const size_t step = (size_t)gridDim.x * blockDim.x;
     const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (size_t i = first; i < n; i += step) { offs[i] = -1; level[i] = 0; valid[i] = 0; mass[i] = 0.f; }
+    for (size_t i = first; i < n; i += step) { offs[i] = -1; level[i] = 0; valid[i] = 0; mass[i] = 0.f; ek[i] = 0.f; ev[i] = 0.f; }
     for (size_t i = first; i < (size_t)rows; i += step) lens[i] = 0;
 }
 
@@ -1157,16 +1158,16 @@ int gkv_paged_open_blocks(const int64_t* flat, const int64_t* offs, int n, int64
     return GKV_OK;
 }
 
-int gkv_paged_clear_table(int64_t* offs, int32_t* level, int32_t* valid, float* mass, int32_t* lens, int rows, int cap,
-                          void* stream) {
+int gkv_paged_clear_table(int64_t* offs, int32_t* level, int32_t* valid, float* mass, float* ek, float* ev, int32_t* lens,
+                          int rows, int cap, void* stream) {
     using namespace gkv;
     if (rows < 0 || cap < 0) return GKV_E_SHAPE;
     if (rows == 0) return GKV_OK;
-    if (!lens || (cap > 0 && (!offs || !level || !valid || !mass))) return GKV_E_NULL;
+    if (!lens || (cap > 0 && (!offs || !level || !valid || !mass || !ek || !ev))) return GKV_E_NULL;
     const size_t n = (size_t)rows * cap > (size_t)rows ? (size_t)rows * cap : (size_t)rows;
     const size_t want = (n + 255) / 256;
-    clear_table_kernel<<<(unsigned)(want < 4096 ? want : 4096), 256, 0, (cudaStream_t)stream>>>(offs, level, valid, mass, lens,
-                                                                                               (size_t)rows * cap, rows);
+    clear_table_kernel<<<(unsigned)(want < 4096 ? want : 4096), 256, 0, (cudaStream_t)stream>>>(offs, level, valid, mass, ek, ev,
+                                                                                               lens, (size_t)rows * cap, rows);
     GKV_LAUNCH_CHECK();
     return GKV_OK;
 }

@@ -479,7 +479,8 @@ class PagedLayerCache:
         dev = self.device
         with on(dev):
             rc = self.lib.gkv_paged_clear_table(self.offs.data_ptr(), self.level.data_ptr(), self.valid.data_ptr(),
-                                                self.mass.data_ptr(), self.lens.data_ptr(), self.rows, self.cap, _stream(dev))
+                                                self.mass.data_ptr(), self.ek.data_ptr(), self.ev.data_ptr(), self.lens.data_ptr(),
+                                                self.rows, self.cap, _stream(dev))
         _lib.check(rc, "gkv_paged_clear_table")
 
     def dequantise(self):

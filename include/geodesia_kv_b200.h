@@ -332,9 +332,9 @@ int gkv_paged_demote_entries(uint8_t *pool, const int64_t *off_old, const int32_
 int gkv_paged_open_blocks(const int64_t *flat, const int64_t *offs, int n, int64_t *tab_offs,
                           int32_t *tab_level, float *tab_mass, float *tab_ek, float *tab_ev, void *stream);
 
-/* A table without blocks: offs -1, level, valid, mass and the row lengths 0. */
-int gkv_paged_clear_table(int64_t *offs, int32_t *level, int32_t *valid, float *mass, int32_t *lens,
-                          int rows, int cap, void *stream);
+/* A table without blocks: offs -1; level, valid, mass, the radii and the row lengths 0. */
+int gkv_paged_clear_table(int64_t *offs, int32_t *level, int32_t *valid, float *mass, float *ek, float *ev,
+                          int32_t *lens, int rows, int cap, void *stream);
 
 /* Distortion table and rung allocation (gkv_block_distortion, gkv_allocate_ragged) straight from a block
  * table: the ladder index follows from level, the blocks in use and what must stay exact (the first

@@ -385,3 +385,22 @@ def test_other_shapes_through_the_pool(oracle, D, group, Hq, Hkv):
     assert np.abs(mass.cpu().numpy()[:, :wm.shape[1]] - wm).max() <= 1e-5
     assert pool.bytes_in_use == layer.bytes_in_pool()
     assert (layer.level_h[layer.level_h > 0] < 16).any()
+
+
+def test_a_second_batch_starts_without_the_first_ones_radii():
+    from geodesia_kv_b200.paged import PagedLayerCache, PagedPool
+    layer = PagedLayerCache(PagedPool(64 << 20, 128, 32), 2, 2)
+    k, v = dense_batch(3, 2, 2, 30 * P, 128)
+
+    def batch(lengths):
+        layer.prefill(k, v, lengths)
+        assert layer.maintain(3.0, mass=power_law_mass(layer)) > 0
+        return layer.ek.clone(), layer.ev.clone()
+
+    first = batch([30 * P, 21 * P])
+    layer.release()
+    assert not layer.ek.any() and not layer.ev.any()
+    again = batch([30 * P, 21 * P])
+    assert all(torch.equal(a, b) and a.any() for a, b in zip(first, again))
+    layer.release()
+    assert not torch.cat([t[:, 12:] for t in batch([12 * P, 9 * P])]).any()      # shorter rows: nothing of the longer ones
