@@ -467,10 +467,10 @@ class PagedLayerCache:
         return float(bits.sum()) / max(1, int(used.sum()) * 2 * BLOCK * self.D)
 
     def release(self) -> None:
-        """Give every slot back to the pool."""
-        used = np.arange(self.cap)[None, :] < self._row_blocks()[:, None]
+        """Give every slot back to the pool, also those that :meth:`reserve` opened and no token has reached."""
+        held = self.offs_h >= 0
         for rung in LADDER:
-            sel = used & (self.level_h == rung) & (self.offs_h >= 0)
+            sel = held & (self.level_h == rung)
             if sel.any():
                 self.pool.free(rung, self.offs_h[sel])
         self.offs_h[:] = -1

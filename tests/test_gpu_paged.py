@@ -404,3 +404,21 @@ def test_a_second_batch_starts_without_the_first_ones_radii():
     assert all(torch.equal(a, b) and a.any() for a, b in zip(first, again))
     layer.release()
     assert not torch.cat([t[:, 12:] for t in batch([12 * P, 9 * P])]).any()      # shorter rows: nothing of the longer ones
+
+
+def test_release_returns_slots_that_no_token_reached():
+    from geodesia_kv_b200.paged import PagedLayerCache, PagedPool
+    pool = PagedPool(64 << 20, 128, 32)
+    layer = PagedLayerCache(pool, 2, 2)
+    k, v = dense_batch(4, 2, 2, 5 * P, 128)
+    layer.prefill(k, v, [5 * P, 3 * P + 7])
+    layer.maintain(3.0, mass=power_law_mass(layer), window=64)
+    layer.reserve(200)                                          # three or four blocks per row, none of them written
+    layer.release()
+    assert pool.bytes_in_use == 0 and pool.bytes_reserved == 0
+    layer.prefill(k, v)
+    layer.reserve(100)
+    for _ in range(70):
+        layer.append_device(k[:, :, :1].contiguous(), v[:, :, :1].contiguous())     # the host has not counted these
+    layer.release()
+    assert pool.bytes_in_use == 0 and int(layer.status.item()) == 0
