@@ -228,7 +228,12 @@ class PagedLayerCache:
         total = int(row_nblk.sum())
         row_of = np.repeat(np.arange(self.rows), row_nblk)                        # row of every block
         blk_of = np.arange(total) - np.repeat(np.cumsum(row_nblk) - row_nblk, row_nblk)
-        slots = self.pool.alloc(16, total)
+        if int(self.offs_h.max(initial=-1)) < 0:
+            slots = self.pool.alloc(16, total)
+        else:                                                                     # slots reserved earlier are used first
+            slots = self.offs_h[row_of, blk_of]
+            fresh = np.nonzero(slots < 0)[0]
+            slots[fresh] = self.pool.alloc(16, fresh.size)
         src_off = (row_of * T + blk_of * BLOCK) * D
         nvalid = np.minimum(BLOCK, lengths[rows_b[row_of]] - blk_of * BLOCK).astype(np.int32)
         self.offs_h[row_of, blk_of] = slots

@@ -422,3 +422,17 @@ def test_release_returns_slots_that_no_token_reached():
         layer.append_device(k[:, :, :1].contiguous(), v[:, :, :1].contiguous())     # the host has not counted these
     layer.release()
     assert pool.bytes_in_use == 0 and int(layer.status.item()) == 0
+
+
+def test_prefill_uses_slots_that_were_reserved_before_it():
+    from geodesia_kv_b200.paged import PagedLayerCache, PagedPool
+    pool = PagedPool(64 << 20, 128, 32)
+    layer = PagedLayerCache(pool, 2, 2)
+    k, v = dense_batch(5, 2, 2, 5 * P, 128)
+    layer.reserve(3 * P)
+    layer.prefill(k, v)
+    assert pool.bytes_in_use == layer.bytes_in_pool() == 2 * 2 * 5 * pool.slot[16]
+    got_k, got_v = layer.dequantise()
+    assert torch.equal(got_k.view_as(k), k.float()) and torch.equal(got_v.view_as(v), v.float())
+    layer.release()
+    assert pool.bytes_in_use == 0
