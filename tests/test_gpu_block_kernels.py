@@ -169,6 +169,26 @@ def test_table_form_plans_as_the_array_form():
         assert step or layer.apply_demotion(got.cpu().numpy()) > 0
 
 
+@pytest.mark.parametrize("B,Hkv", [(3, 2), (1, 1)])
+def test_plan_takes_mass_in_every_shape(B, Hkv):
+    """What the decode calls return, flat values, wider rows, other types and strides: the plan of the plain (rows, nb)."""
+    from geodesia_kv_b200.paged import PagedLayerCache, PagedPool
+    nb, rows = 20, B * Hkv
+    layer = PagedLayerCache(PagedPool(64 << 20, 64, 32), B, Hkv)
+    k = torch.randn(B, Hkv, nb * 64, 64, device="cuda", dtype=torch.bfloat16)
+    layer.prefill(k, k)
+    m = torch.rand(rows, nb, device="cuda")
+    want = layer.plan_demotion(4.0, mass=m)
+    assert (want > 0).any()
+    wide, spread = torch.rand(rows, nb + 9, device="cuda"), torch.zeros(rows, nb, 3, device="cuda")
+    wide[:, :nb], spread[..., 1] = m, m
+    for form in (m.view(B, Hkv, nb), m.view(-1), m.view(B, Hkv * nb), wide, wide[:, :nb], m.double(), wide.double(), m.t().contiguous().t(), spread[..., 1]):
+        assert torch.equal(layer.plan_demotion(4.0, mass=form), want), (tuple(form.shape), form.stride())
+    assert torch.equal(layer.plan_demotion(4.0, mass=m[:1]), layer.plan_demotion(4.0, mass=m[0]))
+    with pytest.raises(RuntimeError):
+        layer.plan_demotion(4.0, mass=m[:, :-1])
+
+
 @pytest.mark.parametrize("B,Hq,Hkv", [(1, 7, 1), (200, 8, 8), (120, 8, 2), (64, 64, 8), (3, 12, 4)])
 def test_merge_widths_and_mass(oracle, B, Hq, Hkv):
     """From 7 to 4096 output rows the merge runs with 8, 2, 4, 1 and 8 warps per row; the mass takes 1 to 8 heads per cache row.
