@@ -73,10 +73,10 @@ class _Extension:
         return int(word.value)
 
     # -- per-stream scratch and per-metadata block lists ------------------------------------
-    def _workspace(self, dev, need: int) -> torch.Tensor:
+    def _workspace(self, dev, need: int, stream: Optional[int] = None) -> torch.Tensor:
         if torch.cuda.is_current_stream_capturing():
             return torch.empty(need, dtype=torch.uint8, device=dev)        # lives in the graph's own pool
-        key = (dev.index, _stream(dev))
+        key = (dev.index, _stream(dev) if stream is None else stream)
         ws = self._workspaces.get(key)
         if ws is None or ws.numel() < need:
             ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=dev)
@@ -86,27 +86,34 @@ class _Extension:
     def invalidate_plans(self) -> None:
         self._plans.clear()
 
-    def _plan(self, offs, level, valid, meta_rows: int, nb: int):
+    def _plan(self, offs, level, valid, meta_rows: int, nb: int, stream: Optional[int] = None):
         if nb == 0:
             return None
         key = (offs.data_ptr(), offs._version, level.data_ptr(), level._version, valid.data_ptr(), valid._version,
                meta_rows, nb)
-        hit = self._plans.get(key)
-        if hit is not None:
-            # also while a CUDA graph is being captured: the graph then replays over the lists made for the
-            # metadata as it stood at capture (whoever edits level/valid/offs in place captures again)
+        made = self._plans.get(key)
+        here = _stream(level.device) if stream is None else stream
+        if made is not None:
             self._plans.move_to_end(key)
-            return hit[0]
+            # Lists belong to the stream they were made on: another one would have to wait for them, and their memory
+            # for it, so it makes its own.
+            hit = made[0].get(here)
+            if hit is not None:
+                return hit
         if torch.cuda.is_current_stream_capturing():
-            return None                                                    # built inside the workspace by the call
+            # A graph replays over the lists made before its capture, for the metadata as it stood then (whoever edits
+            # level/valid/offs in place captures again); without any, the call builds them inside its workspace.
+            return None if made is None else next(iter(made[0].values()))
         plan = torch.empty(self.lib.gkv_decode_plan_bytes(meta_rows, nb), dtype=torch.uint8, device=level.device)
         rc = self.lib.gkv_decode_build_plan(offs.data_ptr(), level.data_ptr(), valid.data_ptr(), plan.data_ptr(),
-                                            meta_rows, nb, _stream(level.device))
+                                            meta_rows, nb, here)
         _lib.check(rc, "gkv_decode_build_plan")
-        # the entry keeps the metadata tensors alive, so their addresses cannot be handed to other tensors
-        self._plans[key] = (plan, offs, level, valid)
-        while len(self._plans) > self.PLAN_CACHE_ENTRIES:
-            self._plans.popitem(last=False)
+        if made is None:
+            # the entry keeps the metadata tensors alive, so their addresses cannot be handed to other tensors
+            made = self._plans[key] = ({}, offs, level, valid)
+            while len(self._plans) > self.PLAN_CACHE_ENTRIES:
+                self._plans.popitem(last=False)
+        made[0][here] = plan
         return plan
 
     # -- the reference entry point ------------------------------------------------
@@ -169,9 +176,10 @@ class _Extension:
         klo, kstep, vlo, vstep = (t.contiguous() for t in (klo, kstep, vlo, vstep))
         if mass:
             with on(dev):
+                stream = _stream(dev)
                 need = self.lib.gkv_decode_mass_workspace_bytes(B, Hq, Hkv, D, nb, int(group))
-                ws = self._workspace(dev, need)
-                plan = self._plan(offs, level, valid, meta_rows, nb)
+                ws = self._workspace(dev, need, stream)
+                plan = self._plan(offs, level, valid, meta_rows, nb, stream)
                 out = torch.empty((B, Hq, D), dtype=torch.float32, device=dev)
                 bm = torch.empty((B, Hkv, nb), dtype=torch.float32, device=dev)       # every entry is written
                 rc = 0
@@ -179,20 +187,21 @@ class _Extension:
                     rc = self.lib.gkv_mixed_attn_decode_mass(
                         q.data_ptr(), _ptr(data), _ptr(offs), _ptr(klo), _ptr(kstep), _ptr(vlo), _ptr(vstep),
                         _ptr(level), _ptr(valid), out.data_ptr(), bm.data_ptr(), _ptr(plan), ws.data_ptr(), ws.numel(),
-                        B, Hq, Hkv, D, nb, int(block), int(group), data.size(-1), meta_rows, _stream(dev))
+                        B, Hq, Hkv, D, nb, int(block), int(group), data.size(-1), meta_rows, stream)
                 else:
                     out.zero_()
             _lib.check(rc, "gkv_mixed_attn_decode_mass")
             return out, bm
         with on(dev):
+            stream = _stream(dev)
             need = self.lib.gkv_decode_workspace_bytes(B, Hq, Hkv, D, nb)
-            ws = self._workspace(dev, need)
-            plan = self._plan(offs, level, valid, meta_rows, nb)
+            ws = self._workspace(dev, need, stream)
+            plan = self._plan(offs, level, valid, meta_rows, nb, stream)
             out = torch.empty((B, Hq, D + 2) if partial else (B, Hq, D), dtype=torch.float32, device=dev)
             rc = self.lib.gkv_mixed_attn_decode_planned(
                 q.data_ptr(), _ptr(data), _ptr(offs), _ptr(klo), _ptr(kstep), _ptr(vlo), _ptr(vstep),
                 _ptr(level), _ptr(valid), out.data_ptr(), _ptr(plan), 1 if partial else 0, ws.data_ptr(), ws.numel(),
-                B, Hq, Hkv, D, nb, int(block), int(group), data.size(-1), meta_rows, _stream(dev))
+                B, Hq, Hkv, D, nb, int(block), int(group), data.size(-1), meta_rows, stream)
         _lib.check(rc, "gkv_mixed_attn_decode")
         return out, ws
 

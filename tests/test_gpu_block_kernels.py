@@ -309,3 +309,35 @@ def test_decode_ring_of_short_and_hand_copied_blocks(oracle, D, group, Hq):
     got = get_ext().mixed_attn_decode(torch.from_numpy(q).cuda(), *kernel_args(t, c)).cpu().numpy()
     assert np.abs(got - oracle.mixed_attn_decode(q, *oracle_args(c))).max() < 5e-5
     assert get_ext().decode_status() == 0
+
+
+def test_decode_from_two_streams():
+    """Block lists made on one stream and used on another before they are finished; eager work before, between and
+    after calls whose launches overlap."""
+    from geodesia_kv_b200.cuda_ext import get_ext
+    from geodesia_kv_b200.pack_layout import pack_cache
+    ext, D, group, Hkv, nb = get_ext(), 128, 32, 2, 70
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    k = torch.randn(2, Hkv, nb * 64 - 9, D, device="cuda", generator=gen)
+    level = torch.from_numpy(LADDER).cuda()[torch.randint(0, 5, (2, Hkv, nb), device="cuda", generator=gen)]
+    q = torch.randn(2, 8, D, device="cuda", generator=gen) * D ** -0.5
+    cache = pack_cache(k, k, level, group)
+    scales = [0.25 * (i + 1) for i in range(12)]
+    want = [ext.mixed_attn_decode(q * x, *cache.kernel_args()) + x for x in scales]
+    fresh = pack_cache(k, k, level, group)                       # the same metadata at new addresses: no lists yet
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    got = [[], []]
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(100_000_000)                           # the lists wait behind some 50 ms of other work
+    for x in scales:
+        for s, outs in zip(streams, got):
+            with torch.cuda.stream(s):
+                scaled = q * x
+                out = ext.mixed_attn_decode(scaled, *fresh.kernel_args())
+                scaled.fill_(float("nan"))                       # queued behind the call that reads it
+                outs.append(out.add_(x))
+    torch.cuda.synchronize()
+    for outs in got:
+        for a, b in zip(outs, want):
+            assert (a - b).abs().max() < 5e-5                    # the kernel's stated error; the order of records varies
