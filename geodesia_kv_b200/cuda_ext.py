@@ -25,6 +25,7 @@ Differences a caller can rely on:
 from __future__ import annotations
 
 import os
+import weakref
 from collections import OrderedDict
 from typing import Any, Optional
 
@@ -50,6 +51,7 @@ class _Extension:
         self.lib = _lib.load()
         self._plans: "OrderedDict[tuple, tuple]" = OrderedDict()
         self._workspaces: dict = {}
+        self._captured: dict = {}          # lists that a captured graph reads, by address
 
     # -- kernel choice (tensor-core kernel by shape, or always the CUDA-core kernel) ------
     def set_decode_kernel(self, which: str) -> None:
@@ -73,8 +75,8 @@ class _Extension:
         return int(word.value)
 
     # -- per-stream scratch and per-metadata block lists ------------------------------------
-    def _workspace(self, dev, need: int, stream: Optional[int] = None) -> torch.Tensor:
-        if torch.cuda.is_current_stream_capturing():
+    def _workspace(self, dev, need: int, stream: Optional[int] = None, capturing: Optional[bool] = None) -> torch.Tensor:
+        if torch.cuda.is_current_stream_capturing() if capturing is None else capturing:
             return torch.empty(need, dtype=torch.uint8, device=dev)        # lives in the graph's own pool
         key = (dev.index, _stream(dev) if stream is None else stream)
         ws = self._workspaces.get(key)
@@ -86,24 +88,33 @@ class _Extension:
     def invalidate_plans(self) -> None:
         self._plans.clear()
 
-    def _plan(self, offs, level, valid, meta_rows: int, nb: int, stream: Optional[int] = None):
+    def _plan(self, offs, level, valid, meta_rows: int, nb: int, stream: Optional[int] = None,
+              capturing: Optional[bool] = None):
         if nb == 0:
             return None
         key = (offs.data_ptr(), offs._version, level.data_ptr(), level._version, valid.data_ptr(), valid._version,
                meta_rows, nb)
-        made = self._plans.get(key)
         here = _stream(level.device) if stream is None else stream
+        capturing = torch.cuda.is_current_stream_capturing() if capturing is None else capturing
+        made = self._plans.get(key)
         if made is not None:
             self._plans.move_to_end(key)
             # Lists belong to the stream they were made on: another one would have to wait for them, and their memory
             # for it, so it makes its own.
             hit = made[0].get(here)
-            if hit is not None:
+            if hit is not None and not capturing:
                 return hit
-        if torch.cuda.is_current_stream_capturing():
+        if capturing:
             # A graph replays over the lists made before its capture, for the metadata as it stood then (whoever edits
             # level/valid/offs in place captures again); without any, the call builds them inside its workspace.
-            return None if made is None else next(iter(made[0].values()))
+            if made is None:
+                return None
+            plan = next(iter(made[0].values())) if hit is None else hit
+            if plan.data_ptr() not in self._captured:
+                # the graph reads them for as long as it lives, which is no longer than the metadata it was captured with
+                self._captured[plan.data_ptr()] = plan
+                weakref.finalize(level, self._captured.pop, plan.data_ptr(), None)
+            return plan
         plan = torch.empty(self.lib.gkv_decode_plan_bytes(meta_rows, nb), dtype=torch.uint8, device=level.device)
         rc = self.lib.gkv_decode_build_plan(offs.data_ptr(), level.data_ptr(), valid.data_ptr(), plan.data_ptr(),
                                             meta_rows, nb, here)
@@ -176,10 +187,10 @@ class _Extension:
         klo, kstep, vlo, vstep = (t.contiguous() for t in (klo, kstep, vlo, vstep))
         if mass:
             with on(dev):
-                stream = _stream(dev)
+                stream, capturing = _stream(dev), torch.cuda.is_current_stream_capturing()
                 need = self.lib.gkv_decode_mass_workspace_bytes(B, Hq, Hkv, D, nb, int(group))
-                ws = self._workspace(dev, need, stream)
-                plan = self._plan(offs, level, valid, meta_rows, nb, stream)
+                ws = self._workspace(dev, need, stream, capturing)
+                plan = self._plan(offs, level, valid, meta_rows, nb, stream, capturing)
                 out = torch.empty((B, Hq, D), dtype=torch.float32, device=dev)
                 bm = torch.empty((B, Hkv, nb), dtype=torch.float32, device=dev)       # every entry is written
                 rc = 0
@@ -193,10 +204,10 @@ class _Extension:
             _lib.check(rc, "gkv_mixed_attn_decode_mass")
             return out, bm
         with on(dev):
-            stream = _stream(dev)
+            stream, capturing = _stream(dev), torch.cuda.is_current_stream_capturing()
             need = self.lib.gkv_decode_workspace_bytes(B, Hq, Hkv, D, nb)
-            ws = self._workspace(dev, need, stream)
-            plan = self._plan(offs, level, valid, meta_rows, nb, stream)
+            ws = self._workspace(dev, need, stream, capturing)
+            plan = self._plan(offs, level, valid, meta_rows, nb, stream, capturing)
             out = torch.empty((B, Hq, D + 2) if partial else (B, Hq, D), dtype=torch.float32, device=dev)
             rc = self.lib.gkv_mixed_attn_decode_planned(
                 q.data_ptr(), _ptr(data), _ptr(offs), _ptr(klo), _ptr(kstep), _ptr(vlo), _ptr(vstep),

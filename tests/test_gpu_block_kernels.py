@@ -341,3 +341,40 @@ def test_decode_from_two_streams():
     for outs in got:
         for a, b in zip(outs, want):
             assert (a - b).abs().max() < 5e-5                    # the kernel's stated error; the order of records varies
+
+
+@pytest.mark.parametrize("same_stream", [True, False])
+def test_a_graph_keeps_the_block_lists_it_was_captured_with(monkeypatch, same_stream):
+    """Lists that leave the cache of recent metadata stay for a graph that reads them, until its metadata goes."""
+    import gc
+    from geodesia_kv_b200.cuda_ext import get_ext
+    from geodesia_kv_b200.pack_layout import pack_cache
+    ext, nb, D = get_ext(), 40, 64
+    monkeypatch.setattr(ext, "PLAN_CACHE_ENTRIES", 2)
+    gc.collect()
+    before = len(ext._captured)
+    level = torch.from_numpy(LADDER).cuda()[torch.randint(0, 5, (1, 2, nb), device="cuda")]
+    k, q = torch.randn(1, 2, nb * 64, D, device="cuda"), torch.randn(1, 4, D, device="cuda") * D ** -0.5
+    caches = [pack_cache(k, k, level, 32) for _ in range(4)]
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = ext.mixed_attn_decode(q, *caches[0].kernel_args())
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side if same_stream else torch.cuda.Stream()):
+        out = ext.mixed_attn_decode(q, *caches[0].kernel_args())
+    assert len(ext._captured) == before + 1
+    kept = list(ext._captured.values())[-1]
+    lists = kept.clone()
+    for c in caches[1:]:
+        ext.mixed_attn_decode(q, *c.kernel_args())               # the cache of lists holds two entries
+    assert not any(kept is plan for entry in ext._plans.values() for plan in entry[0].values())
+    torch.cuda.synchronize()
+    assert torch.equal(kept, lists)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (out - want).abs().max() < 5e-5
+    del graph, caches, c, out
+    ext.invalidate_plans()
+    gc.collect()
+    assert len(ext._captured) == before
