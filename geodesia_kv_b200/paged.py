@@ -97,6 +97,12 @@ class PagedPool:
         st[top:top + offs.size] = offs
         self._top[rung] = top + offs.size
 
+    def _histogram(self, n: int) -> bool:
+        """Whether to count n slots' slabs by a histogram over all slabs: quicker while the pool has no more slabs than slots
+        are moved (256 slots of 60 slabs: 1.3 us against 1.8 for an indexed add), ruinous when it is long (16 of 110,000:
+        73 against 2.5)."""
+        return self.n_slabs <= n
+
     def alloc(self, rung: int, n: int) -> np.ndarray:
         """Offsets of n free slots of a rung (int64)."""
         if n <= 0:
@@ -117,7 +123,11 @@ class PagedPool:
         top = self._top[rung]
         out = self._stack[rung][top - n:top][::-1].copy()
         self._top[rung] = top - n
-        self._slab_live += np.bincount(out // self.slab_bytes, minlength=self.n_slabs)
+        slabs = out // self.slab_bytes
+        if self._histogram(n):
+            self._slab_live += np.bincount(slabs, minlength=self.n_slabs)
+        else:
+            np.add.at(self._slab_live, slabs, 1)
         self.bytes_in_use += n * size
         self.peak_bytes_in_use = max(self.peak_bytes_in_use, self.bytes_in_use)
         return out
@@ -130,20 +140,23 @@ class PagedPool:
         slabs = offs // self.slab_bytes
         if np.any(self._slab_rung[slabs] != rung):
             raise ValueError("a freed offset does not belong to a slab of that rung")
-        gone = np.bincount(slabs, minlength=self.n_slabs)
-        self._slab_live -= gone
+        if self._histogram(slabs.size):
+            gone = np.bincount(slabs, minlength=self.n_slabs)
+            self._slab_live -= gone
+            empty = np.nonzero((gone > 0) & (self._slab_live == 0))[0]
+        else:
+            np.subtract.at(self._slab_live, slabs, 1)
+            idle = slabs[self._slab_live[slabs] == 0]
+            empty = np.unique(idle) if idle.size else idle
         self.bytes_in_use -= offs.size * self.slot[rung]
         self._push(rung, offs)
-        empty = np.nonzero((gone > 0) & (self._slab_live == 0))[0]
         if empty.size:
+            self._slab_rung[empty] = 0
             top = self._top[rung]
             st = self._stack[rung][:top]
-            idle = np.zeros(self.n_slabs, dtype=bool)
-            idle[empty] = True
-            keep = st[~idle[st // self.slab_bytes]]
+            keep = st[self._slab_rung[st // self.slab_bytes] == rung]       # the stack's other slots are of slabs in use
             self._stack[rung][:keep.size] = keep
             self._top[rung] = keep.size
-            self._slab_rung[empty] = 0
             self._free_slabs.extend(empty[::-1].tolist())
 
 

@@ -61,3 +61,70 @@ def test_exhaustion_and_wrong_rung_are_errors():
         pool.free(8, a[:1])
     pool.free(16, a)
     assert pool.alloc(4, 144).size == 144
+
+
+class PlainPool:
+    """The bookkeeping one slot at a time."""
+
+    def __init__(self, slot, slab_bytes, n_slabs):
+        self.slot, self.slab, self.free_slabs = slot, slab_bytes, list(range(n_slabs - 1, -1, -1))
+        self.stack, self.rung, self.live = {r: [] for r in slot}, {}, {}
+
+    def alloc(self, rung, n):
+        while len(self.stack[rung]) < n:
+            s = self.free_slabs.pop()
+            self.rung[s], self.live[s] = rung, 0
+            self.stack[rung] += [s * self.slab + i * self.slot[rung] for i in reversed(range(self.slab // self.slot[rung]))]
+        out = [self.stack[rung].pop() for _ in range(n)]
+        for o in out:
+            self.live[o // self.slab] += 1
+        return out
+
+    def free(self, rung, offs):
+        for o in offs:
+            self.live[o // self.slab] -= 1
+        self.stack[rung] += offs
+        for s in sorted({o // self.slab for o in offs if self.live[o // self.slab] == 0}, reverse=True):
+            self.stack[rung] = [o for o in self.stack[rung] if o // self.slab != s]
+            self.free_slabs.append(s)
+            del self.rung[s], self.live[s]
+
+
+@pytest.mark.parametrize("slabs", [30, 400, 20000])      # below, among and far above the numbers of slots moved
+def test_bookkeeping_is_the_plain_one_for_short_and_long_pools(slabs):
+    from geodesia_kv_b200.paged import LADDER, PagedPool
+    pool = PagedPool(slabs * 1474560, 128, 32, device="meta")
+    plain = PlainPool(pool.slot, pool.slab_bytes, slabs)
+    rng = np.random.default_rng(slabs)
+    held = {r: [] for r in LADDER}
+    for _ in range(300):
+        rung = int(rng.choice(LADDER))
+        n = int(rng.choice([1, 7, 60, 150]))
+        if rng.random() < 0.55 and sum(map(len, held.values())) < 800:
+            got = pool.alloc(rung, n).tolist()
+            assert got == plain.alloc(rung, n)
+            held[rung] += got
+        elif held[rung]:
+            offs = [held[rung].pop(int(rng.integers(len(held[rung])))) for _ in range(min(n, len(held[rung])))]
+            pool.free(rung, np.array(offs))
+            plain.free(rung, offs)
+        assert pool._free_slabs == plain.free_slabs
+        assert pool._stack[rung][:pool._top[rung]].tolist() == plain.stack[rung]
+        assert pool.slots_in_use(rung) == len(held[rung])
+    assert pool.bytes_in_use == sum(len(h) * pool.slot[r] for r, h in held.items())
+
+
+def test_moving_a_few_slots_does_not_cost_the_length_of_the_pool():
+    """Scratch of a few slots' worth, in a pool of 160 GB whose per-slab arrays are 880 KB long."""
+    import tracemalloc
+    from geodesia_kv_b200.paged import PagedPool
+    pool = PagedPool(110_000 * 1474560, 128, 32, device="meta")
+    pool.alloc(16, 500)
+    tracemalloc.start()
+    try:
+        for _ in range(3):
+            pool.free(16, pool.alloc(16, 16))
+            pool.free(16, pool.alloc(16, 100))                  # some slabs empty
+        assert tracemalloc.get_traced_memory()[1] < 64 << 10
+    finally:
+        tracemalloc.stop()
