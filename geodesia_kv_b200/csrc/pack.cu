@@ -938,19 +938,36 @@ __global__ void __launch_bounds__(1024) layout_rows_kernel(const int32_t* __rest
     if (tid == 0) row_bytes[blockIdx.x] = run;
 }
 
-// Rows are as wide as the longest: what lies behind a row's last block reads as zeros.
-__global__ void zero_tails_kernel(uint8_t* data, const int64_t* row_bytes, int64_t stride, int rows) {
-    for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+// Rows are as wide as the longest: what lies behind a row's last block reads as zeros.  Bound: the stores.  A row's tail
+// is cut among gridDim.x CTAs (its length is known on the device only, so each finds its share, or that there is none).
+// pack_cache of two rows of 1M tokens, D = 128, one exact and one at 2 bits (470 MB of tail): 7950 us with one CTA per
+// row, 528 us; rows of equal bytes 513 and 507 us.
+__global__ void __launch_bounds__(256) zero_tails_kernel(uint8_t* data, const int64_t* row_bytes, int64_t stride, int rows) {
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int row = blockIdx.y; row < rows; row += gridDim.y) {
         uint8_t* d = data + (size_t)row * stride;
         const int64_t lo = row_bytes[row], mid = (lo + 15) & ~(int64_t)15;
         if (((reinterpret_cast<uintptr_t>(d) | (uintptr_t)stride) & 15) == 0) {
-            for (int64_t i = lo + threadIdx.x; i < mid && i < stride; i += blockDim.x) d[i] = 0;
-            for (int64_t i = mid + 16 * (int64_t)threadIdx.x; i < stride; i += 16 * (int64_t)blockDim.x)
+            for (int64_t i = lo + first; i < mid && i < stride; i += step) d[i] = 0;
+            for (int64_t i = mid + 16 * first; i < stride; i += 16 * step)
                 *reinterpret_cast<uint4*>(d + i) = make_uint4(0, 0, 0, 0);
         } else {
-            for (int64_t i = lo + threadIdx.x; i < stride; i += blockDim.x) d[i] = 0;
+            for (int64_t i = lo + first; i < stride; i += step) d[i] = 0;
         }
     }
+}
+
+// CTAs per row: four per SM over all rows, none with less than 16 KB to look after.
+static int launch_zero_tails(uint8_t* data, const int64_t* row_bytes, int64_t stride, int rows, cudaStream_t stream) {
+    int dev = 0, sms = 0;
+    GKV_CUDA_TRY(cudaGetDevice(&dev));
+    GKV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t most = (stride + 16383) / 16384, share = 4 * sms / rows;
+    const int64_t x = most < share ? most : share;
+    zero_tails_kernel<<<dim3((unsigned)(x > 1 ? x : 1), (unsigned)(rows < 65535 ? rows : 65535)), 256, 0, stream>>>(data, row_bytes, stride,
+                                                                                                              rows);
+    GKV_LAUNCH_CHECK();
+    return GKV_OK;
 }
 
 }  // namespace gkv
@@ -999,8 +1016,7 @@ int gkv_pack_rows(const void* k, const void* v, int src_dtype, int64_t T, uint8_
     using namespace gkv;
     if (T <= 0 || (T + kP - 1) / kP != nb || rows <= 0 || stride_bh < 0) return GKV_E_SHAPE;
     if (!valid || !row_bytes || !data) return GKV_E_NULL;
-    zero_tails_kernel<<<rows < 65535 ? rows : 65535, 128, 0, (cudaStream_t)stream>>>(data, row_bytes, stride_bh, rows);
-    GKV_LAUNCH_CHECK();
+    if (const int rc = launch_zero_tails(data, row_bytes, stride_bh, rows, (cudaStream_t)stream)) return rc;
     return pack_impl(k, v, src_dtype, T, data, offs, klo, kstep, vlo, vstep, level, valid, rows, nb, 0, nb, D, block, group,
                      stride_bh, rows, stream);
 }

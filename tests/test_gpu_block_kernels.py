@@ -93,6 +93,36 @@ def test_layout_of_rows(nb):
         assert not cache.data[behind].any()
 
 
+def test_tails_of_unequal_rows():
+    """Rows of very different rungs: the tails are zeros, whatever the row count, and cost no more than filling the
+    whole buffer a few times over (one CTA per row takes some hundred times as long)."""
+    from geodesia_kv_b200.pack_layout import layout_offsets, pack_cache
+    for rows, nb in ((1, 3), (2, 2048), (9, 50), (700, 2)):
+        level = torch.full((1, rows, nb), 1, dtype=torch.int32, device="cuda")
+        level[:, rows // 2] = 16
+        level[:, 0, ::2] = 2
+        k = torch.randn(1, rows, nb * 64, 128, device="cuda", dtype=torch.bfloat16)
+        junk = torch.full((1, rows, nb * 32768), 255, dtype=torch.uint8, device="cuda")
+        del junk                                                 # the buffer that follows is likely to hold it
+        cache = pack_cache(k, k, level, 32)
+        _, row_bytes = layout_offsets(level, 128)
+        for r in range(rows if rows < 10 else 20):
+            assert not cache.data[0, r, int(row_bytes[0, r]):].any(), (rows, r)
+        if nb < 2048:
+            continue
+        def best(fn):
+            times = []
+            for _ in range(8):
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+                fn()
+                b.record()
+                torch.cuda.synchronize()
+                times.append(a.elapsed_time(b))
+            return min(times)
+        assert best(lambda: pack_cache(k, k, level, 32)) < 10 * best(lambda: cache.data.fill_(0))
+
+
 @pytest.mark.parametrize("D,group", [(128, 32), (128, 16), (128, 64), (64, 16), (64, 64), (96, 32)])
 @pytest.mark.parametrize("value_weight", [0.0, 0.5])
 def test_distortion_edges(oracle, D, group, value_weight):
