@@ -1016,9 +1016,11 @@ int gkv_pack_rows(const void* k, const void* v, int src_dtype, int64_t T, uint8_
     using namespace gkv;
     if (T <= 0 || (T + kP - 1) / kP != nb || rows <= 0 || stride_bh < 0) return GKV_E_SHAPE;
     if (!valid || !row_bytes || !data) return GKV_E_NULL;
-    if (const int rc = launch_zero_tails(data, row_bytes, stride_bh, rows, (cudaStream_t)stream)) return rc;
-    return pack_impl(k, v, src_dtype, T, data, offs, klo, kstep, vlo, vstep, level, valid, rows, nb, 0, nb, D, block, group,
-                     stride_bh, rows, stream);
+    // the blocks first: what they refuse leaves the buffer as it was
+    if (const int rc = pack_impl(k, v, src_dtype, T, data, offs, klo, kstep, vlo, vstep, level, valid, rows, nb, 0, nb, D, block, group,
+                                 stride_bh, rows, stream))
+        return rc;
+    return launch_zero_tails(data, row_bytes, stride_bh, rows, (cudaStream_t)stream);
 }
 
 int gkv_layout_rows(const int32_t* level, int64_t* offs, int32_t* valid, int64_t* row_bytes, int64_t T, int rows, int nb,

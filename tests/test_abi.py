@@ -55,6 +55,16 @@ def test_argument_validation_happens_before_any_cuda_call():
     assert lib.gkv_mixed_attn_decode(*small, 1, 4, 4, 64, 8, 64, 32, 1024, 1, None) == -4
 
 
+def test_packing_rows_validates_before_it_clears_their_tails():
+    from geodesia_kv_b200 import _lib
+    lib = _lib.load()
+    one = ctypes.c_void_p(256)      # never dereferenced, as above
+    def pack(k=one, dtype=1, T=512, nb=8, D=64, block=64, group=32):
+        return lib.gkv_pack_rows(k, one, dtype, T, one, one, one, one, one, one, one, one, one, 4, nb, D, block, group, 1024, None)
+    assert pack(block=32) == -1 and pack(nb=9) == -2 and pack(D=60) == -2 and pack(group=24) == -2
+    assert pack(dtype=3) == -6 and pack(k=None) == -3
+
+
 def test_get_ext_follows_the_reference_contract(monkeypatch):
     import torch
     from geodesia_kv_b200 import cuda_ext
