@@ -972,10 +972,10 @@ static int launch_zero_tails(uint8_t* data, const int64_t* row_bytes, int64_t st
 
 }  // namespace gkv
 
-static int pack_impl(const void* k, const void* v, int src_dtype, int64_t T, uint8_t* data, const int64_t* offs,
-                     void* klo, void* kstep, void* vlo, void* vstep, const int32_t* level,
-                     const int32_t* valid, int rows, int nb, int b_lo, int b_hi, int D, int block,
-                     int group, int64_t stride_bh, int meta_rows, void* stream) {
+// What a pack of rows does not take.
+static int pack_refuses(const void* k, const void* v, int src_dtype, const uint8_t* data, const int64_t* offs, const void* klo,
+                        const void* kstep, const void* vlo, const void* vstep, const int32_t* level, int rows, int nb, int b_lo,
+                        int b_hi, int D, int block, int group, int meta_rows) {
     using namespace gkv;
     if (block != kP) return GKV_E_BLOCK;
     if (rows <= 0 || nb <= 0 || D <= 0 || D > kMaxD || D % 8 || group <= 0) return GKV_E_SHAPE;
@@ -983,6 +983,17 @@ static int pack_impl(const void* k, const void* v, int src_dtype, int64_t T, uin
     if (meta_rows != 1 && meta_rows != rows) return GKV_E_SHAPE;
     if (b_lo < 0 || b_hi > nb || b_lo > b_hi || src_dtype < 0 || src_dtype > 2) return GKV_E_ARG;
     if (!k || !v || !data || !offs || !klo || !kstep || !vlo || !vstep || !level) return GKV_E_NULL;
+    return GKV_OK;
+}
+
+static int pack_impl(const void* k, const void* v, int src_dtype, int64_t T, uint8_t* data, const int64_t* offs,
+                     void* klo, void* kstep, void* vlo, void* vstep, const int32_t* level,
+                     const int32_t* valid, int rows, int nb, int b_lo, int b_hi, int D, int block,
+                     int group, int64_t stride_bh, int meta_rows, void* stream) {
+    using namespace gkv;
+    if (const int rc = pack_refuses(k, v, src_dtype, data, offs, klo, kstep, vlo, vstep, level, rows, nb, b_lo, b_hi, D, block, group,
+                                    meta_rows))
+        return rc;
     if (b_lo == b_hi) return GKV_OK;
     PackParams p;
     p.k = k; p.v = v; p.src_dtype = src_dtype; p.data = data; p.offs = offs;
@@ -1016,11 +1027,12 @@ int gkv_pack_rows(const void* k, const void* v, int src_dtype, int64_t T, uint8_
     using namespace gkv;
     if (T <= 0 || (T + kP - 1) / kP != nb || rows <= 0 || stride_bh < 0) return GKV_E_SHAPE;
     if (!valid || !row_bytes || !data) return GKV_E_NULL;
-    // the blocks first: what they refuse leaves the buffer as it was
-    if (const int rc = pack_impl(k, v, src_dtype, T, data, offs, klo, kstep, vlo, vstep, level, valid, rows, nb, 0, nb, D, block, group,
-                                 stride_bh, rows, stream))
+    if (const int rc = pack_refuses(k, v, src_dtype, data, offs, klo, kstep, vlo, vstep, level, rows, nb, 0, nb, D, block, group, rows))
         return rc;
-    return launch_zero_tails(data, row_bytes, stride_bh, rows, (cudaStream_t)stream);
+    // the tails first: they run while the pack is being launched
+    if (const int rc = launch_zero_tails(data, row_bytes, stride_bh, rows, (cudaStream_t)stream)) return rc;
+    return pack_impl(k, v, src_dtype, T, data, offs, klo, kstep, vlo, vstep, level, valid, rows, nb, 0, nb, D, block, group,
+                     stride_bh, rows, stream);
 }
 
 int gkv_layout_rows(const int32_t* level, int64_t* offs, int32_t* valid, int64_t* row_bytes, int64_t T, int rows, int nb,
