@@ -54,7 +54,8 @@ constexpr int kCombineThreads = 256;
 // records, and the NW states are merged through shared memory — the same recurrence at both levels.
 // KPER = channels per lane (D <= 32 * KPER): head dims up to 128 take the instantiation with half the
 // registers, which lets half as many more CTAs sit on an SM (the kernel is bound by the latency of its few
-// loads per warp, i.e. by how many CTAs are resident).
+// loads per warp, i.e. by how many CTAs are resident).  One warp per row: 26 CTAs per SM, for which 72 registers (and
+// 24 bytes of spills) are what it gets.
 template <int NW, int KPER = kMaxD / 32>
 __global__ void __launch_bounds__(NW * 32, NW == 1 ? 26 : 1) combine_kernel(CombineParams p) {
     __shared__ float sm_m[NW], sm_l[NW], sm_o[NW][32 * KPER];
@@ -81,9 +82,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 1 ? 26 : 1) combine_kernel(Comb
     const int s_lo = p.segs > 1 ? (int)blockIdx.y * p.per_seg : 0;
     const int s_hi = p.segs > 1 ? min(parts, s_lo + p.per_seg) : parts;
     const size_t out_row = p.segs > 1 ? (size_t)blockIdx.y * gridDim.x + orow : (size_t)orow;
-    // kBatch records at a time: all their loads are issued before the first is merged (the merge
-    // itself is a serial recurrence, and one load round trip per record made this kernel
-    // latency-bound); the order of the merge is unchanged.
+    // kBatch records at a time: all their loads are issued before the first is merged (one load round
+    // trip per record made this kernel latency-bound).
     constexpr int kBatch = KPER <= 4 ? 8 : 4;         // as many as fit the registers
     for (int s0 = s_lo + warp; s0 < s_hi; s0 += NW * kBatch) {
         float ms[kBatch], ls[kBatch], v[kBatch][kPer];
@@ -574,16 +574,35 @@ static int launch_plan(const int32_t* level, const int32_t* valid, const int64_t
     return GKV_OK;
 }
 
-// Warps per output row of a merge: as many as keep all rows resident at once (about 26 warps of 80 registers per
-// SM), 8 at most.  The kernel is bound by the latency of one row's loads; a second wave of CTAs costs all of it again, which is
-// more than a warp's longer share of the records.  Together with the query warp's shorter item set-up: 256 ragged
-// sequences (4096 rows of about 60 records) 412 -> 404 us per call, 32 x 16k tokens (1024 rows) 230.5 -> 223 us.
+// CTAs of an instantiation of the merge that the current device holds at once (asked once per device).
+template <int NW>
+static long combine_resident() {
+    static int per_sm[kMaxDevices] = {0};
+    const int dev = current_device();
+    if (dev < 0) return 0;
+    if (per_sm[dev] == 0) {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, combine_kernel<NW, 4>, NW * 32, 0) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            return 0;
+        }
+        per_sm[dev] = n;
+    }
+    return (long)per_sm[dev] * sm_count();
+}
+
+// Warps per output row of a merge: as many as keep all rows resident at once, 8 at most.  The kernel is bound by the
+// latency of one row's loads; a second wave of CTAs costs all of it again, which is more than a warp's longer share of the
+// records.  Today that is 2 CTAs of 8 warps per SM, 5 of 4 or 11 of 2 (87 registers), i.e. up to 296, 740 and 1628 rows on
+// 148 SMs, and one warp per row beyond.  Against widths that leave a second wave (8 warps at 400 rows, 4 at 896): 50
+// sequences of 2k tokens with 8 heads 33.6 -> 31.7 us per call, of 16k 115.4 -> 112.3, one of 1M tokens with 28 heads (32
+// slices per head) 208.7 -> 206.9; 900 rows of 64 blocks 77.7 -> 78.3.
 static int launch_combine(const CombineParams& c, dim3 grid, cudaStream_t stream) {
-    const long rows = (long)grid.x * grid.y, warps = 26L * sm_count();
+    const long rows = (long)grid.x * grid.y;
     if (c.D > 128) return launch_overlapped(combine_kernel<8>, grid, kCombineThreads, 0, stream, c);
-    if (rows * 8 <= warps) return launch_overlapped(combine_kernel<8, 4>, grid, 256, 0, stream, c);
-    if (rows * 4 <= warps) return launch_overlapped(combine_kernel<4, 4>, grid, 128, 0, stream, c);
-    if (rows * 2 <= warps) return launch_overlapped(combine_kernel<2, 4>, grid, 64, 0, stream, c);
+    if (rows <= combine_resident<8>()) return launch_overlapped(combine_kernel<8, 4>, grid, 256, 0, stream, c);
+    if (rows <= combine_resident<4>()) return launch_overlapped(combine_kernel<4, 4>, grid, 128, 0, stream, c);
+    if (rows <= combine_resident<2>()) return launch_overlapped(combine_kernel<2, 4>, grid, 64, 0, stream, c);
     return launch_overlapped(combine_kernel<1, 4>, grid, 32, 0, stream, c);
 }
 

@@ -219,9 +219,11 @@ def test_plan_takes_mass_in_every_shape(B, Hkv):
         layer.plan_demotion(4.0, mass=m[:, :-1])
 
 
-@pytest.mark.parametrize("B,Hq,Hkv", [(1, 7, 1), (200, 8, 8), (120, 8, 2), (64, 64, 8), (3, 12, 4)])
+@pytest.mark.parametrize("B,Hq,Hkv", [(1, 7, 1), (200, 8, 8), (120, 8, 2), (64, 64, 8), (3, 12, 4), (40, 16, 2),
+                                      (296, 1, 1), (297, 1, 1), (740, 1, 1), (741, 1, 1), (1628, 1, 1), (1629, 1, 1)])
 def test_merge_widths_and_mass(oracle, B, Hq, Hkv):
-    """From 7 to 4096 output rows the merge runs with 8, 2, 4, 1 and 8 warps per row; the mass takes 1 to 8 heads per cache row.
+    """From 7 to 4096 output rows the merge runs with 8, 4, 2 and 1 warps per row, on 148 SMs up to 296, 740 and 1628 rows and
+    beyond; the mass takes 1 to 8 heads per cache row.
 
     Both are sums of fp32 products whose operands carry 22 bits: 5e-5 absolute is what the kernel states for outputs of
     order one, masses are sums of weights that add up to one."""
