@@ -52,6 +52,7 @@ SIGNATURES = {
     "gkv_paged_demote_entries": (_i, [_vp] * 10 + [_i] * 4 + [_vp]),
     "gkv_paged_open_blocks": (_i, [_vp, _vp, _i] + [_vp] * 6),
     "gkv_paged_clear_table": (_i, [_vp] * 7 + [_i, _i, _vp]),
+    "gkv_paged_plan_ratio_bytes": (_sz, [C.POINTER(_f), _i, _i]),
     "gkv_paged_plan_demotion": (_i, [_vp] * 5 + [_i64, C.POINTER(_f), C.c_double, _i, _i, _f, _f, _vp, _vp, _vp] + [_i] * 6 + [_vp]),
     "gkv_paged_unpack_blocks": (_i, [_vp] * 5 + [_i] * 4 + [_vp]),
     "gkv_paged_append_token": (_i, [_vp, _vp, _i] + [_vp] * 5 + [_i] * 4 + [_vp]),

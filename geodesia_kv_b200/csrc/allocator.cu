@@ -296,9 +296,12 @@ static bool whole_bits(const float (&bits)[5]) {
     return true;
 }
 
+// Which of the two kernels: one block per thread and ratios in registers, or ratios in memory.
+static bool allocates_in_registers(int nb, const float (&bits)[5]) { return nb <= kAllocThreads && whole_bits(bits); }
+
 template <bool TABLE>
 static int launch_allocate(const AllocParams& p, int problems, cudaStream_t stream) {
-    if (p.nb <= kAllocThreads && whole_bits(p.bits)) {
+    if (allocates_in_registers(p.nb, p.bits)) {
         const int threads = (p.nb + 31) & ~31;
         allocate_small_kernel<TABLE><<<problems, threads, 0, stream>>>(p);
     } else {
@@ -667,6 +670,13 @@ int gkv_block_distortion(const uint8_t* data, const int64_t* offs, const int32_t
     return launch_distortion(p, rows, (cudaStream_t)stream);
 }
 
+size_t gkv_paged_plan_ratio_bytes(const float* bits_host, int rows, int nb) {
+    if (!bits_host || rows <= 0 || nb <= 0) return 0;
+    float bits[5];
+    for (int i = 0; i < 5; ++i) bits[i] = bits_host[i];
+    return gkv::allocates_in_registers(nb, bits) ? 0 : (size_t)rows * nb * 4 * sizeof(float);
+}
+
 int gkv_paged_plan_demotion(const uint8_t* pool, const int64_t* offs, const int32_t* level, const int32_t* lens,
                             const float* mass, int64_t mass_stride, const float* bits_host, double target_per_block,
                             int sink_blocks, int window_blocks, float mass_power, float value_weight, float* E,
@@ -678,16 +688,16 @@ int gkv_paged_plan_demotion(const uint8_t* pool, const int64_t* offs, const int3
     if (nb == 0) return GKV_OK;
     if (mass_stride < nb) return GKV_E_ARG;
     if (!pool || !offs || !level || !lens || !mass || !bits_host || !E || !tgt_idx) return GKV_E_NULL;
+    const bool in_registers = gkv_paged_plan_ratio_bytes(bits_host, rows, nb) == 0;
+    if (!in_registers && !ratio) return GKV_E_NULL;
     DistParams d;
     d.data = pool; d.offs = offs; d.level = level; d.E = E; d.nb = nb; d.D = D; d.group = group;
     d.per_row_meta = 1; d.value_weight = value_weight; d.stride_bh = 0; d.tab_stride = cap;
     if (const int rc = launch_distortion(d, rows, (cudaStream_t)stream)) return rc;
     AllocParams p;
     p.mass = mass; p.E = E; p.idx = nullptr; p.hot = nullptr; p.target_bits = nullptr;
-    p.ratio = ratio; p.tgt = tgt_idx; p.mass_power = mass_power; p.nb = nb; p.nb_of = nullptr;
+    p.ratio = in_registers ? nullptr : ratio; p.tgt = tgt_idx; p.mass_power = mass_power; p.nb = nb; p.nb_of = nullptr;
     for (int i = 0; i < 5; ++i) p.bits[i] = bits_host[i];
-    if (nb <= kAllocThreads && whole_bits(p.bits)) p.ratio = nullptr;      // the kernel that keeps ratios in registers
-    else if (!ratio) return GKV_E_NULL;
     p.level = level; p.lens = lens; p.mass_stride = mass_stride; p.level_stride = cap;
     p.sink_blocks = sink_blocks; p.window_blocks = window_blocks; p.target_per_block = target_per_block;
     return launch_allocate<true>(p, rows, (cudaStream_t)stream);

@@ -169,6 +169,7 @@ class PagedLayerCache:
         self.D, self.group, self.device = pool.D, pool.group, pool.device
         self.lib = _lib.load()
         self.cap = 0
+        self._bits = None
         self.len_h = np.zeros(B, dtype=np.int64)                     # tokens per sequence (host mirror)
         self.offs_h = np.full((self.rows, 0), -1, dtype=np.int64)
         self.level_h = np.zeros((self.rows, 0), dtype=np.int32)          # 0 = no block here
@@ -408,29 +409,39 @@ class PagedLayerCache:
               (b >= nbr - max(1, (window + BLOCK - 1) // BLOCK))
         return (hot & (b < nbr)).to(torch.uint8).contiguous()
 
+    def _ladder_bits(self):
+        """Bits of a block at each rung, as the library takes them."""
+        if self._bits is None:
+            from .policies import ladder_bits
+            self._bits = (C.c_float * 5)(*ladder_bits(BLOCK, self.D, self.group))
+        return self._bits
+
     def plan_demotion(self, budget_bits: float, sinks: int = 4, window: int = 128, mass_power: float = 1.0,
                       value_weight: float = 0.0, mass: torch.Tensor | None = None) -> torch.Tensor:
         """Run the distortion and allocator kernels over every row; returns the target ladder index
         (rows, nb) int32 ON THE DEVICE (nothing is read back here).  ``mass``: (rows, nb) or wider, any shape of
         rows * nb values in that order (the (B, Hkv, nb) of the decode calls), or what broadcasts to (rows, nb)."""
-        from .policies import ladder_bits
         nb, dev, rows, D = self.nb, self.device, self.rows, self.D
         m = self.mass if mass is None else mass
-        if m.dim() != 2 or m.shape[0] != rows:
+        shape = m.shape
+        if len(shape) != 2 or shape[0] != rows:
             m = m.reshape(rows, nb) if m.numel() == rows * nb else m.expand(rows, nb)
-        if m.dtype != torch.float32 or m.stride(-1) != 1 or m.stride(0) < nb or m.shape[1] < nb:
-            m = (m[:, :nb] if m.shape[1] > nb else m.expand(rows, nb)).to(torch.float32).contiguous()
+            shape = m.shape
+        apart, step = m.stride()
+        if m.dtype != torch.float32 or step != 1 or apart < nb or shape[1] < nb:
+            m = (m[:, :nb] if shape[1] > nb else m.expand(rows, nb)).to(torch.float32).contiguous()
+            apart = nb                               # a single row may have any stride
         E = torch.empty(rows, nb, 5, dtype=torch.float32, device=dev)
-        ratio = torch.empty(rows, nb, 4, dtype=torch.float32, device=dev) if nb > 512 else None     # longer rows keep them in memory
         tgt = torch.empty(rows, nb, dtype=torch.int32, device=dev)
-        bits = (C.c_float * 5)(*ladder_bits(BLOCK, D, self.group))
+        bits = self._ladder_bits()
+        need = self.lib.gkv_paged_plan_ratio_bytes(bits, rows, nb)
+        ratio = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         with on(dev):
             rc = self.lib.gkv_paged_plan_demotion(self.pool.data.data_ptr(), self.offs.data_ptr(), self.level.data_ptr(),
-                                                  self.lens.data_ptr(), m.data_ptr(),
-                                                  max(m.stride(0), nb), bits,      # a single row may have any stride
+                                                  self.lens.data_ptr(), m.data_ptr(), apart, bits,
                                                   float(budget_bits * 2.0 * BLOCK * D), max(1, (sinks + BLOCK - 1) // BLOCK),
                                                   max(1, (window + BLOCK - 1) // BLOCK), float(mass_power), float(value_weight),
-                                                  E.data_ptr(), ratio.data_ptr() if nb > 512 else None, tgt.data_ptr(), rows, nb,
+                                                  E.data_ptr(), ratio.data_ptr() if need else None, tgt.data_ptr(), rows, nb,
                                                   self.cap, D, BLOCK, self.group, _stream(dev))
         _lib.check(rc, "gkv_paged_plan_demotion")
         return tgt

@@ -340,8 +340,9 @@ int gkv_paged_clear_table(int64_t *offs, int32_t *level, int32_t *valid, float *
  * table: the ladder index follows from level, the blocks in use and what must stay exact (the first
  * sink_blocks, the open block, its predecessor, the last window_blocks; policies.py:677-681) from lens, the
  * budget of a row is target_per_block bits times its blocks in use.  mass: rows mass_stride floats apart.
- * E (rows, nb, 5) and ratio (rows, nb, 4) are scratch (ratio may be NULL for nb <= 512 and whole bits);
- * tgt_idx (rows, nb) int32.                                                                            */
+ * E (rows, nb, 5) floats and ratio are scratch (ratio: gkv_paged_plan_ratio_bytes bytes, NULL where that is
+ * 0: short rows on a ladder of whole bits); tgt_idx (rows, nb) int32.                                  */
+size_t gkv_paged_plan_ratio_bytes(const float *bits_host, int rows, int nb);
 int gkv_paged_plan_demotion(const uint8_t *pool, const int64_t *offs, const int32_t *level,
                             const int32_t *lens, const float *mass, int64_t mass_stride,
                             const float *bits_host, double target_per_block, int sink_blocks,

@@ -65,6 +65,18 @@ def test_packing_rows_validates_before_it_clears_their_tails():
     assert pack(dtype=3) == -6 and pack(k=None) == -3
 
 
+def test_the_library_says_what_scratch_a_plan_needs():
+    from geodesia_kv_b200 import _lib
+    lib = _lib.load()
+    whole, split = (ctypes.c_float * 5)(1024, 512, 256, 128, 64), (ctypes.c_float * 5)(1024, 512, 256.5, 128, 64)
+    assert lib.gkv_paged_plan_ratio_bytes(whole, 3, 512) == 0
+    assert lib.gkv_paged_plan_ratio_bytes(whole, 3, 513) == 3 * 513 * 16
+    assert lib.gkv_paged_plan_ratio_bytes(split, 3, 5) == 3 * 5 * 16
+    one = ctypes.c_void_p(256)      # never dereferenced: the missing scratch is refused before any launch
+    tail = (one, None, one, 3, 5, 5, 64, 64, 32, None)
+    assert lib.gkv_paged_plan_demotion(one, one, one, one, one, 5, split, 1e5, 1, 2, 1.0, 0.0, *tail) == -3
+
+
 def test_get_ext_follows_the_reference_contract(monkeypatch):
     import torch
     from geodesia_kv_b200 import cuda_ext

@@ -168,13 +168,14 @@ def test_allocate_sizes(oracle, nb, whole):
         assert np.array_equal(ratio[r].cpu().numpy(), ref)
 
 
-def test_table_form_plans_as_the_array_form():
-    """The allocator's inputs derived from a ragged block table, against the same inputs spelled out."""
+@pytest.mark.parametrize("D,group,Hkv,lengths", [(128, 32, 2, [1, 64, 65, 640, 1999]), (64, 32, 1, [33000, 500, 32768]), (64, 16, 2, [32769])])
+def test_table_form_plans_as_the_array_form(D, group, Hkv, lengths):
+    """The allocator's inputs derived from a ragged block table, against the same inputs spelled out; rows beyond 512 blocks
+    keep their ratios in memory."""
     import ctypes as C
     from geodesia_kv_b200 import _lib, policies
     from geodesia_kv_b200.paged import PagedLayerCache, PagedPool
-    lib, D, group, B, Hkv = _lib.load(), 128, 32, 5, 2
-    lengths = [1, 64, 65, 640, 1999]
+    lib, B = _lib.load(), len(lengths)
     layer = PagedLayerCache(PagedPool(64 << 20, D, group), B, Hkv)
     k = torch.randn(B, Hkv, max(lengths), D, device="cuda", dtype=torch.bfloat16)
     layer.prefill(k, k, lengths)
