@@ -52,6 +52,11 @@ class PoolExhausted(RuntimeError):
 class PagedPool:
     """Byte pool with one free list per rung (host-side bookkeeping, device-side bytes)."""
 
+    # Slots moved are counted per slab by a histogram over all slabs in pools of up to so many (or of no more than the
+    # slots moved), by indexing the slabs touched in longer ones.  alloc and free of 64
+    # slots: 22.3 us against 23.1 at 500 slabs, 23.1 against 22.9 at 1000, 36.5 against 22.9 at 8000; of 16 at 110,000: 268 against 15.
+    HISTOGRAM_SLABS = 1000
+
     def __init__(self, capacity_bytes: int, D: int = 128, group: int = 32, device="cuda"):
         lib = _lib.load()
         self.D, self.group, self.device = D, group, torch.device(device)
@@ -97,12 +102,6 @@ class PagedPool:
         st[top:top + offs.size] = offs
         self._top[rung] = top + offs.size
 
-    def _histogram(self, n: int) -> bool:
-        """Whether to count n slots' slabs by a histogram over all slabs: quicker while the pool has no more slabs than slots
-        are moved (256 slots of 60 slabs: 1.3 us against 1.8 for an indexed add), ruinous when it is long (16 of 110,000:
-        73 against 2.5)."""
-        return self.n_slabs <= n
-
     def alloc(self, rung: int, n: int) -> np.ndarray:
         """Offsets of n free slots of a rung (int64)."""
         if n <= 0:
@@ -124,7 +123,7 @@ class PagedPool:
         out = self._stack[rung][top - n:top][::-1].copy()
         self._top[rung] = top - n
         slabs = out // self.slab_bytes
-        if self._histogram(n):
+        if self.n_slabs <= self.HISTOGRAM_SLABS or self.n_slabs <= n:
             self._slab_live += np.bincount(slabs, minlength=self.n_slabs)
         else:
             np.add.at(self._slab_live, slabs, 1)
@@ -140,7 +139,7 @@ class PagedPool:
         slabs = offs // self.slab_bytes
         if np.any(self._slab_rung[slabs] != rung):
             raise ValueError("a freed offset does not belong to a slab of that rung")
-        if self._histogram(slabs.size):
+        if self.n_slabs <= self.HISTOGRAM_SLABS or self.n_slabs <= slabs.size:
             gone = np.bincount(slabs, minlength=self.n_slabs)
             self._slab_live -= gone
             empty = np.nonzero((gone > 0) & (self._slab_live == 0))[0]
