@@ -574,21 +574,19 @@ static int launch_plan(const int32_t* level, const int32_t* valid, const int64_t
     return GKV_OK;
 }
 
-// CTAs of an instantiation of the merge that the current device holds at once (asked once per device).
+// CTAs of an instantiation of the merge that a device holds at once; asked once per device (0: it did not answer).
 template <int NW>
-static long combine_resident() {
-    static int per_sm[kMaxDevices] = {0};
-    const int dev = current_device();
-    if (dev < 0) return 0;
-    if (per_sm[dev] == 0) {
+static long combine_resident(int dev) {
+    static long kept[kMaxDevices] = {0};
+    if (dev >= 0 && kept[dev] == 0) {
         int n = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, combine_kernel<NW, 4>, NW * 32, 0) != cudaSuccess || n < 1) {
             cudaGetLastError();
             return 0;
         }
-        per_sm[dev] = n;
+        kept[dev] = (long)n * sm_count();
     }
-    return (long)per_sm[dev] * sm_count();
+    return dev < 0 ? 0 : kept[dev];
 }
 
 // Warps per output row of a merge: as many as keep all rows resident at once, 8 at most.  The kernel is bound by the
@@ -599,10 +597,11 @@ static long combine_resident() {
 // slices per head) 208.7 -> 206.9; 900 rows of 64 blocks 77.7 -> 78.3.
 static int launch_combine(const CombineParams& c, dim3 grid, cudaStream_t stream) {
     const long rows = (long)grid.x * grid.y;
+    const int dev = current_device();
     if (c.D > 128) return launch_overlapped(combine_kernel<8>, grid, kCombineThreads, 0, stream, c);
-    if (rows <= combine_resident<8>()) return launch_overlapped(combine_kernel<8, 4>, grid, 256, 0, stream, c);
-    if (rows <= combine_resident<4>()) return launch_overlapped(combine_kernel<4, 4>, grid, 128, 0, stream, c);
-    if (rows <= combine_resident<2>()) return launch_overlapped(combine_kernel<2, 4>, grid, 64, 0, stream, c);
+    if (rows <= combine_resident<8>(dev)) return launch_overlapped(combine_kernel<8, 4>, grid, 256, 0, stream, c);
+    if (rows <= combine_resident<4>(dev)) return launch_overlapped(combine_kernel<4, 4>, grid, 128, 0, stream, c);
+    if (rows <= combine_resident<2>(dev)) return launch_overlapped(combine_kernel<2, 4>, grid, 64, 0, stream, c);
     return launch_overlapped(combine_kernel<1, 4>, grid, 32, 0, stream, c);
 }
 
