@@ -344,6 +344,28 @@ def test_decode_ring_of_short_and_hand_copied_blocks(oracle, D, group, Hq):
     assert get_ext().decode_status() == 0
 
 
+@pytest.mark.parametrize("D,group,Hq", [(128, 32, 14), (64, 16, 6), (128, 64, 2)])
+def test_queries_at_any_address(oracle, D, group, Hq):
+    """Queries that start 4, 8 or 12 bytes off a 16-byte boundary are read element by element: the same numbers.
+
+    5e-5: the kernel's stated error for outputs of order one."""
+    from geodesia_kv_b200.cuda_ext import get_ext
+    from helpers import kernel_args, oracle_args
+    c = oracle_cache(oracle, 77 + D, 3, 2, 13, D, group, last_valid=21)
+    t = to_torch(c, "cuda")
+    q = np.random.default_rng(D).standard_normal((3, Hq, D), dtype=np.float32) * np.float32(D ** -0.5)
+    want = oracle.mixed_attn_decode(q, *oracle_args(c))
+    for shift in (1, 2, 3):
+        buf = torch.full((q.size + 8,), float("nan"), device="cuda")
+        buf[shift:shift + q.size] = torch.from_numpy(q).cuda().view(-1)
+        view = buf[shift:shift + q.size].view(3, Hq, D)
+        assert view.data_ptr() % 16 == 4 * shift
+        out, mass = get_ext().mixed_attn_decode_with_mass(view, *kernel_args(t, c))
+        for got in (out, get_ext().mixed_attn_decode(view, *kernel_args(t, c))):
+            assert np.abs(got.cpu().numpy() - want).max() < 5e-5, shift
+        assert (mass.sum(-1) - 1).abs().max() < 1e-5
+
+
 def test_decode_from_two_streams():
     """Block lists made on one stream and used on another before they are finished; eager work before, between and
     after calls whose launches overlap."""
