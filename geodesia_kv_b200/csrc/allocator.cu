@@ -431,8 +431,8 @@ __global__ void __launch_bounds__(kDistThreads) distortion_kernel(DistParams p) 
 
 // Head dims 64 and 128.  Every sum of the table is a serial fp32 chain in the reference's order (the allocator's
 // decisions hang on its last bit), so what bounds a block is the length of those chains, and what bounds the
-// launch is how many blocks an SM holds: the block stays in shared memory as the 16-bit rows it came as (17 KB),
-// three warps work on it, and ten CTAs fit an SM.  Columns first (a thread owns a channel pair: means, and the K
+// launch is how many blocks an SM holds: half a block at a time stays in shared memory as the 16-bit rows it came as
+// (17 KB at D = 128, 24 KB with the squares and means), three warps work on it, and nine CTAs fit an SM.  Columns first (a thread owns a channel pair: means, and the K
 // ranges by packed minimum and maximum, squared for the three rungs right away), then rows (a thread owns a token; rows are
 // padded by 16 bytes, so that eight lanes' 16-byte loads meet no bank twice) while the third warp adds up the
 // rungs' squares.  Square roots are monotonic and correctly rounded, so the maxima are taken over the sums.

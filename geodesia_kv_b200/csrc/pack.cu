@@ -10,9 +10,9 @@
 // are taken, code = clamp(rint((x-lo16)/step16), 0, 2^b-1), codes packed little-endian in the
 // byte (geodesia_kv/packed.py:23-40).  This file is compiled without fast-math.
 //
-// Head dims 64 and 128 (with a group that is a multiple of 8) take the register-resident path of
-// requantise.cuh instead: no fp32 tile in shared memory, every load of the block in flight at once.
-// The tile kernels below remain for the other shapes.
+// Head dims 64 and 128 (with the groups of rq::shape_ok) take the bodies of requantise.cuh
+// instead: 16-bit rows and packed blocks out of stages that bulk copies fill, fp32 rows held in registers.  The tile
+// kernels below remain for the other shapes.
 //
 // Two addressings share the block code: cache ROWS (a byte string per row, dense scale tensors
 // (rows, nb, ...) beside it — the reference's layout) and a paged POOL (every block an offset into
@@ -826,8 +826,7 @@ __global__ void __launch_bounds__(kStagedThreads, kCtasPerSM) staged_kernel(P p,
                 rq::work_sync();
             }
             rq::Job j;
-            j.src_kind = 0; j.ksrc = j.vsrc = nullptr; j.src_stride = 0; j.nvalid = kP; j.old_blk = nullptr; j.old_level = 0;
-            j.oklo = j.okstep = j.ovlo = j.ovstep = nullptr;
+            j.ksrc = j.vsrc = nullptr; j.src_stride = 0; j.nvalid = kP;
             j.dst = d.dst; j.level = d.level; j.klo = d.klo; j.kstep = d.kstep; j.vlo = d.vlo; j.vstep = d.vstep;
             j.zero_scales = d.zero_scales; j.ek = d.ek; j.ev = d.ev; j.group = group;
             rq::StagedSrc src;
@@ -862,19 +861,20 @@ __global__ void __launch_bounds__(rq::kThreads, 2) direct_kernel(P p, int group)
     if (threadIdx.x == 0) commit(p, (int)blockIdx.x);
     if (d.skip) return;
     rq::Job j;
-    j.src_kind = d.src_kind; j.ksrc = d.ksrc; j.vsrc = d.vsrc; j.src_stride = d.src_stride; j.nvalid = d.nvalid;
-    j.old_blk = d.old_blk; j.old_level = d.old_level; j.oklo = d.oklo; j.okstep = d.okstep; j.ovlo = d.ovlo; j.ovstep = d.ovstep;
+    j.ksrc = d.ksrc; j.vsrc = d.vsrc; j.src_stride = d.src_stride; j.nvalid = d.nvalid;
     j.dst = d.dst; j.level = d.level; j.klo = d.klo; j.kstep = d.kstep; j.vlo = d.vlo; j.vstep = d.vstep;
     j.zero_scales = d.zero_scales; j.ek = d.ek; j.ev = d.ev; j.group = group;
-    rq::requantise<D, false>(j, sm);
+    rq::requantise<D>(j, sm);
 }
 
 template <int D, class P>
 static int launch(const P& p, int n, int group, bool fp32_rows, cudaStream_t stream) {
-    if (fp32_rows) {
-        direct_kernel<D, P><<<n, rq::kThreads, 0, stream>>>(p, group);
-        GKV_LAUNCH_CHECK();
-        return GKV_OK;
+    if constexpr (!P::kPacked) {
+        if (fp32_rows) {
+            direct_kernel<D, P><<<n, rq::kThreads, 0, stream>>>(p, group);
+            GKV_LAUNCH_CHECK();
+            return GKV_OK;
+        }
     }
     int dev = 0, sms = 0;
     GKV_CUDA_TRY(cudaGetDevice(&dev));

@@ -1,15 +1,14 @@
-// Register-resident (re)quantisation of one 64-token block: the work of the pack and demote kernels
-// for head dims 64 and 128.
+// (Re)quantisation of one 64-token block: the work of the pack and demote kernels for head dims 64 and 128.
 //
-// A CTA of 256 threads takes one block.  Thread (tr, c8) holds eight consecutive channels
-// (8*c8 .. 8*c8+7) of the tokens tr, tr + ROWS, ... of K and of V — one 16-byte load per token half
-// when the source is bf16/fp16 — so all of a block's global loads are in flight at once and nothing
-// is staged as an fp32 tile in shared memory.  K ranges (per channel over `group` consecutive
-// tokens) are reduced in the thread, across the lanes that hold the same channels, and across warps
-// with integer min/max atomics on the order-preserving image of fp32 in shared memory; V ranges
-// (per token over `group` consecutive channels) live inside a few neighbouring lanes.  Codes come out
-// eight per thread and token, i.e. as one 8/4/2-byte store in exactly the block's byte order, and a
-// warp's stores cover whole token rows.
+// A CTA of 256 threads takes one block.  Two bodies:
+//   * `requantise`, for fp32 rows: thread (tr, c8) holds eight consecutive channels (8*c8 .. 8*c8+7) of the tokens tr,
+//     tr + ROWS, ... of K and of V in registers, so all of a block's global loads are in flight at once and no fp32 tile is
+//     staged in shared memory.  K ranges (per channel over `group` consecutive tokens) are reduced in the thread, across the
+//     lanes that hold the same channels, and across warps with integer min/max atomics on the order-preserving image of fp32
+//     in shared memory; V ranges (per token over `group` consecutive channels) live inside a few neighbouring lanes.
+//   * `requantise_staged`, for 16-bit rows and packed blocks, which a bulk copy has put into shared memory: passes read the
+//     source again instead of holding it, K ranges leave a warp as partial rows, V is worked out a quarter row per thread.
+// In both, codes come out eight per thread and token, as one 8/4/2-byte store in exactly the block's byte order.
 //
 // The arithmetic is the reference's (geodesia_kv/policies.py:61-77 quant_grouped, packed.py:14-44):
 // step = max(hi - lo, 1e-8) / qmax in fp32, lo and step rounded to fp16, code = clamp(rint((x - lo16)
@@ -25,15 +24,11 @@ namespace rq {
 constexpr int kThreads = 256;
 
 struct Job {
-    // source: dense rows (src_kind 0 fp32, 1 bf16, 2 fp16) or a packed block (src_kind 3)
-    int src_kind;
-    const void* ksrc;           // dense: first token row of the block
+    // source of `requantise`: dense fp32 rows (`requantise_staged` is told its source by a StagedSrc)
+    const void* ksrc;           // first token row of the block
     const void* vsrc;
-    int64_t src_stride;         // dense: elements between consecutive tokens
-    int nvalid;                 // dense: rows beyond nvalid repeat row nvalid - 1
-    const uint8_t* old_blk;     // packed source
-    int old_level;
-    const __half* oklo; const __half* okstep; const __half* ovlo; const __half* ovstep;
+    int64_t src_stride;         // elements between consecutive tokens
+    int nvalid;                 // rows beyond nvalid repeat row nvalid - 1
     // destination
     uint8_t* dst;
     int level;
@@ -99,108 +94,22 @@ __device__ __forceinline__ void unpack8_16(const uint4 r, bool bf, float* out) {
     }
 }
 
-// Eight channels (8*c8 ..) of token t of the K (which = 0) or V (which = 1) half of the source.
-template <int D>
+// Eight channels (8*c8 ..) of token t of the K (which = 0) or V (which = 1) rows, fp32.
 __device__ __forceinline__ void load8(const Job& j, int which, int t, int c8, float* out) {
-    if (j.src_kind != 3) {
-        const int ts = min(t, j.nvalid - 1);
-        const size_t e = (size_t)ts * (size_t)j.src_stride + 8 * c8;
-        const void* base = which ? j.vsrc : j.ksrc;
-        if (j.src_kind == 0) {
-            const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(base) + e);
-            if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-                const float4 a = p[0], b = p[1];
-                out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w;
-                out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) out[i] = static_cast<const float*>(base)[e + i];
-            }
-        } else {
-            const uint16_t* p = static_cast<const uint16_t*>(base) + e;
-            uint4 r;
-            if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-                r = *reinterpret_cast<const uint4*>(p);
-            } else {
-                r.x = p[0] | ((uint32_t)p[1] << 16); r.y = p[2] | ((uint32_t)p[3] << 16);
-                r.z = p[4] | ((uint32_t)p[5] << 16); r.w = p[6] | ((uint32_t)p[7] << 16);
-            }
-            unpack8_16(r, j.src_kind == 1, out);
-        }
-        return;
-    }
-    const int lv = j.old_level;
-    const uint8_t* half = j.old_blk + (which ? half_bytes(lv, D) : 0);
-    if (lv == 16) {
-        const uint16_t* p = reinterpret_cast<const uint16_t*>(half) + (size_t)t * D + 8 * c8;
-        uint4 r;
-        if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-            r = *reinterpret_cast<const uint4*>(p);
-        } else {
-            r.x = p[0] | ((uint32_t)p[1] << 16); r.y = p[2] | ((uint32_t)p[3] << 16);
-            r.z = p[4] | ((uint32_t)p[5] << 16); r.w = p[6] | ((uint32_t)p[7] << 16);
-        }
-        unpack8_16(r, true, out);
-        return;
-    }
-    if (lv == 1) {
-        const uint16_t* p = reinterpret_cast<const uint16_t*>(half) + 8 * c8;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) out[i] = half_bits_to_float(p[i]);
-        return;
-    }
-    // eight codes = lv bytes at byte (t*D + 8*c8) * lv / 8, little-endian
-    const uint8_t* cp = half + ((size_t)t * D + 8 * c8) * lv / 8;
-    unsigned long long bits = 0;
-    if ((reinterpret_cast<uintptr_t>(cp) & (uintptr_t)(lv - 1)) == 0) {          // lv bytes, naturally aligned
-        if (lv == 8) { const uint2 r = *reinterpret_cast<const uint2*>(cp); bits = ((unsigned long long)r.y << 32) | r.x; }
-        else if (lv == 4) bits = *reinterpret_cast<const uint32_t*>(cp);
-        else bits = *reinterpret_cast<const uint16_t*>(cp);
+    const float* x = static_cast<const float*>(which ? j.vsrc : j.ksrc) + (size_t)min(t, j.nvalid - 1) * (size_t)j.src_stride + 8 * c8;
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        const float4 a = reinterpret_cast<const float4*>(x)[0], b = reinterpret_cast<const float4*>(x)[1];
+        out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w;
+        out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
     } else {
-        for (int i = 0; i < lv; ++i) bits |= (unsigned long long)cp[i] << (8 * i);
-    }
-    const uint32_t mask = (1u << lv) - 1u;
-    const int kg = min(j.group, kP), vg = min(j.group, D);
-    if (which == 0) {
-        const int s0 = (t / kg) * D + 8 * c8;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float c = (float)((uint32_t)(bits >> (i * lv)) & mask);
-            out[i] = __fmaf_rn(c, __half2float(j.okstep[s0 + i]), __half2float(j.oklo[s0 + i]));
-        }
-    } else {
-        const int s = t * (D / vg) + (8 * c8) / vg;
-        const float st = __half2float(j.ovstep[s]), lo = __half2float(j.ovlo[s]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float c = (float)((uint32_t)(bits >> (i * lv)) & mask);
-            out[i] = __fmaf_rn(c, st, lo);
-        }
+        for (int i = 0; i < 8; ++i) out[i] = x[i];
     }
 }
 
-// One element (token t, channel d) of the source — the centroid path walks a channel token by token.
-template <int D>
+// One element (token t, channel d) of the rows — the centroid path walks a channel token by token.
 __device__ __forceinline__ float load1(const Job& j, int which, int t, int d) {
-    if (j.src_kind != 3) {
-        const size_t e = (size_t)min(t, j.nvalid - 1) * (size_t)j.src_stride + d;
-        const void* base = which ? j.vsrc : j.ksrc;
-        if (j.src_kind == 0) return static_cast<const float*>(base)[e];
-        const uint16_t h = static_cast<const uint16_t*>(base)[e];
-        return j.src_kind == 1 ? bf16_bits_to_float(h) : half_bits_to_float(h);
-    }
-    const int lv = j.old_level;
-    const uint8_t* half = j.old_blk + (which ? half_bytes(lv, D) : 0);
-    if (lv == 16) return bf16_bits_to_float(reinterpret_cast<const uint16_t*>(half)[t * D + d]);
-    if (lv == 1) return half_bits_to_float(reinterpret_cast<const uint16_t*>(half)[d]);
-    const float c = (float)unpack_code(half, t * D + d, lv);
-    const int kg = min(j.group, kP), vg = min(j.group, D);
-    if (which == 0) {
-        const int s = (t / kg) * D + d;
-        return __fmaf_rn(c, __half2float(j.okstep[s]), __half2float(j.oklo[s]));
-    }
-    const int s = t * (D / vg) + d / vg;
-    return __fmaf_rn(c, __half2float(j.ovstep[s]), __half2float(j.ovlo[s]));
+    return static_cast<const float*>(which ? j.vsrc : j.ksrc)[(size_t)min(t, j.nvalid - 1) * (size_t)j.src_stride + d];
 }
 
 // Eight codes of `lv` bits each -> lv bytes at `out` (byte order of the block).
@@ -225,16 +134,14 @@ __device__ __forceinline__ void store_codes(uint8_t* out, const uint32_t* c, int
     }
 }
 
-// Shapes this path takes: D 64 or 128, group a multiple of 8 that divides 64 and D (or exceeds them).
+// Shapes this path takes: D 64 or 128, group 16, 32, 64 or a multiple of 8 from D up.
 __host__ __device__ __forceinline__ bool shape_ok(int D, int group) {
     if (D != 64 && D != 128) return false;
     const int kg = group < kP ? group : kP, vg = group < D ? group : D;
     return group % 8 == 0 && kP % kg == 0 && D % vg == 0 && kP / kg <= 4;
 }
 
-// STAGED: the source sits in shared memory (a bulk copy put it there) and is simply read again by every
-// pass; otherwise the block's values are loaded once from global memory and held in registers.
-template <int D, bool STAGED>
+template <int D>
 __device__ void requantise(const Job& j, Shared& sm) {
     constexpr int OPR = D / 8;                 // channel octets per token row
     constexpr int ROWS = kThreads / OPR;       // token rows the CTA covers per pass
@@ -263,14 +170,14 @@ __device__ void requantise(const Job& j, Shared& sm) {
         if (tid < 2 * D) {
             float s = 0.f;
 #pragma unroll 8
-            for (int t = 0; t < kP; ++t) s = __fadd_rn(s, load1<D>(j, which, t, d));
+            for (int t = 0; t < kP; ++t) s = __fadd_rn(s, load1(j, which, t, d));
             mean = __half2float(__float2half_rn(__fdiv_rn(s, (float)kP)));
         }
         if (radii) for (int u = tid; u < 2 * kP; u += kThreads) sm.csum[u / kP][u % kP] = 0.f;
         __syncthreads();                       // every source byte has been read (the destination may overlap it)
         if (radii && tid < 2 * D) {
             for (int t = 0; t < kP; ++t) {
-                const float e = __fsub_rn(load1<D>(j, which, t, d), mean);
+                const float e = __fsub_rn(load1(j, which, t, d), mean);
                 float s = e * e;
 #pragma unroll
                 for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -293,19 +200,13 @@ __device__ void requantise(const Job& j, Shared& sm) {
 
     // ---- all loads first ------------------------------------------------------------------
     float kx[NI][8], vx[NI][8];
-    if constexpr (!STAGED) {
 #pragma unroll
-        for (int i = 0; i < NI; ++i) load8<D>(j, 0, tr + i * ROWS, c8, kx[i]);
+    for (int i = 0; i < NI; ++i) load8(j, 0, tr + i * ROWS, c8, kx[i]);
 #pragma unroll
-        for (int i = 0; i < NI; ++i) load8<D>(j, 1, tr + i * ROWS, c8, vx[i]);
-    }
+    for (int i = 0; i < NI; ++i) load8(j, 1, tr + i * ROWS, c8, vx[i]);
     auto values = [&](int which, int i, float* out) {
-        if constexpr (STAGED) {
-            load8<D>(j, which, tr + i * ROWS, c8, out);
-        } else {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) out[c] = which ? vx[i][c] : kx[i][c];
-        }
+        for (int c = 0; c < 8; ++c) out[c] = which ? vx[i][c] : kx[i][c];
     };
 
     if (lv == 16) {

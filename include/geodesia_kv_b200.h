@@ -86,8 +86,8 @@ int gkv_decode_launch_count(int B, int Hq, int Hkv, int D, int nb, int group, in
 int gkv_set_decode_kernel(int which);
 
 /* Blocks per work item of the tensor-core kernel for every later decode call of the process:
- * 0 = chosen from the problem size (about six items per multiprocessor, between 6 and 64 blocks),
- * 1..64 = fixed.  A tuning and test knob: results do not depend on it, only the split does (and with
+ * 0 = chosen from the problem size (one item per multiprocessor where that gives 6 to 64 blocks),
+ * 1..128 = fixed.  A tuning and test knob: results do not depend on it, only the split does (and with
  * it gkv_decode_workspace_bytes: query the size after setting the knob).  No counterpart in the
  * reference, whose split is fixed by its launcher (geodesia_kv_cuda/mixed_attn.cu:222-224).      */
 int gkv_set_decode_item_blocks(int blocks);
@@ -114,7 +114,7 @@ int gkv_mixed_attn_decode(const float *q, const uint8_t *data, const int64_t *of
 /* The tensor-core kernel walks every cache row's blocks sorted by rung.  Those lists depend only
  * on offs / level / valid, so a caller whose metadata is unchanged since the last call can build
  * them once (gkv_decode_build_plan into gkv_decode_plan_bytes(meta_rows, nb) bytes, 16-byte
- * aligned) and pass them to gkv_mixed_attn_decode_planned, which then launches one kernel less.
+ * aligned) and pass them to gkv_mixed_attn_decode_planned, which then only resets the call's counter.
  * `plan` may be NULL (the lists are then rebuilt inside the workspace, exactly as
  * gkv_mixed_attn_decode does); `partial` != 0 gives gkv_mixed_attn_decode_partial's output.
  * A stale plan (metadata changed since it was built) gives wrong results, not an error.
@@ -286,7 +286,7 @@ int gkv_maintenance_status(int *status_host);
  * at D = 128, g = 32).  Slot management (size-class free lists) is the caller's; these entry points
  * only read and write blocks.  Block offsets must be multiples of 16 (of 128 for the tiled copies
  * of the decode kernel to be used; other offsets fall back to a slower copy).  D in {64, 128},
- * group a multiple of 8; else GKV_E_SHAPE.  No counterpart in the reference's C++ (its kernel
+ * group 16, 32, 64 or a multiple of 8 from D up; else GKV_E_SHAPE.  No counterpart in the reference's C++ (its kernel
  * takes dense side tensors, mixed_attn.cu:202-216).                                          */
 size_t gkv_paged_block_bytes(int level, int D, int group);
 
