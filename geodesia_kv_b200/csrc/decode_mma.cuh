@@ -625,11 +625,11 @@ __device__ __forceinline__ bool produce_item(const Params& p, const TensorMaps& 
             ps.head = head;
             ps.used = used;
         }
-        // The copies below may land on scale planes and blocks that this warp's lanes once stored in the ring.  One fence
-        // per batch here, not one per block in the warps that release the slots: 32 x 16k tokens 221.6 against 222.4 us,
-        // one sequence of 1M tokens 208.3 against 211.7.
+        // The copies below may land on scale planes and blocks that this warp's lanes once stored in the ring: every lane has
+        // seen the slots released and fences before the copy it starts.  One fence per batch here, not one per block in the
+        // warps that release the slots: 32 x 16k tokens 221.6 against 222.4 us, one sequence of 1M tokens 208.3 against 211.7.
+        // (Fencing only where a slot held such bytes costs this warp's chain more than the fence: 226.8 us.)
         fence_before_bulk();
-        __syncwarp();
         const int my_seq = ps.seq_alloc + lane;
         const int my_slot = my_seq % kNSlot;
         uint4 cur = make_uint4(0, 0, 0, 0);
