@@ -110,15 +110,13 @@ class PagedPool:
         per_slab = self.slab_bytes // size
         need = max(0, -(-(n - self._top[rung]) // per_slab))
         if need:
-            took = [self._free_slabs.pop() for _ in range(min(need, len(self._free_slabs)))]
-            if took:
-                s = np.array(took, dtype=np.int64)
-                self._slab_rung[s] = rung
-                # pushed high to low, so low addresses are handed out first
-                self._push(rung, (s[:, None] * self.slab_bytes + np.arange(per_slab - 1, -1, -1, dtype=np.int64) * size).reshape(-1))
-            if len(took) < need:
+            if len(self._free_slabs) < need:             # refused with every slab where it was: smaller slots may still fit
                 raise PoolExhausted(f"pool of {self.capacity_bytes} bytes exhausted asking for {n} slots of rung {rung} "
                                     f"({self.bytes_in_use} bytes in use)")
+            s = np.array([self._free_slabs.pop() for _ in range(need)], dtype=np.int64)
+            self._slab_rung[s] = rung
+            # pushed high to low, so low addresses are handed out first
+            self._push(rung, (s[:, None] * self.slab_bytes + np.arange(per_slab - 1, -1, -1, dtype=np.int64) * size).reshape(-1))
         top = self._top[rung]
         out = self._stack[rung][top - n:top][::-1].copy()
         self._top[rung] = top - n
@@ -459,10 +457,17 @@ class PagedLayerCache:
         lv_old, lv_new = cur[r, b].copy(), new[r, b].astype(np.int32)
         off_old = self.offs_h[r, b].copy()
         off_new = np.empty(n, dtype=np.int64)
-        for rung in LADDER[1:]:
-            sel = np.nonzero(lv_new == rung)[0]
-            if sel.size:
-                off_new[sel] = self.pool.alloc(rung, sel.size)
+        taken = []
+        try:
+            for rung in LADDER[1:]:
+                sel = np.nonzero(lv_new == rung)[0]
+                if sel.size:
+                    off_new[sel] = self.pool.alloc(rung, sel.size)
+                    taken.append((rung, sel))
+        except PoolExhausted:
+            for rung, sel in taken:
+                self.pool.free(rung, off_new[sel])
+            raise
         dev = self.device
         with on(dev):
             staged, (old, new, at, lo, ln) = self._upload(off_old, off_new, r * self.cap + b, lv_old, lv_new)

@@ -128,3 +128,21 @@ def test_moving_a_few_slots_does_not_cost_the_length_of_the_pool():
         assert tracemalloc.get_traced_memory()[1] < 64 << 10
     finally:
         tracemalloc.stop()
+
+
+def test_running_out_leaves_the_pool_as_it_was():
+    from geodesia_kv_b200.paged import LADDER, PagedLayerCache, PagedPool, PoolExhausted
+    pool = PagedPool(4 * 1474560, 128, 32, device="cpu")         # four slabs
+    with pytest.raises(PoolExhausted):
+        pool.alloc(16, 5 * 45)
+    assert pool.bytes_reserved == 0                              # no slab stays behind for the slots refused
+    eights = pool.alloc(8, 3 * 80)
+    layer = PagedLayerCache(pool, 1, 1)
+    layer.offs_h[0, :40], layer.level_h[0, :40], layer.len_h[0] = pool.alloc(16, 40), 16, 40 * 64
+    pool.free(8, eights[:10])                                    # ten slots of 8 bits are free, a slab for 4 bits is not
+    before, tgt = pool.bytes_in_use, np.zeros((1, 40), dtype=np.int32)
+    tgt[0, 10:20], tgt[0, 20:30] = LADDER.index(8), LADDER.index(4)
+    with pytest.raises(PoolExhausted):
+        layer.apply_demotion(tgt)
+    assert pool.bytes_in_use == before and (layer.level_h[0, :40] == 16).all()
+    assert pool.alloc(8, 10).size == 10
