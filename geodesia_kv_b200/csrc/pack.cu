@@ -941,7 +941,7 @@ __global__ void __launch_bounds__(1024) layout_rows_kernel(const int32_t* __rest
 // Rows are as wide as the longest: what lies behind a row's last block reads as zeros.  Bound: the stores.  A row's tail
 // is cut among gridDim.x CTAs (its length is known on the device only, so each finds its share, or that there is none).
 // pack_cache of two rows of 1M tokens, D = 128, one exact and one at 2 bits (470 MB of tail): 7950 us with one CTA per
-// row, 528 us; rows of equal bytes 513 and 507 us.
+// row, 552 us; rows of equal bytes 513 and 506 us.
 __global__ void __launch_bounds__(256) zero_tails_kernel(uint8_t* data, const int64_t* row_bytes, int64_t stride, int rows) {
     const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
     for (int row = blockIdx.y; row < rows; row += gridDim.y) {
@@ -957,12 +957,13 @@ __global__ void __launch_bounds__(256) zero_tails_kernel(uint8_t* data, const in
     }
 }
 
-// CTAs per row: four per SM over all rows, none with less than 16 KB to look after.
+// CTAs per row: one per SM over all rows, none with less than 16 KB to look after.  (Four per SM: 526 instead of 552 us in
+// the case above, but 1 us more for 32 equal rows of 16k tokens, 150.6 against 149.5.)
 static int launch_zero_tails(uint8_t* data, const int64_t* row_bytes, int64_t stride, int rows, cudaStream_t stream) {
     int dev = 0, sms = 0;
     GKV_CUDA_TRY(cudaGetDevice(&dev));
     GKV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int64_t most = (stride + 16383) / 16384, share = 4 * sms / rows;
+    const int64_t most = (stride + 16383) / 16384, share = sms / rows;
     const int64_t x = most < share ? most : share;
     zero_tails_kernel<<<dim3((unsigned)(x > 1 ? x : 1), (unsigned)(rows < 65535 ? rows : 65535)), 256, 0, stream>>>(data, row_bytes, stride,
                                                                                                               rows);
