@@ -12,20 +12,23 @@ namespace gkv {
 int g_last_cuda_error = 0;
 
 // ---- LSE merge of split records -----------------------------------------------------------
-// Records are D+2 floats [m, l, o[D]].  Record s of output row r lives at
-//   rec + r_base(r) + s * stride_s.
+// A record is (m, l) and o[D].  Records that stay inside a call are kept in two planes, o[D] (whose rows start on 16 bytes,
+// so that the split kernel and the merge move four channels per access) and (m, l); the records a caller sees
+// (partial outputs) are D+2 floats [m, l, o[D]].  Both take D+2 floats each.
 // Follows geodesia_kv_cuda/mixed_attn.cu:171-200 (splits with m = -inf are skipped, the
 // denominator clamps at 1e-20); `normalise == 0` writes the merged record instead of o/l.
 struct CombineParams {
     const float* rec;
+    const float2* ml;    // (m, l) plane of the records in `rec`; null: `rec` holds [m, l, o[D]] records
     float* out;
+    float2* out_ml;      // segs > 1: (m, l) plane of the partial merges, whose o plane is `out`
     int parts, D;
-    int rep, nsplit;     // internal layout (rows, nsplit, rep, D+2) when rep > 0
-    int64_t stride_s;    // external layout (parts, rows, D+2) when rep == 0
+    int rep, nsplit;     // records (rows, nsplit, rep) when rep > 0
+    int64_t stride_s;    // records (parts, rows), this many apart, when rep == 0
     int normalise;
     const int* status;   // when non-null and non-zero the producing kernel gave up: poison the output
     int segs;            // > 1: blockIdx.y merges records [y*per_seg, (y+1)*per_seg) into record y of
-    int per_seg;         //      an external-layout (segs, rows, D+2) buffer (normalise must be 0)
+    int per_seg;         //      a (segs, rows) list of records
     float2* ml_out;      // optional, final level only: (M, L) of every output row (for the per-block softmax mass)
     // Internal layout written by the tensor-core kernel: a row's used item slots are a prefix of its
     // slots (the rest hold "empty" records), and how many are used follows from the row's rung-class
@@ -49,6 +52,41 @@ __device__ __forceinline__ int live_parts(const CombineParams& p, int orow) {
 
 constexpr int kCombineThreads = 256;
 
+// First record of an output row and the distance to its next one, counted in records.
+__device__ __forceinline__ void record_walk(const CombineParams& p, int orow, size_t& first, size_t& step) {
+    if (p.rep > 0) {
+        first = (size_t)(orow / p.rep) * p.nsplit * p.rep + orow % p.rep;
+        step = (size_t)p.rep;
+    } else {
+        first = (size_t)orow;
+        step = (size_t)p.stride_s;
+    }
+}
+
+// A lane's channels of a record: 4 * lane .. + 3 of every 128.
+template <int KPER, bool PLANES>
+__device__ __forceinline__ void load_record(const CombineParams& p, size_t r, int lane, float& m, float& l, float (&v)[KPER]) {
+    if (PLANES) {
+        const float2 ml = p.ml[r];
+        m = ml.x; l = ml.y;
+        const float4* o = reinterpret_cast<const float4*>(p.rec + r * p.D);      // D is a multiple of 8
+#pragma unroll
+        for (int j = 0; j < KPER / 4; ++j) {
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (128 * j + 4 * lane < p.D) x = o[32 * j + lane];
+            v[4 * j] = x.x; v[4 * j + 1] = x.y; v[4 * j + 2] = x.z; v[4 * j + 3] = x.w;
+        }
+    } else {
+        const float* rec = p.rec + r * (p.D + 2);
+        m = rec[0]; l = rec[1];
+#pragma unroll
+        for (int i = 0; i < KPER; ++i) {
+            const int d = 128 * (i / 4) + 4 * lane + i % 4;
+            v[i] = d < p.D ? rec[2 + d] : 0.f;
+        }
+    }
+}
+
 // One CTA per output row.  The records of a row are shared out over the NW warps (record s goes
 // to warp s mod NW, whose lanes read it coalesced), each warp keeps a running (m, l, o) of its
 // records, and the NW states are merged through shared memory — the same recurrence at both levels.
@@ -56,21 +94,14 @@ constexpr int kCombineThreads = 256;
 // registers, which lets half as many more CTAs sit on an SM (the kernel is bound by the latency of its few
 // loads per warp, i.e. by how many CTAs are resident).  One warp per row: 26 CTAs per SM, for which 72 registers (and
 // 24 bytes of spills) are what it gets.
-template <int NW, int KPER = kMaxD / 32>
+template <int NW, int KPER = kMaxD / 32, bool PLANES = true>
 __global__ void __launch_bounds__(NW * 32, NW == 1 ? 26 : 1) combine_kernel(CombineParams p) {
-    __shared__ float sm_m[NW], sm_l[NW], sm_o[NW][32 * KPER];
+    __shared__ float sm_m[NW], sm_l[NW];
+    __shared__ __align__(16) float sm_o[NW][32 * KPER];
     const int orow = blockIdx.x, D = p.D;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float* base;
-    int64_t stride;
-    if (p.rep > 0) {
-        const int row = orow / p.rep, r = orow % p.rep;
-        base = p.rec + ((size_t)row * p.nsplit * p.rep + r) * (D + 2);
-        stride = (int64_t)p.rep * (D + 2);
-    } else {
-        base = p.rec + (size_t)orow * (D + 2);
-        stride = p.stride_s;
-    }
+    size_t first, step;
+    record_walk(p, orow, first, step);
     mma::grid_release();
     mma::grid_wait();
     const float poison = (p.status && *p.status) ? __int_as_float(0x7fc00000) : 0.f;
@@ -91,14 +122,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 1 ? 26 : 1) combine_kernel(Comb
         for (int b = 0; b < kBatch; ++b) {
             const int s = s0 + NW * b;
             const bool live = s < s_hi;
-            const float* rec = base + (live ? s : s0) * stride;
-            ms[b] = live ? rec[0] : -INFINITY;
-            ls[b] = rec[1];
-#pragma unroll
-            for (int i = 0; i < kPer; ++i) {
-                const int d = lane + 32 * i;
-                v[b][i] = d < D ? rec[2 + d] : 0.f;
-            }
+            load_record<kPer, PLANES>(p, first + (size_t)(live ? s : s0) * step, lane, ms[b], ls[b], v[b]);
+            if (!live) ms[b] = -INFINITY;
         }
         // one reference for the batch: its exponentials are independent of one another, where a running
         // reference makes a chain of two per record
@@ -122,10 +147,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 1 ? 26 : 1) combine_kernel(Comb
     }
     if (lane == 0) { sm_m[warp] = m; sm_l[warp] = l; }
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        const int d = lane + 32 * i;
-        if (d < D) sm_o[warp][d] = o[i];
-    }
+    for (int j = 0; j < kPer / 4; ++j)
+        *reinterpret_cast<float4*>(&sm_o[warp][128 * j + 4 * lane]) = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
     __syncthreads();
     float M = -INFINITY;
 #pragma unroll
@@ -142,9 +165,12 @@ __global__ void __launch_bounds__(NW * 32, NW == 1 ? 26 : 1) combine_kernel(Comb
         for (int w = 0; w < NW; ++w) a += sm_o[w][d] * wgt[w];
         a += poison;
         if (p.normalise) p.out[out_row * D + d] = a / fmaxf(L, 1e-20f);
+        else if (p.out_ml) p.out[out_row * D + d] = a;
         else p.out[out_row * (D + 2) + 2 + d] = a;
     }
-    if (!p.normalise && threadIdx.x == 0) {
+    if (p.out_ml) {
+        if (threadIdx.x == 0) p.out_ml[out_row] = make_float2(M, L);
+    } else if (!p.normalise && threadIdx.x == 0) {
         p.out[out_row * (D + 2) + 0] = M;
         p.out[out_row * (D + 2) + 1] = L;
     }
@@ -223,21 +249,14 @@ __device__ __forceinline__ void st_relaxed_sys(int* p, int v) {
 }
 
 __global__ void __launch_bounds__(kCombineThreads) exchange_combine_kernel(CombineParams p, ExchangeParams x) {
-    __shared__ float sm_m[8], sm_l[8], sm_o[8][kMaxD];
+    __shared__ float sm_m[8], sm_l[8];
+    __shared__ __align__(16) float sm_o[8][kMaxD];
     __shared__ float xm[kMaxWorld], xl[kMaxWorld];
     __shared__ int s_seq, s_fail;
     const int orow = blockIdx.x, D = p.D;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float* base;
-    int64_t stride;
-    if (p.rep > 0) {
-        const int row = orow / p.rep, r = orow % p.rep;
-        base = p.rec + ((size_t)row * p.nsplit * p.rep + r) * (D + 2);
-        stride = (int64_t)p.rep * (D + 2);
-    } else {
-        base = p.rec + (size_t)orow * (D + 2);
-        stride = p.stride_s;
-    }
+    size_t first, step;
+    record_walk(p, orow, first, step);
     const bool local_fail = p.status && *p.status;
     constexpr int kPer = kMaxD / 32;
     float m = -INFINITY, l = 0.f, o[kPer];
@@ -251,14 +270,8 @@ __global__ void __launch_bounds__(kCombineThreads) exchange_combine_kernel(Combi
         for (int b = 0; b < kBatch; ++b) {
             const int s = s0 + 8 * b;
             const bool live = s < parts;
-            const float* rec = base + (live ? s : s0) * stride;
-            ms[b] = live ? rec[0] : -INFINITY;
-            ls[b] = rec[1];
-#pragma unroll
-            for (int i = 0; i < kPer; ++i) {
-                const int d = lane + 32 * i;
-                v[b][i] = d < D ? rec[2 + d] : 0.f;
-            }
+            load_record<kPer, true>(p, first + (size_t)(live ? s : s0) * step, lane, ms[b], ls[b], v[b]);
+            if (!live) ms[b] = -INFINITY;
         }
 #pragma unroll
         for (int b = 0; b < kBatch; ++b) {
@@ -273,10 +286,8 @@ __global__ void __launch_bounds__(kCombineThreads) exchange_combine_kernel(Combi
     }
     if (lane == 0) { sm_m[warp] = m; sm_l[warp] = l; }
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        const int d = lane + 32 * i;
-        if (d < D) sm_o[warp][d] = o[i];
-    }
+    for (int j = 0; j < kPer / 4; ++j)
+        *reinterpret_cast<float4*>(&sm_o[warp][128 * j + 4 * lane]) = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
     if (threadIdx.x == 0) { s_seq = x.seq[orow] + 1; s_fail = 0; }
     __syncthreads();
     float M = -INFINITY;
@@ -632,7 +643,10 @@ static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs,
                                           reinterpret_cast<uintptr_t>(vlo) | reinterpret_cast<uintptr_t>(vstep)) & 15) == 0;
     const Plan pl = make_plan(rows, nb, D, group, rep, scales_aligned && nb > 0);
     int* header = static_cast<int*>(workspace);
+    // the o plane of the records, then their (m, l) plane, then the same two of the partial merges
     float* records = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + kHeaderBytes);
+    const size_t n_records = (size_t)B * Hq * pl.parts;
+    float2* records_ml = reinterpret_cast<float2*>(records + n_records * D);
 
     if ((mass_out || paged) && !pl.mma) return GKV_E_SHAPE;  // the by-product and the pool form exist in the tensor-core kernel only
     float2* mass_part = mass_out ? reinterpret_cast<float2*>(static_cast<uint8_t*>(workspace) + need) : nullptr;
@@ -658,7 +672,7 @@ static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs,
         mp.q = q; mp.data = data; mp.offs = offs;
         mp.klo = static_cast<const __half*>(klo); mp.kstep = static_cast<const __half*>(kstep);
         mp.vlo = static_cast<const __half*>(vlo); mp.vstep = static_cast<const __half*>(vstep);
-        mp.level = level; mp.valid = valid; mp.part = records; mp.counter = header; mp.status = header + 1;
+        mp.level = level; mp.valid = valid; mp.part = records; mp.part_ml = records_ml; mp.counter = header; mp.status = header + 1;
         mp.mass_part = mass_part;
         mp.B = B; mp.Hq = Hq; mp.Hkv = Hkv; mp.nb = nb; mp.rep = rep; mp.chunk = pl.bps;
         mp.items_per_row = pl.nsplit; mp.items = rows * pl.nsplit; mp.per_row_meta = meta_rows != 1;
@@ -684,7 +698,7 @@ static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs,
         p.klo = static_cast<const __half*>(klo); p.kstep = static_cast<const __half*>(kstep);
         p.vlo = static_cast<const __half*>(vlo); p.vstep = static_cast<const __half*>(vstep);
         p.level = level; p.valid = valid;
-        p.part = records;
+        p.part = records; p.part_ml = records_ml;
         p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.nb = nb; p.group = group;
         p.G = (kP + group - 1) / group; p.gv = (D + group - 1) / group; p.rep = rep;
         p.nsplit = pl.nsplit; p.bps = pl.bps; p.per_row_meta = meta_rows != 1; p.stride_bh = stride_bh;
@@ -696,7 +710,7 @@ static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs,
     }
 
     CombineParams c;
-    c.rec = records; c.out = out; c.parts = pl.parts; c.D = D; c.rep = rep; c.nsplit = pl.parts;
+    c.rec = records; c.ml = records_ml; c.out = out; c.out_ml = nullptr; c.parts = pl.parts; c.D = D; c.rep = rep; c.nsplit = pl.parts;
     c.stride_s = 0; c.normalise = normalise; c.status = pl.mma ? header + 1 : nullptr;
     c.segs = 1; c.per_seg = 0; c.ml_out = nullptr;
     c.plan_tab = nullptr; c.chunk = 1; c.tab_per_row = 0; c.warps_per_item = 1;
@@ -704,12 +718,14 @@ static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs,
         c.plan_tab = combine_tab; c.chunk = pl.bps; c.tab_per_row = meta_rows != 1; c.warps_per_item = mma::kConsumerWarps;
     }
     if (pl.segs > 1) {
-        // level 1: (rows, parts, rep, D+2) -> (segs, B*Hq, D+2) behind the records
-        float* mid = records + (size_t)B * Hq * pl.parts * (D + 2);
-        c.out = mid; c.normalise = 0; c.segs = pl.segs; c.per_seg = (pl.parts + pl.segs - 1) / pl.segs;
+        // level 1: (rows, parts, rep) records -> (segs, B*Hq) records behind them
+        const size_t n_mid = (size_t)B * Hq * pl.segs;
+        float* mid = records + n_records * (D + 2);
+        float2* mid_ml = reinterpret_cast<float2*>(mid + n_mid * D);
+        c.out = mid; c.out_ml = mid_ml; c.normalise = 0; c.segs = pl.segs; c.per_seg = (pl.parts + pl.segs - 1) / pl.segs;
         if (const int rc = launch_combine(c, dim3(B * Hq, pl.segs), stream)) return rc;
-        c.rec = mid; c.out = out; c.parts = pl.segs; c.rep = 0; c.nsplit = 0; c.plan_tab = nullptr;
-        c.stride_s = (int64_t)B * Hq * (D + 2); c.normalise = normalise; c.segs = 1; c.per_seg = 0;
+        c.rec = mid; c.ml = mid_ml; c.out = out; c.out_ml = nullptr; c.parts = pl.segs; c.rep = 0; c.nsplit = 0; c.plan_tab = nullptr;
+        c.stride_s = (int64_t)B * Hq; c.normalise = normalise; c.segs = 1; c.per_seg = 0;
     }
     c.ml_out = mass_ml;
     if (xch) exchange_combine_kernel<<<B * Hq, kCombineThreads, 0, stream>>>(c, *xch);
@@ -897,12 +913,12 @@ int gkv_combine_partials(const float* partials, float* out, int parts, int rows,
     if (!partials || !out) return GKV_E_NULL;
     if (parts <= 0 || rows <= 0 || D <= 0) return GKV_E_SHAPE;
     gkv::CombineParams c;
-    c.rec = partials; c.out = out; c.parts = parts; c.D = D; c.rep = 0; c.nsplit = 0;
-    c.stride_s = (int64_t)rows * (D + 2); c.normalise = 1; c.status = nullptr; c.segs = 1; c.per_seg = 0; c.ml_out = nullptr;
+    c.rec = partials; c.ml = nullptr; c.out = out; c.out_ml = nullptr; c.parts = parts; c.D = D; c.rep = 0; c.nsplit = 0;
+    c.stride_s = (int64_t)rows; c.normalise = 1; c.status = nullptr; c.segs = 1; c.per_seg = 0; c.ml_out = nullptr;
     c.plan_tab = nullptr; c.chunk = 1; c.tab_per_row = 0; c.warps_per_item = 1;
     // the records come from anywhere in the stream: launched the ordinary way
-    if (D <= 128) gkv::combine_kernel<8, 4><<<rows, gkv::kCombineThreads, 0, static_cast<cudaStream_t>(stream)>>>(c);
-    else gkv::combine_kernel<8><<<rows, gkv::kCombineThreads, 0, static_cast<cudaStream_t>(stream)>>>(c);
+    if (D <= 128) gkv::combine_kernel<8, 4, false><<<rows, gkv::kCombineThreads, 0, static_cast<cudaStream_t>(stream)>>>(c);
+    else gkv::combine_kernel<8, gkv::kMaxD / 32, false><<<rows, gkv::kCombineThreads, 0, static_cast<cudaStream_t>(stream)>>>(c);
     GKV_LAUNCH_CHECK();
     return GKV_OK;
 }

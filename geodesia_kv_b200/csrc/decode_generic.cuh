@@ -24,7 +24,8 @@ struct DecodeParams {
     const __half* vstep;
     const int32_t* level;
     const int32_t* valid;
-    float* part;      // (rows, nsplit, rep, D+2): m, l, o[D]
+    float* part;      // (rows, nsplit, rep, D): o of every record
+    float2* part_ml;  // (rows, nsplit, rep): its (m, l)
     int B, Hq, Hkv, D, nb, group, G, gv, rep;
     int nsplit, bps;
     int per_row_meta; // 0: one metadata row shared by all cache rows
@@ -189,19 +190,13 @@ __global__ void __launch_bounds__(kGenThreads) decode_generic_kernel(DecodeParam
         __syncthreads();
     }
 
-    float* part = p.part + ((size_t)row * p.nsplit + sp) * rep * (D + 2);
+    const size_t rec0 = ((size_t)row * p.nsplit + sp) * rep;
 #pragma unroll
     for (int i = 0; i < kMaxAcc; ++i) {
         const int pr = tid + i * kGenThreads;
-        if (pr < rep * D) {
-            const int h = pr / D, d = pr - h * D;
-            part[(size_t)h * (D + 2) + 2 + d] = acc[i];
-        }
+        if (pr < rep * D) p.part[rec0 * D + pr] = acc[i];
     }
-    if (tid < rep) {
-        part[(size_t)tid * (D + 2) + 0] = sm[tid];
-        part[(size_t)tid * (D + 2) + 1] = sl[tid];
-    }
+    if (tid < rep) p.part_ml[rec0 + tid] = make_float2(sm[tid], sl[tid]);
 }
 
 inline size_t decode_generic_smem(int rep, int D) {

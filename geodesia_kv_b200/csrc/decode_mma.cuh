@@ -135,7 +135,8 @@ struct Params {
     const int32_t* valid;
     const uint4* plan;       // (metadata rows, nb) block entries of every row sorted by rung, from plan_kernel
     const int32_t* plan_tab; // (metadata rows, kPlanTabInts) start of each rung class in that list
-    float* part;             // (rows, items per row, consumer warps, rep, D+2)
+    float* part;             // (rows, items per row, consumer warps, rep, D): o of every record
+    float2* part_ml;         // (rows, items per row, consumer warps, rep): its (m, l)
     float2* mass_part;       // optional (rows, nb, 2 units, rep): (reference, sum of weights against it) per block half and head,
                              // natural-log domain; the by-product from which the per-block softmax mass is made
     int* counter;            // work-item counter (zeroed before launch)
@@ -1355,60 +1356,68 @@ __device__ __forceinline__ void clear_invalid_tail(uint8_t* blk, int level, int 
     __syncwarp();
 }
 
-// Channel of row r (odd = 0) or r+8 (odd = 1) of output m-tile mt, for each rung's value layout.
-template <int D, int G, int BITS>
-__device__ __forceinline__ int out_channel(int mt, int r, int odd) {
-    if (BITS == 16) return 16 * mt + r + 8 * odd;
-    using V = VT<D, G, BITS == 16 ? 8 : BITS>;
-    return V::SP * (mt / V::MTS) + V::F * r + 2 * (mt % V::MTS) + odd;
+// F neighbouring floats of a record's o row (F = 2, 4 or 8; the row starts on 16 bytes).
+template <int F>
+__device__ __forceinline__ void store_run(float* dst, const float (&x)[F]) {
+    if (F == 2) *reinterpret_cast<float2*>(dst) = make_float2(x[0], x[1]);
+    else {
+#pragma unroll
+        for (int i = 0; i < F; i += 4)
+            *reinterpret_cast<float4*>(dst + i) = make_float4(x[i], x[(i + 1) % F], x[(i + 2) % F], x[(i + 3) % F]);
+    }
 }
 
-// This warp's record of an item (natural-log domain): m, l, o[D] per head.
+// This warp's record of an item (natural-log domain): (m, l) and o[D] per head.
+//
+// A thread's channels of a span are F neighbours (channel SP * s + F * r + field), so they go out as one run.  One float
+// at a time, each store touched 32 sectors, eight times what its bytes need, and an item's records took about 1.5 us of
+// its CTA.  Runs here and 16-byte loads in the merge: 256 ragged sequences with mass 401.5 -> 380.1 us, 32 x 16k tokens with
+// eight heads per row 248 -> 242; from a graph, one sequence of 1000 tokens 14.6 -> 12.3 us and of 16k 19.9 -> 17.3.
 template <int D, int G, int BITS, bool DUP>
-__device__ __forceinline__ void write_record(const Params& p, const Ctx<D, G>& c, const WarpState<D, G>& st, float* rec0) {
+__device__ __forceinline__ void write_record(const Params& p, const Ctx<D, G>& c, const WarpState<D, G>& st, size_t rec0) {
     using C = Cfg<D, G>;
     float l = st.l;
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
     const int myhead = head_of_row<DUP>(c.r);
-    if (c.t == 0 && myhead < p.rep && (!DUP || (c.r & 1) == 0)) {
-        float* rec = rec0 + (size_t)myhead * (D + 2);
-        rec[0] = st.m * 0.6931471805599453f;
-        rec[1] = l;
-    }
-    // p . vlo of channel group cg and column n sits in the lane of row cg, quad position n / 2, scaled 2^8
-    const float ob0 = DUP ? st.ob[0] + st.ob[1] : st.ob[0], ob1 = st.ob[1];
+    if (c.t == 0 && myhead < p.rep && (!DUP || (c.r & 1) == 0))
+        p.part_ml[rec0 + myhead] = make_float2(st.m * 0.6931471805599453f, l);
     constexpr float kRow = 65536.f, kRow8 = 65536.f / v_rowscale(BITS);
+    // heads of this thread's columns: t when the columns 2t, 2t+1 are its hi and lo halves, else 2t and 2t+1
+    const int h0 = DUP ? c.t : 2 * c.t;
+    float* out0 = p.part + (rec0 + h0) * D;
+    float* out1 = out0 + D;
+    const bool has0 = h0 < p.rep, has1 = !DUP && h0 + 1 < p.rep;
+    if (BITS == 16) {
+        // channels 16 m + r and 16 m + 8 + r: eight lanes fill a 32-byte sector
 #pragma unroll
-    for (int mt = 0; mt < C::MT; ++mt) {
-        const int ch0 = out_channel<D, G, BITS>(mt, c.r, 0), ch1 = out_channel<D, G, BITS>(mt, c.r, 1);
-        float bias00 = 0.f, bias01 = 0.f, bias10 = 0.f, bias11 = 0.f;      // [channel row][column]
-        if (BITS != 16) {
-            const int l0 = ((ch0 / G) % 8) * 4 + c.t, l1 = ((ch1 / G) % 8) * 4 + c.t;
-            bias00 = __shfl_sync(0xffffffffu, ob0, l0) * 0.00390625f;
-            bias10 = __shfl_sync(0xffffffffu, ob0, l1) * 0.00390625f;
-            if (!DUP) {
-                bias01 = __shfl_sync(0xffffffffu, ob1, l0) * 0.00390625f;
-                bias11 = __shfl_sync(0xffffffffu, ob1, l1) * 0.00390625f;
-            }
+        for (int mt = 0; mt < C::MT; ++mt) {
+            const float (&o)[4] = st.o[mt];
+            const int ch = 16 * mt + c.r;
+            if (has0) { out0[ch] = (DUP ? o[0] + o[1] : o[0]) * kRow; out0[ch + 8] = (DUP ? o[2] + o[3] : o[2]) * kRow; }
+            if (has1) { out1[ch] = o[1] * kRow; out1[ch + 8] = o[3] * kRow; }
         }
-        if (DUP) {
-            if (c.t < p.rep) {
-                float* rec = rec0 + (size_t)c.t * (D + 2) + 2;
-                rec[ch0] = fmaf(st.o[mt][0] + st.o[mt][1], kRow, bias00);
-                rec[ch1] = fmaf(st.o[mt][2] + st.o[mt][3], kRow8, bias10);
+    } else {
+        using V = VT<D, G, BITS == 16 ? 8 : BITS>;
+        // p . vlo of channel group cg and column n sits in the lane of row cg, quad position n / 2, scaled 2^8
+        const float ob0 = DUP ? st.ob[0] + st.ob[1] : st.ob[0], ob1 = st.ob[1];
+#pragma unroll
+        for (int s = 0; s < V::NSPAN; ++s) {
+            const int from = ((s / V::SPC) % 8) * 4 + c.t;             // a span lies in one channel group
+            const float bias0 = __shfl_sync(0xffffffffu, ob0, from) * 0.00390625f;
+            const float bias1 = DUP ? 0.f : __shfl_sync(0xffffffffu, ob1, from) * 0.00390625f;
+            float x0[V::F], x1[V::F];
+#pragma unroll
+            for (int k = 0; k < V::MTS; ++k) {
+                const float (&o)[4] = st.o[s * V::MTS + k];
+                x0[2 * k] = fmaf(DUP ? o[0] + o[1] : o[0], kRow, bias0);
+                x0[2 * k + 1] = fmaf(DUP ? o[2] + o[3] : o[2], kRow8, bias0);
+                x1[2 * k] = fmaf(o[1], kRow, bias1);
+                x1[2 * k + 1] = fmaf(o[3], kRow8, bias1);
             }
-        } else {
-            if (2 * c.t < p.rep) {
-                float* rec = rec0 + (size_t)(2 * c.t) * (D + 2) + 2;
-                rec[ch0] = fmaf(st.o[mt][0], kRow, bias00);
-                rec[ch1] = fmaf(st.o[mt][2], kRow8, bias10);
-            }
-            if (2 * c.t + 1 < p.rep) {
-                float* rec = rec0 + (size_t)(2 * c.t + 1) * (D + 2) + 2;
-                rec[ch0] = fmaf(st.o[mt][1], kRow, bias01);
-                rec[ch1] = fmaf(st.o[mt][3], kRow8, bias11);
-            }
+            const int ch = V::SP * s + V::F * c.r;
+            if (has0) store_run<V::F>(out0 + ch, x0);
+            if (has1) store_run<V::F>(out1 + ch, x1);
         }
     }
 }
@@ -1426,7 +1435,7 @@ __device__ __forceinline__ void report_mass(const Params& p, const Ctx<D, G>& c,
 template <int D, int G, int BITS, bool DUP, bool MASS>
 __device__ __forceinline__ int ring_item(
                                          const Params& p, Smem<D, G>& sm, const Ctx<D, G>& c, const ItemDesc& it,
-                                      int stream, int u0, int u1, int& seq, float* rec0) {
+                                      int stream, int u0, int u1, int& seq, size_t rec0) {
     using C = Cfg<D, G>;
     using UU = Unit<D, G>;
     WarpState<D, G> st;
@@ -1484,7 +1493,7 @@ __device__ __forceinline__ int ring_item(
 // 8(l & 15) .. +7 of the key (for the scores, reduced over the half) and of the value.
 template <int D, int G, bool MASS>
 __device__ __forceinline__ void centroid_item(const Params& p, const Ctx<D, G>& c, const ItemDesc& it, const uint4* tab,
-                                              int warp, float* rec0) {
+                                              int warp, size_t rec0) {
     constexpr int kMaxMine = (kMaxCentroidItemBlocks + kConsumerWarps - 1) / kConsumerWarps;
     constexpr int LPV = D / 8;                            // lanes that cover one vector with 16 bytes each
     static_assert(LPV <= 16, "head dim too large for the centroid path");
@@ -1577,11 +1586,10 @@ __device__ __forceinline__ void centroid_item(const Params& p, const Ctx<D, G>& 
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
         if (h0 + h < p.rep && hl < LPV) {
-            float* rec = rec0 + (size_t)(h0 + h) * (D + 2);
-            if (hl == 0) { rec[0] = m[h]; rec[1] = l[h]; }
-            float2* d2 = reinterpret_cast<float2*>(rec + 2 + 8 * hl);      // records are 8-byte aligned
-            d2[0] = make_float2(o[h][0], o[h][1]); d2[1] = make_float2(o[h][2], o[h][3]);
-            d2[2] = make_float2(o[h][4], o[h][5]); d2[3] = make_float2(o[h][6], o[h][7]);
+            float* o8 = p.part + (rec0 + h0 + h) * D + 8 * hl;
+            if (hl == 0) p.part_ml[rec0 + h0 + h] = make_float2(m[h], l[h]);
+            reinterpret_cast<float4*>(o8)[0] = make_float4(o[h][0], o[h][1], o[h][2], o[h][3]);
+            reinterpret_cast<float4*>(o8)[1] = make_float4(o[h][4], o[h][5], o[h][6], o[h][7]);
         }
     }
 }
@@ -1613,7 +1621,7 @@ __device__ void consumer_loop(const Params& p, Smem<D, G>& sm, int* abort_flag) 
         c.sq = smem_u32(sm.sq) + (uint32_t)(ib * C::SQ_BYTES);
         c.f = sm.sf[ib * 16 + head_of_row<DUP>(c.r)];
         const size_t rec_idx = (size_t)it.row * p.items_per_row + (size_t)(it.item / p.rows);
-        float* rec0 = p.part + (rec_idx * kConsumerWarps + warp) * p.rep * (D + 2);
+        const size_t rec0 = (rec_idx * kConsumerWarps + warp) * p.rep;
         if (it.level == 1) {
             centroid_item<D, G, MASS>(p, c, it, sm.item_tab + is * kMaxItemBlocks, warp, rec0);
         }
