@@ -44,7 +44,7 @@ __device__ __forceinline__ int live_parts(const CombineParams& p, int orow) {
     int used = 0;
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
-        const int ck = k == 4 ? min(p.chunk, mma::kMaxCentroidItemBlocks) : p.chunk;     // as the kernel cuts the runs
+        const int ck = k == 4 ? mma::centroid_chunk(p.chunk) : p.chunk;     // as the kernel cuts the runs
         used += (tab[k + 1] - tab[k] + ck - 1) / ck;
     }
     return min(p.parts, used * p.warps_per_item);
@@ -431,8 +431,7 @@ static Plan make_plan(int rows, int nb, int D, int group, int rep, bool allow_mm
         // mix of rungs, ceil(nb / chunk) + 4 slots hold them all (five runs, each with one short item
         // at most).  Slots a row does not need stay empty.
         pl.bps = chunk;
-        const int cmin = chunk < mma::kMaxCentroidItemBlocks ? chunk : mma::kMaxCentroidItemBlocks;
-        pl.nsplit = (nb + cmin - 1) / cmin + 4;
+        pl.nsplit = (nb + chunk - 1) / chunk + 4;               // centroid items are no shorter
         pl.parts = pl.nsplit * mma::kConsumerWarps;
         pl.segs = pl.parts > kCombineDirect ? (pl.parts / 64 < kCombineSegs ? pl.parts / 64 : kCombineSegs) : 1;
         return pl;

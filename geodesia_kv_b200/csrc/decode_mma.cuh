@@ -26,7 +26,7 @@
 //     one half of the block's tokens, with a private online softmax.  Nothing is merged
 //     inside the CTA: the combine kernel merges the per-warp records;
 //   * items of centroid blocks (512 bytes each) bypass the rings: the consumer warps read
-//     them straight from global memory with one coalesced 16-byte load per lane.
+//     them straight from global memory, sixteen at a time as the MMA fragments of both products.
 //
 // Arithmetic.  Integer codes are fed to the MMA as fp16 values from the LINEAR range of the
 // format: bit patterns 0..2047 (subnormals and the first binade) are worth pattern * 2^-24, so a
@@ -94,7 +94,8 @@ constexpr int kHelperRegs = 56, kConsumerRegs = 152;
 constexpr int kNSlot = GKV_NSLOT;        // descriptor slots (blocks in flight) per stream
 constexpr uint32_t kRingBytes = GKV_RING_KB * 1024;
 constexpr int kMaxItemBlocks = 128;      // blocks per work item (the item's block table in shared memory)
-constexpr int kMaxCentroidItemBlocks = 64;   // centroid items are held in registers by the warps that read them: shorter
+// Blocks of a centroid item: sixteen are one warp's tile, so items are at least that and twice as long as the others.
+__host__ __device__ constexpr int centroid_chunk(int chunk) { return chunk < 8 ? 16 : 2 * chunk < kMaxItemBlocks ? 2 * chunk : kMaxItemBlocks; }
 constexpr int kMinItemBlocks = kConsumerWarps / 2;   // one block per pair
 constexpr int kItemSlots = 4;            // item descriptors in flight: finishing, current, announced, spare
 #ifndef GKV_WAIT_LIMIT_NS
@@ -521,7 +522,7 @@ __device__ __forceinline__ Span span_of(const Params& p, int id) {
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
         const int start = st[k], cnt = st[k + 1] - start;
-        const int ck = k == 4 ? min(p.chunk, kMaxCentroidItemBlocks) : p.chunk;
+        const int ck = k == 4 ? centroid_chunk(p.chunk) : p.chunk;
         const int n = (cnt + ck - 1) / ck;
         if (slot < n) {
             sp.level = ladder_level(k);
@@ -861,7 +862,7 @@ __device__ void query_loop(const Params& p, Smem<D, G>& sm, int* abort_flag) {
         __half* qp = sm.qprep + (size_t)ib * (C::QPREP_BYTES / 2);
 #pragma unroll
         for (int i = 0; i < NV; ++i) *reinterpret_cast<float4*>(sq + (i * 32 + lane) * 4) = v[i];
-        if (it.level != 1) {     // a centroid item needs the fp32 rows only (its blocks are not scored through the MMA planes)
+        {
             // per-head power-of-two scale bringing max|q| into [8, 16); lane h ends up with head h's maximum
             float top = 0.f;
 #pragma unroll
@@ -884,7 +885,8 @@ __device__ void query_loop(const Params& p, Smem<D, G>& sm, int* abort_flag) {
                 sf[8 + lane] = ldexpf(1.0f, eq);
             }
             __syncwarp();
-            if (it.level == 16) query_planes<D, G, DUP, 16>(sq, sf, qp);
+            if (it.level == 1) query_planes<D, G, false, 8>(sq, sf, qp);          // fp16 rows: heads are rows for any number of them
+            else if (it.level == 16) query_planes<D, G, DUP, 16>(sq, sf, qp);
             else if (it.level == 8) query_planes<D, G, DUP, 8>(sq, sf, qp);
             else if (it.level == 4) query_planes<D, G, DUP, 4>(sq, sf, qp);
             else query_planes<D, G, DUP, 2>(sq, sf, qp);
@@ -1486,110 +1488,142 @@ __device__ __forceinline__ int ring_item(
     return 0;
 }
 
-// An item of centroid blocks (one key and one value vector stand for nvalid tokens; 512 bytes per
-// block at D = 128).  No ring: warp w takes blocks w, w + 12, ... of the item and reads each with one
-// 16-byte load per lane straight from global memory — all of its loads are in flight before the first
-// is used.  Lanes 0-15 own heads 0-3 and lanes 16-31 heads 4-7; lane l of a half owns channels
-// 8(l & 15) .. +7 of the key (for the scores, reduced over the half) and of the value.
+// Sixteen bytes of a cache row, which may stand at any address.
+__device__ __forceinline__ uint4 ldg16(const uint8_t* src) {
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) return __ldg(reinterpret_cast<const uint4*>(src));
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        w[i] = (uint32_t)src[4 * i] | ((uint32_t)src[4 * i + 1] << 8) | ((uint32_t)src[4 * i + 2] << 16) | ((uint32_t)src[4 * i + 3] << 24);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// An item of centroid blocks: one key and one value vector stand for nvalid tokens (512 bytes per block at D = 128).  No
+// ring: a warp takes TILES of sixteen blocks and treats them as sixteen tokens of fp16 rows whose weights are multiplied by
+// the blocks' counts.  The fragments of both products come straight from global memory: a thread's keys are its quad
+// position's channels of the tokens r and r + 8 (the B operand of S[head][token], query halves in rows 0-7 and 8-15), its
+// values D / 8 neighbouring channels of the tokens 2t, 2t+1, 2t+8, 2t+9, paired up by one permutation per register (the B
+// operand of O[head][channel], weight halves in the rows).  So O's columns 2t and 2t+1 of this thread are the D / 4 channels
+// from t * D / 4, whole runs of its record.
+//
+// On the FP32 pipes, a block at a time with a shuffle reduction per head, a block took a warp 4200 cycles, as much as one of
+// 64 tokens at 4 bits.  32 x 16k tokens, all centroids: 64.8 -> 39.3 us with four heads per row, 76.6 -> 45.3 with eight; 256
+// ragged sequences demoted to 4 bits 381 -> 350; one of a million tokens 209 -> 197.  Against 64 bits the error of such a
+// cache is what it was (4.2e-5 of the result's norm at worst, 4.3e-5 before).
 template <int D, int G, bool MASS>
 __device__ __forceinline__ void centroid_item(const Params& p, const Ctx<D, G>& c, const ItemDesc& it, const uint4* tab,
-                                              int warp, size_t rec0) {
-    constexpr int kMaxMine = (kMaxCentroidItemBlocks + kConsumerWarps - 1) / kConsumerWarps;
-    constexpr int LPV = D / 8;                            // lanes that cover one vector with 16 bytes each
-    static_assert(LPV <= 16, "head dim too large for the centroid path");
-    const int lane = c.lane, hl = lane & 15, h0 = (lane >> 4) * 4;
-    // this warp's blocks are entries warp, warp + 12, ... of the item's table (shared memory)
-    const int nmine = it.nblk > warp ? (it.nblk - warp + kConsumerWarps - 1) / kConsumerWarps : 0;
-    uint4 kraw[kMaxMine], vraw[kMaxMine];
-    int nval[kMaxMine];
+                                              int first, float f, size_t rec0) {
+    using C = Cfg<D, G>;
+    constexpr int NK = C::DT / 8;                         // 16-byte pieces of this thread's key channels
+    constexpr int VC = D / 8, NV = VC / 8;                // its value channels per token, and their 16-byte pieces
+    constexpr float kScale = 256.f;                       // weights are at most 64: well inside fp16, and far from its subnormals
+    const int tiles = (it.nblk + 15) >> 4;
+    float o[VC][4];
 #pragma unroll
-    for (int j = 0; j < kMaxMine; ++j) {
-        nval[j] = 0;
-        kraw[j] = vraw[j] = make_uint4(0, 0, 0, 0);
-        if (j < nmine) {
-            const uint4 e = tab[warp + kConsumerWarps * j];
-            nval[j] = (int)((e.z >> 8) & 0xffu);
+    for (int i = 0; i < VC; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    float m = -INFINITY, l = 0.f;
+    for (int tile = first; tile < tiles; tile += kConsumerWarps) {
+        const int b0 = tile * 16;
+        // entries beyond the item repeat its last one; their scores are masked
+        auto entry = [&](int i) { return tab[min(b0 + i, it.nblk - 1)]; };
+        auto source = [&](const uint4& e) { return p.data + (((unsigned long long)e.y << 32) | e.x); };
+        // the values come after the scores are known (registers); until then they move as far as L2
+        if (2 * D >= 128 * (c.lane >> 4) + 128) prefetch_l2(source(entry(c.lane & 15)) + 2 * D + 128 * (c.lane >> 4));
+        uint4 kw[2][NK];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint8_t* src = source(entry(c.r + 8 * j)) + 2 * C::DT * c.t;
+#pragma unroll
+            for (int i = 0; i < NK; ++i) kw[j][i] = ldg16(src + 16 * i);
         }
-        if (j < nmine && hl < LPV) {
-            const uint4 e = tab[warp + kConsumerWarps * j];
-            const uint8_t* src = p.data + (((unsigned long long)e.y << 32) | e.x);
-            if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-                kraw[j] = __ldg(reinterpret_cast<const uint4*>(src) + hl);
-                vraw[j] = __ldg(reinterpret_cast<const uint4*>(src + 2 * D) + hl);
-            } else {                                      // a cache row at an odd address: byte loads
-                uint32_t w[8];
-                for (int i = 0; i < 8; ++i) {
-                    const uint8_t* s4 = src + (i < 4 ? 0 : 2 * D) + 16 * hl + 4 * (i & 3);
-                    w[i] = (uint32_t)s4[0] | ((uint32_t)s4[1] << 8) | ((uint32_t)s4[2] << 16) | ((uint32_t)s4[3] << 24);
+        float cnt[4];
+        int orig[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = 2 * c.t + (j & 1) + 8 * (j >> 1);
+            const uint4 e = entry(i);
+            cnt[j] = b0 + i < it.nblk ? (float)((e.z >> 8) & 0xffu) : 0.f;
+            orig[j] = (int)e.w;
+        }
+        float z[4];
+        {
+            float acc[2][4];
+#pragma unroll
+            for (int i = 0; i < C::CH; ++i) {
+                const uint4 qa = qchunk(c, 0, i), qb = qchunk(c, 1, i);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const uint4 w = kw[j][i % NK];
+                    if (i == 0) mma_f16_z(acc[j], qa.x, qa.y, qa.z, qa.w, w.x, w.y);
+                    else mma_f16(acc[j], qa.x, qa.y, qa.z, qa.w, w.x, w.y);
+                    mma_f16(acc[j], qb.x, qb.y, qb.z, qb.w, w.z, w.w);
                 }
-                kraw[j] = make_uint4(w[0], w[1], w[2], w[3]);
-                vraw[j] = make_uint4(w[4], w[5], w[6], w[7]);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                z[2 * j] = cnt[2 * j] > 0.f ? (acc[j][0] + acc[j][2]) * f : -INFINITY;          // log2 domain
+                z[2 * j + 1] = cnt[2 * j + 1] > 0.f ? (acc[j][1] + acc[j][3]) * f : -INFINITY;
             }
         }
-    }
-    // this lane's slice of its four heads' queries (fp32 rows prepared by the query warp)
-    float q[4][8];
+        uint4 vw[4][NV];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        const uint4 a = lds_v4(c.sq + (uint32_t)(((h0 + h) * D + 8 * (hl % LPV)) * 4));
-        const uint4 b = lds_v4(c.sq + (uint32_t)(((h0 + h) * D + 8 * (hl % LPV) + 4) * 4));
-        q[h][0] = __uint_as_float(a.x); q[h][1] = __uint_as_float(a.y); q[h][2] = __uint_as_float(a.z); q[h][3] = __uint_as_float(a.w);
-        q[h][4] = __uint_as_float(b.x); q[h][5] = __uint_as_float(b.y); q[h][6] = __uint_as_float(b.z); q[h][7] = __uint_as_float(b.w);
-    }
-    float m[4], l[4], o[4][8];
+        for (int j = 0; j < 4; ++j) {
+            const uint8_t* src = source(entry(2 * c.t + (j & 1) + 8 * (j >> 1))) + 2 * D + 2 * VC * c.r;
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        m[h] = -INFINITY; l[h] = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[h][i] = 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < kMaxMine; ++j) {
-        if (j >= nmine) break;                            // warp-uniform
-        const uint32_t kw[4] = {kraw[j].x, kraw[j].y, kraw[j].z, kraw[j].w};
-        const uint32_t vw[4] = {vraw[j].x, vraw[j].y, vraw[j].z, vraw[j].w};
-        float kf[8], vf[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 a = __half22float2(u32_as_h2(kw[i])), b = __half22float2(u32_as_h2(vw[i]));
-            kf[2 * i] = a.x; kf[2 * i + 1] = a.y; vf[2 * i] = b.x; vf[2 * i + 1] = b.y;
+            for (int h = 0; h < NV; ++h) vw[j][h] = ldg16(src + 16 * h);
         }
-        const float cnt = (float)nval[j];
+        float mx = fmaxf(fmaxf(z[0], z[1]), fmaxf(z[2], z[3]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        if (__any_sync(0xffffffffu, mx > m)) {
+            const float mn = fmaxf(m, mx);
+            const float corr = m > -INFINITY ? ex2(m - mn) : 0.f;         // rows are heads, on both operands
+            l *= corr;
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            float s = 0.f;
+            for (int i = 0; i < VC; ++i) { o[i][0] *= corr; o[i][1] *= corr; o[i][2] *= corr; o[i][3] *= corr; }
+            m = mn;
+        }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) s = fmaf(q[h][i], kf[i], s);
-            if (hl >= LPV) s = 0.f;
-#pragma unroll
-            for (int o2 = 1; o2 < 16; o2 <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o2);
-            if (s > m[h]) {                               // exact running maximum (natural-log domain)
-                const float corr = expf(m[h] - s);
-                l[h] *= corr;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[h][i] *= corr;
-                m[h] = s;
-            }
-            const float w = expf(s - m[h]) * cnt;
-            l[h] += w;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o[h][i] = fmaf(w, vf[i], o[h][i]);
-            if (MASS && hl == 0 && h0 + h < p.rep) {     // the block's whole mass is reported as its first unit
+        for (int j = 0; j < 4; ++j) {
+            z[j] = ex2(z[j] - m) * cnt[j];
+            l += z[j];
+            if (MASS && c.r < p.rep && cnt[j] > 0.f) {   // the block's whole mass is reported as its first unit
                 constexpr int UPB = kP / G;
-                const int orig = (int)tab[warp + kConsumerWarps * j].w;
-                float2* mp = p.mass_part + ((size_t)it.row * p.nb + orig) * UPB * p.rep + (h0 + h);
-                mp[0] = make_float2(m[h], w);
+                float2* mp = p.mass_part + ((size_t)it.row * p.nb + orig[j]) * UPB * p.rep + c.r;
+                mp[0] = make_float2(m * 0.6931471805599453f, z[j]);
                 for (int u = 1; u < UPB; ++u) mp[(size_t)u * p.rep] = make_float2(-INFINITY, 0.f);
             }
         }
-    }
+        uint32_t ph[2], pl[2];
+        split_f16x2(z[0] * kScale, z[1] * kScale, ph[0], pl[0]);
+        split_f16x2(z[2] * kScale, z[3] * kScale, ph[1], pl[1]);
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        if (h0 + h < p.rep && hl < LPV) {
-            float* o8 = p.part + (rec0 + h0 + h) * D + 8 * hl;
-            if (hl == 0) p.part_ml[rec0 + h0 + h] = make_float2(m[h], l[h]);
-            reinterpret_cast<float4*>(o8)[0] = make_float4(o[h][0], o[h][1], o[h][2], o[h][3]);
-            reinterpret_cast<float4*>(o8)[1] = make_float4(o[h][4], o[h][5], o[h][6], o[h][7]);
+        for (int h = 0; h < NV; ++h) {
+            const uint32_t x0[4] = {vw[0][h].x, vw[0][h].y, vw[0][h].z, vw[0][h].w}, x1[4] = {vw[1][h].x, vw[1][h].y, vw[1][h].z, vw[1][h].w};
+            const uint32_t x2[4] = {vw[2][h].x, vw[2][h].y, vw[2][h].z, vw[2][h].w}, x3[4] = {vw[3][h].x, vw[3][h].y, vw[3][h].z, vw[3][h].w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;
+                mma_f16(o[8 * h + i], ph[0], pl[0], ph[1], pl[1], prmt(x0[i >> 1], x1[i >> 1], sel), prmt(x2[i >> 1], x3[i >> 1], sel));
+            }
+        }
+    }
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    if (c.r < p.rep) {
+        if (c.t == 0) p.part_ml[rec0 + c.r] = make_float2(m * 0.6931471805599453f, l);
+        if (first < tiles) {                              // the merge does not read the rows of a record without blocks
+            float* out = p.part + (rec0 + c.r) * D + 2 * VC * c.t;
+#pragma unroll
+            for (int i = 0; i < VC; i += 4) {
+                float a[4], b[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) { a[k] = (o[i + k][0] + o[i + k][2]) / kScale; b[k] = (o[i + k][1] + o[i + k][3]) / kScale; }
+                store_run<4>(out + i, a);
+                store_run<4>(out + VC + i, b);
+            }
         }
     }
 }
@@ -1623,7 +1657,8 @@ __device__ void consumer_loop(const Params& p, Smem<D, G>& sm, int* abort_flag) 
         const size_t rec_idx = (size_t)it.row * p.items_per_row + (size_t)(it.item / p.rows);
         const size_t rec0 = (rec_idx * kConsumerWarps + warp) * p.rep;
         if (it.level == 1) {
-            centroid_item<D, G, MASS>(p, c, it, sm.item_tab + is * kMaxItemBlocks, warp, rec0);
+            // a short item is the work of a few warps: they take turns
+            centroid_item<D, G, MASS>(p, c, it, sm.item_tab + is * kMaxItemBlocks, (warp + 4 * iseq) % kConsumerWarps, sm.sf[ib * 16 + c.r], rec0);
         }
         else if (it.level == 16) code = ring_item<D, G, 16, DUP, MASS>(
                 p, sm, c, it, stream, u0, u1, seq, rec0);
