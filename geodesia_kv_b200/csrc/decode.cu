@@ -524,9 +524,30 @@ static bool encode_rows(CUtensorMap* map, const uint8_t* data, size_t total_byte
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The four scale planes of the row form as one tensor (plane, block, bytes of a block): they may be four allocations, but
+// where they lie at equal distances (four parts of one buffer) a block's share of all four is a single box.
+static bool encode_planes(CUtensorMap* map, const mma::Params& p, int plane_bytes) {
+    TensorMapEncodeFn enc = tensor_map_encoder();
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p.klo), b = reinterpret_cast<uintptr_t>(p.kstep),
+                    c = reinterpret_cast<uintptr_t>(p.vlo), d = reinterpret_cast<uintptr_t>(p.vstep);
+    const size_t blocks = (size_t)p.rows * p.nb, apart = b - a;
+    if (!enc || b <= a || c - b != apart || d - c != apart || (a & 15) || (apart & 15) || apart < blocks * plane_bytes ||
+        apart >= ((size_t)1 << 40) || blocks > 0x7fffffffu)
+        return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)plane_bytes / 4, blocks, 4};
+    const cuuint64_t strides[2] = {(cuuint64_t)plane_bytes, apart};
+    const cuuint32_t box[3] = {(cuuint32_t)plane_bytes / 4, 1, 4};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<__half*>(p.klo), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int D, int G>
-static void make_tensor_maps(mma::TensorMaps& tm, const uint8_t* data, size_t total_bytes) {
+static void make_tensor_maps(mma::TensorMaps& tm, const mma::Params& p, size_t total_bytes) {
     memset(&tm, 0, sizeof(tm));
+    const uint8_t* data = p.data;
+    if (!p.paged) tm.planes_tiled = encode_planes(&tm.planes, p, mma::Cfg<D, G>::KSCALE) ? 1 : 0;
     if (reinterpret_cast<uintptr_t>(data) & 15) return;             // the copy engine wants a 16-byte aligned base
     bool ok = true;
     // rows per block = both halves of the block (2 x 64 token rows) in tile rows of w bytes
@@ -569,7 +590,7 @@ static int launch_mma2(const mma::Params& p, const mma::TensorMaps& tm, int grid
 template <int D, int G>
 static int launch_mma(const mma::Params& p, size_t total_bytes, int grid, cudaStream_t stream) {
     mma::TensorMaps tm;
-    make_tensor_maps<D, G>(tm, p.data, total_bytes);
+    make_tensor_maps<D, G>(tm, p, total_bytes);
     return p.rep <= 4 ? launch_mma2<D, G, true>(p, tm, grid, stream) : launch_mma2<D, G, false>(p, tm, grid, stream);
 }
 
