@@ -52,6 +52,16 @@ SIGNATURES = {
     "gkv_paged_demote_entries": (_i, [_vp] * 10 + [_i] * 4 + [_vp]),
     "gkv_paged_open_blocks": (_i, [_vp, _vp, _i] + [_vp] * 6),
     "gkv_paged_clear_table": (_i, [_vp] * 7 + [_i, _i, _vp]),
+    "gkv_pool_create": (_vp, [_i64, _i64] + [_vp] * 5),
+    "gkv_pool_destroy": (None, [_vp]),
+    "gkv_pool_stack": (_vp, [_vp, _i]),
+    "gkv_pool_alloc": (_i, [_vp, _i, _i64, _vp]),
+    "gkv_pool_free": (_i, [_vp, _i, _i64, _vp]),
+    "gkv_table_release": (_i, [_vp] * 3 + [_i64]),
+    "gkv_table_enter": (_i, [_vp] * 3 + [_i] * 3 + [_i64, _i] + [_vp] * 9),
+    "gkv_table_demotions": (_i64, [_vp, _vp] + [_i] * 3 + [_vp, _vp, _i]),
+    "gkv_table_plan_demotion": (_i, [_vp] * 3 + [_i] * 3 + [_vp, _vp, _i, _i64] + [_vp] * 5),
+    "gkv_table_apply_demotion": (_i, [_vp] * 3 + [_i64] + [_vp] * 5),
     "gkv_paged_plan_ratio_bytes": (_sz, [C.POINTER(_f), _i, _i]),
     "gkv_paged_plan_demotion": (_i, [_vp] * 5 + [_i64, C.POINTER(_f), C.c_double, _i, _i, _f, _f, _vp, _vp, _vp] + [_i] * 6 + [_vp]),
     "gkv_paged_unpack_blocks": (_i, [_vp] * 5 + [_i] * 4 + [_vp]),
@@ -70,8 +80,10 @@ class GkvError(RuntimeError):
 def bind(path) -> C.CDLL:
     """Open a build of the library and attach the signatures of the header to it."""
     lib = C.CDLL(str(path))
+    held = C.PyDLL(str(path), handle=lib._handle)      # host bookkeeping: short, and one caller at a time
     for name, (res, args) in SIGNATURES.items():
-        fn = getattr(lib, name)          # AttributeError here = header and library disagree
+        fn = getattr(held if name.startswith(("gkv_pool_", "gkv_table_")) else lib, name)   # AttributeError here = header and library disagree
+        setattr(lib, name, fn)
         fn.restype, fn.argtypes = res, args
     return lib
 

@@ -178,13 +178,15 @@ class _Extension:
         if offs.dtype != torch.int64 or level.dtype != torch.int32 or valid.dtype != torch.int32:
             raise RuntimeError("offs must be int64, level and valid int32")
         G, gv = (64 + group - 1) // group, (D + group - 1) // group
-        for name, t, shp in (("klo", klo, (B, Hkv, nb, G, D)), ("kstep", kstep, (B, Hkv, nb, G, D)),
-                             ("vlo", vlo, (B, Hkv, nb, 64, gv)), ("vstep", vstep, (B, Hkv, nb, 64, gv))):
-            if t.dtype != torch.float16 or tuple(t.shape) != shp:
-                raise RuntimeError(f"{name} must be float16 of shape {shp}, got {t.dtype} {tuple(t.shape)}")
+        ks, vs, half = (B, Hkv, nb, G, D), (B, Hkv, nb, 64, gv), torch.float16
+        if not (klo.shape == ks and kstep.shape == ks and vlo.shape == vs and vstep.shape == vs and
+                klo.dtype == kstep.dtype == vlo.dtype == vstep.dtype == half):
+            for name, t, shp in (("klo", klo, ks), ("kstep", kstep, ks), ("vlo", vlo, vs), ("vstep", vstep, vs)):
+                if t.dtype != half or tuple(t.shape) != shp:
+                    raise RuntimeError(f"{name} must be float16 of shape {shp}, got {t.dtype} {tuple(t.shape)}")
         dev = q.device
-        q, data, offs, level, valid = (t.contiguous() for t in (q, data, offs, level, valid))
-        klo, kstep, vlo, vstep = (t.contiguous() for t in (klo, kstep, vlo, vstep))
+        q, data, offs, level, valid = q.contiguous(), data.contiguous(), offs.contiguous(), level.contiguous(), valid.contiguous()
+        klo, kstep, vlo, vstep = klo.contiguous(), kstep.contiguous(), vlo.contiguous(), vstep.contiguous()
         if mass:
             with on(dev):
                 stream, capturing = _stream(dev), torch.cuda.is_current_stream_capturing()

@@ -25,6 +25,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import weakref
 from typing import Sequence
 
 import numpy as np
@@ -45,17 +46,29 @@ def ladder_index_np(level: np.ndarray) -> np.ndarray:
     return (lv <= 8).astype(np.int32) + (lv <= 4) + (lv <= 2) + (lv <= 1)
 
 
+_E_ARG, _E_POOL, _E_MEMORY = -6, -8, -9              # include/geodesia_kv_b200.h
+
+
+def _addr(a: np.ndarray) -> int:
+    return a.ctypes.data
+
+
+def _lists(*sizes_and_types):
+    """Host arrays side by side in one buffer, each from an 8-byte boundary: (buffer, arrays, their byte offsets)."""
+    starts, end = [], 0
+    for n, t in sizes_and_types:
+        starts.append(end)
+        end += (n * np.dtype(t).itemsize + 7) // 8 * 8
+    buf = np.empty(end, dtype=np.uint8)
+    return buf, [buf[at:at + n * np.dtype(t).itemsize].view(t) for (n, t), at in zip(sizes_and_types, starts)], starts
+
+
 class PoolExhausted(RuntimeError):
     pass
 
 
 class PagedPool:
     """Byte pool with one free list per rung (host-side bookkeeping, device-side bytes)."""
-
-    # Slots moved are counted per slab by a histogram over all slabs in pools of up to so many (or of no more than the
-    # slots moved), by indexing the slabs touched in longer ones.  alloc and free of 64
-    # slots: 22.3 us against 23.1 at 500 slabs, 23.1 against 22.9 at 1000, 36.5 against 22.9 at 8000; of 16 at 110,000: 268 against 15.
-    HISTOGRAM_SLABS = 1000
 
     def __init__(self, capacity_bytes: int, D: int = 128, group: int = 32, device="cuda"):
         lib = _lib.load()
@@ -71,15 +84,42 @@ class PagedPool:
         if self.n_slabs < 1:
             raise ValueError(f"capacity below one slab of {self.slab_bytes} bytes")
         self.data = torch.empty(self.n_slabs * self.slab_bytes, dtype=torch.uint8, device=self.device)
-        self._free_slabs = list(range(self.n_slabs - 1, -1, -1))
+        # The bookkeeping itself is native (csrc/pool.cu); these arrays are its memory, the stacks of free slots are its own.
         self._slab_rung = np.zeros(self.n_slabs, dtype=np.int32)           # 0 = unassigned
         self._slab_live = np.zeros(self.n_slabs, dtype=np.int64)
-        self._stack = {r: np.empty(0, dtype=np.int64) for r in LADDER}     # free slot offsets per rung
-        self._top = {r: 0 for r in LADDER}
-        self.bytes_in_use = 0            # bytes of the slots handed out
-        self.peak_bytes_in_use = 0
+        self._slabs = np.empty(self.n_slabs, dtype=np.int64)
+        self._counters = np.zeros(8, dtype=np.int64)     # free slabs, bytes in use, their peak, height of each rung's stack
+        self.lib = lib
+        self.handle = lib.gkv_pool_create(self.slab_bytes, self.n_slabs, (C.c_int64 * 5)(*(self.slot[r] for r in LADDER)),
+                                          _addr(self._slab_rung), _addr(self._slab_live), _addr(self._slabs), _addr(self._counters))
+        if not self.handle:
+            raise MemoryError("no memory for the pool's bookkeeping")
+        weakref.finalize(self, lib.gkv_pool_destroy, self.handle)
 
     # -- accounting ---------------------------------------------------------------------------
+    @property
+    def bytes_in_use(self) -> int:
+        """Bytes of the slots handed out."""
+        return int(self._counters[1])
+
+    @property
+    def peak_bytes_in_use(self) -> int:
+        return int(self._counters[2])
+
+    @property
+    def _free_slabs(self) -> list:
+        return self._slabs[:self._counters[0]].tolist()
+
+    @property
+    def _top(self) -> dict:
+        return {r: int(self._counters[3 + i]) for i, r in enumerate(LADDER)}
+
+    @property
+    def _stack(self) -> dict:
+        """Free slot offsets of every rung (a copy)."""
+        return {r: np.array((C.c_int64 * n).from_address(self.lib.gkv_pool_stack(self.handle, i)) if n else (), dtype=np.int64)
+                for i, (r, n) in enumerate(self._top.items())}
+
     @property
     def capacity_bytes(self) -> int:
         return self.n_slabs * self.slab_bytes
@@ -87,74 +127,33 @@ class PagedPool:
     @property
     def bytes_reserved(self) -> int:
         """Bytes of the slabs that currently belong to a rung (slot granularity is bytes_in_use)."""
-        return (self.n_slabs - len(self._free_slabs)) * self.slab_bytes
+        return (self.n_slabs - int(self._counters[0])) * self.slab_bytes
 
     def slots_in_use(self, rung: int) -> int:
         return int(self._slab_live[self._slab_rung == rung].sum())
 
     # -- allocation ---------------------------------------------------------------------------
-    def _push(self, rung: int, offs: np.ndarray) -> None:
-        st, top = self._stack[rung], self._top[rung]
-        if top + offs.size > st.size:
-            grown = np.empty(max(2 * st.size, top + offs.size, 1024), dtype=np.int64)
-            grown[:top] = st[:top]
-            self._stack[rung] = st = grown
-        st[top:top + offs.size] = offs
-        self._top[rung] = top + offs.size
+    def _check(self, rc: int, what: str) -> None:
+        if rc == _E_POOL:
+            raise PoolExhausted(f"pool of {self.capacity_bytes} bytes exhausted asking for {what} ({self.bytes_in_use} bytes in use)")
+        if rc == _E_MEMORY:
+            raise MemoryError("no memory for the pool's bookkeeping")
+        if rc == _E_ARG:
+            raise ValueError("an offset does not belong to a slab of its rung, or an entry lies beyond the table")
+        _lib.check(rc, "pool")
 
     def alloc(self, rung: int, n: int) -> np.ndarray:
-        """Offsets of n free slots of a rung (int64)."""
-        if n <= 0:
-            return np.empty(0, dtype=np.int64)
-        size = self.slot[rung]
-        per_slab = self.slab_bytes // size
-        need = max(0, -(-(n - self._top[rung]) // per_slab))
-        if need:
-            if len(self._free_slabs) < need:             # refused with every slab where it was: smaller slots may still fit
-                raise PoolExhausted(f"pool of {self.capacity_bytes} bytes exhausted asking for {n} slots of rung {rung} "
-                                    f"({self.bytes_in_use} bytes in use)")
-            s = np.array([self._free_slabs.pop() for _ in range(need)], dtype=np.int64)
-            self._slab_rung[s] = rung
-            # pushed high to low, so low addresses are handed out first
-            self._push(rung, (s[:, None] * self.slab_bytes + np.arange(per_slab - 1, -1, -1, dtype=np.int64) * size).reshape(-1))
-        top = self._top[rung]
-        out = self._stack[rung][top - n:top][::-1].copy()
-        self._top[rung] = top - n
-        slabs = out // self.slab_bytes
-        if self.n_slabs <= self.HISTOGRAM_SLABS or self.n_slabs <= n:
-            self._slab_live += np.bincount(slabs, minlength=self.n_slabs)
-        else:
-            np.add.at(self._slab_live, slabs, 1)
-        self.bytes_in_use += n * size
-        self.peak_bytes_in_use = max(self.peak_bytes_in_use, self.bytes_in_use)
+        """Offsets of n free slots of a rung (int64); refused with every slab where it was: smaller slots may still fit."""
+        out = np.empty(max(int(n), 0), dtype=np.int64)
+        if out.size:
+            self._check(self.lib.gkv_pool_alloc(self.handle, LADDER.index(rung), out.size, _addr(out)), f"{n} slots of rung {rung}")
         return out
 
     def free(self, rung: int, offs: np.ndarray) -> None:
         """Give slots of a rung back; slabs left without a live slot return to the common list."""
-        offs = np.asarray(offs, dtype=np.int64)
-        if offs.size == 0:
-            return
-        slabs = offs // self.slab_bytes
-        if np.any(self._slab_rung[slabs] != rung):
-            raise ValueError("a freed offset does not belong to a slab of that rung")
-        if self.n_slabs <= self.HISTOGRAM_SLABS or self.n_slabs <= slabs.size:
-            gone = np.bincount(slabs, minlength=self.n_slabs)
-            self._slab_live -= gone
-            empty = np.nonzero((gone > 0) & (self._slab_live == 0))[0]
-        else:
-            np.subtract.at(self._slab_live, slabs, 1)
-            idle = slabs[self._slab_live[slabs] == 0]
-            empty = np.unique(idle) if idle.size else idle
-        self.bytes_in_use -= offs.size * self.slot[rung]
-        self._push(rung, offs)
-        if empty.size:
-            self._slab_rung[empty] = 0
-            top = self._top[rung]
-            st = self._stack[rung][:top]
-            keep = st[self._slab_rung[st // self.slab_bytes] == rung]       # the stack's other slots are of slabs in use
-            self._stack[rung][:keep.size] = keep
-            self._top[rung] = keep.size
-            self._free_slabs.extend(empty[::-1].tolist())
+        offs = np.ascontiguousarray(offs, dtype=np.int64)
+        if offs.size:
+            self._check(self.lib.gkv_pool_free(self.handle, LADDER.index(rung), offs.size, _addr(offs)), "a release")
 
 
 class PagedLayerCache:
@@ -205,16 +204,9 @@ class PagedLayerCache:
     def _row_blocks(self) -> np.ndarray:
         return np.repeat(self.blocks_per_seq(), self.Hkv)
 
-    def _upload(self, *arrays: np.ndarray):
-        """Host arrays -> (device buffer, their addresses in it), all in ONE copy, each 8-byte aligned.  The caller
-        holds the buffer until its kernel is launched; after that the stream order of the allocator protects it."""
-        starts, end = [], 0
-        for a in arrays:
-            starts.append(end)
-            end += (a.nbytes + 7) // 8 * 8
-        buf = np.empty(end, dtype=np.uint8)
-        for a, at in zip(arrays, starts):
-            buf[at:at + a.nbytes] = np.ascontiguousarray(a).view(np.uint8)
+    def _upload(self, buf: np.ndarray, starts):
+        """A buffer of host arrays -> (device buffer, the arrays' addresses in it), in ONE copy.  The caller holds the
+        buffer until its kernel is launched; after that the stream order of the allocator protects it."""
         staged = torch.from_numpy(buf).to(self.device, non_blocking=True)
         base = staged.data_ptr()
         return staged, [base + at for at in starts]
@@ -234,36 +226,24 @@ class PagedLayerCache:
         nblk = (lengths + BLOCK - 1) // BLOCK
         if int(nblk.max()) + 1 > self.cap:
             self._grow(int(nblk.max()) + 1 + 16)
-        rows_b = np.repeat(np.arange(B), Hkv)
-        row_nblk = np.repeat(nblk, Hkv)
-        total = int(row_nblk.sum())
-        row_of = np.repeat(np.arange(self.rows), row_nblk)                        # row of every block
-        blk_of = np.arange(total) - np.repeat(np.cumsum(row_nblk) - row_nblk, row_nblk)
-        if int(self.offs_h.max(initial=-1)) < 0:
-            slots = self.pool.alloc(16, total)
-        else:                                                                     # slots reserved earlier are used first
-            slots = self.offs_h[row_of, blk_of]
-            fresh = np.nonzero(slots < 0)[0]
-            slots[fresh] = self.pool.alloc(16, fresh.size)
-        src_off = (row_of * T + blk_of * BLOCK) * D
-        nvalid = np.minimum(BLOCK, lengths[rows_b[row_of]] - blk_of * BLOCK).astype(np.int32)
-        self.offs_h[row_of, blk_of] = slots
-        self.level_h[row_of, blk_of] = 16
+        self._enter(k, v, np.zeros(B, dtype=np.int64), nblk, T, lengths, fresh=False)
         self.len_h[:] = lengths
-        self._enter(k, v, src_off, nvalid, slots, row_of * self.cap + blk_of, fresh=False,
-                    row_len=lengths[rows_b[row_of]].astype(np.int32))
 
-    def _enter(self, k, v, src_off, nvalid, slots, flat, fresh: bool, row_len=None, len_add: int = 0, per_row: int = 0) -> None:
-        """Pack blocks into rung-16 slots and enter them into the table: one upload, one kernel.  ``fresh``
-        clears the entries' mass and radii; the row lengths are set from ``row_len`` (per block) or advanced
-        by ``len_add`` (rows of ``per_row`` consecutive blocks)."""
-        n, dev = int(flat.size), self.device
-        arrays = [src_off.astype(np.int64, copy=False), slots, flat.astype(np.int64, copy=False),
-                  np.ascontiguousarray(nvalid, dtype=np.int32), np.full(n, 16, dtype=np.int32)]
-        if row_len is not None:
-            arrays.append(row_len)
+    def _enter(self, k, v, first: np.ndarray, count: np.ndarray, T: int, tokens, fresh: bool, len_add: int = 0, per_row: int = 0) -> None:
+        """Give every sequence ``count`` blocks from block ``first`` on, at rung 16, in the slots reserved for them or new
+        ones, and pack them: one upload, one kernel.  ``fresh`` clears the entries' mass and radii; the row lengths are set
+        from ``tokens`` (valid tokens per sequence; None: whole blocks) or advanced by ``len_add`` (rows of ``per_row`` blocks)."""
+        dev, n = self.device, int(count.sum()) * self.Hkv
+        i64, i32 = np.int64, np.int32
+        buf, (so, sl, at, nv, lv, *rl), starts = _lists((n, i64), (n, i64), (n, i64), (n, i32), (n, i32), *([(n, i32)] if tokens is not None else []))
+        first, count = np.ascontiguousarray(first, dtype=i64), np.ascontiguousarray(count, dtype=i64)
+        tokens = None if tokens is None else np.ascontiguousarray(tokens, dtype=i64)
+        rc = self.lib.gkv_table_enter(self.pool.handle, _addr(self.offs_h), _addr(self.level_h), self.B, self.Hkv, self.cap, T, self.D,
+                                      _addr(first), _addr(count), None if tokens is None else _addr(tokens), _addr(so), _addr(sl),
+                                      _addr(at), _addr(nv), _addr(lv), _addr(rl[0]) if rl else None)
+        self.pool._check(rc, f"the slots of {n} blocks")
         with on(dev):
-            staged, (src, dst, at, nv, lv, *rl) = self._upload(*arrays)
+            staged, (src, dst, at, nv, lv, *rl) = self._upload(buf, starts)
             rc = self.lib.gkv_paged_enter_blocks(k.data_ptr(), v.data_ptr(), _DT[k.dtype], src, int(self.D), nv,
                                                  self.pool.data.data_ptr(), dst, lv, at, self.offs.data_ptr(),
                                                  self.level.data_ptr(), self.valid.data_ptr(),
@@ -283,17 +263,8 @@ class PagedLayerCache:
         first = self.len_h // BLOCK
         if int(first.max()) + n + 1 > self.cap:
             self._grow(int(first.max()) + n + 1 + 63)
-        row_of = np.repeat(np.arange(self.rows), n)
-        blk_in = np.tile(np.arange(n), self.rows)
-        blk_of = np.repeat(first, Hkv * n) + blk_in
-        slots = self.offs_h[row_of, blk_of].copy()                      # slots reserved earlier are used first
-        fresh = np.nonzero(slots < 0)[0]
-        slots[fresh] = self.pool.alloc(16, fresh.size)
-        self.offs_h[row_of, blk_of] = slots
-        self.level_h[row_of, blk_of] = 16
+        self._enter(k, v, first, np.full(B, n, dtype=np.int64), T, None, fresh=True, len_add=T, per_row=n)
         self.len_h += T
-        self._enter(k, v, (row_of * T + blk_in * BLOCK) * D, np.full(slots.size, BLOCK, np.int32), slots,
-                    row_of * self.cap + blk_of, fresh=True, len_add=T, per_row=n)
 
     def pack_blocks(self, k, v, src_off, token_stride, nvalid, slots, levels, radii: bool = False):
         """Quantise blocks from dense rows into given slots (element offsets into k and v)."""
@@ -313,7 +284,7 @@ class PagedLayerCache:
 
     def append(self, k_new: torch.Tensor, v_new: torch.Tensor) -> None:
         """One more token for every sequence: k_new, v_new (B, Hkv, 1, D) or (B, Hkv, D)."""
-        if np.any(self.len_h % BLOCK == 0):                               # some sequence opens a new block
+        if (self.len_h % BLOCK == 0).any():                               # some sequence opens a new block
             self.reserve(1)
         self.append_device(k_new, v_new)
         self.len_h += 1
@@ -339,7 +310,9 @@ class PagedLayerCache:
         self.level_h[rows, blks] = 16
         flat, dev = rows * self.cap + blks, self.device
         with on(dev):
-            staged, (at, so) = self._upload(flat.astype(np.int64, copy=False), slots)
+            buf, (a, b), starts = _lists((flat.size, np.int64), (slots.size, np.int64))
+            a[:], b[:] = flat, slots
+            staged, (at, so) = self._upload(buf, starts)
             rc = self.lib.gkv_paged_open_blocks(at, so, int(flat.size), self.offs.data_ptr(), self.level.data_ptr(),
                                                 self.mass.data_ptr(), self.ek.data_ptr(), self.ev.data_ptr(), _stream(dev))
         _lib.check(rc, "gkv_paged_open_blocks")
@@ -351,9 +324,9 @@ class PagedLayerCache:
     def append_device(self, k_new: torch.Tensor, v_new: torch.Tensor) -> None:
         """The device half of :meth:`append` (no host bookkeeping): safe inside a CUDA graph as long
         as no row crosses into a block without a slot — the status word says if one did."""
-        k_new, v_new = k_new.reshape(self.rows, self.D), v_new.reshape(self.rows, self.D)
-        if not (k_new.is_contiguous() and v_new.is_contiguous()):
-            k_new, v_new = k_new.contiguous(), v_new.contiguous()
+        n = self.rows * self.D
+        if not (k_new.numel() == v_new.numel() == n and k_new.is_contiguous() and v_new.is_contiguous()):
+            k_new, v_new = k_new.reshape(self.rows, self.D).contiguous(), v_new.reshape(self.rows, self.D).contiguous()
         dev = self.device
         with on(dev):
             rc = self.lib.gkv_paged_append_token(k_new.data_ptr(), v_new.data_ptr(), _DT[k_new.dtype],
@@ -393,7 +366,7 @@ class PagedLayerCache:
     def observe(self, mass: torch.Tensor, decay: float) -> None:
         """Fold one step's per-block mass (rows, nb) into the running mass (policies.py:705-708)."""
         nb = mass.shape[1]
-        self.mass[:, :nb].lerp_(mass, 1.0 - decay)
+        (self.mass if nb == self.cap else self.mass[:, :nb]).lerp_(mass, 1.0 - decay)
 
     # -- maintenance ----------------------------------------------------------------------------
     def hot_blocks(self, nb: int, sinks: int = 4, window: int = 128) -> torch.Tensor:
@@ -446,42 +419,25 @@ class PagedLayerCache:
     def apply_demotion(self, tgt_idx_host: np.ndarray) -> int:
         """Demote to the allocator's result (host array (rows, nb) of ladder indices): allocate the
         smaller slots, re-quantise on the device, free the larger slots.  Returns blocks demoted."""
-        nb = tgt_idx_host.shape[1]
-        cur = self.level_h[:, :nb]
-        new = _LADDER_NP[np.clip(tgt_idx_host, 0, 4)]
-        used = np.arange(nb)[None, :] < self._row_blocks()[:, None]
-        r, b = np.nonzero((new < cur) & used & (self.offs_h[:, :nb] >= 0))
-        n = int(r.size)
+        tgt = np.ascontiguousarray(np.broadcast_to(tgt_idx_host, (self.rows, tgt_idx_host.shape[1])), dtype=np.int32)
+        nb, lib, dev = tgt.shape[1], self.lib, self.device
+        blocks = self.blocks_per_seq()
+        table = (_addr(self.offs_h), _addr(self.level_h), self.B, self.Hkv, self.cap, _addr(blocks), _addr(tgt), nb)
+        n = int(lib.gkv_table_demotions(*table))
         if n == 0:
             return 0
-        lv_old, lv_new = cur[r, b].copy(), new[r, b].astype(np.int32)
-        off_old = self.offs_h[r, b].copy()
-        off_new = np.empty(n, dtype=np.int64)
-        taken = []
-        try:
-            for rung in LADDER[1:]:
-                sel = np.nonzero(lv_new == rung)[0]
-                if sel.size:
-                    off_new[sel] = self.pool.alloc(rung, sel.size)
-                    taken.append((rung, sel))
-        except PoolExhausted:
-            for rung, sel in taken:
-                self.pool.free(rung, off_new[sel])
-            raise
-        dev = self.device
+        i64, i32 = np.int64, np.int32
+        buf, lists, starts = _lists((n, i64), (n, i64), (n, i64), (n, i32), (n, i32))
+        old, new, at, lo, ln = map(_addr, lists)
+        self.pool._check(lib.gkv_table_plan_demotion(self.pool.handle, *table, n, old, new, at, lo, ln), f"the slots of {n} demoted blocks")
         with on(dev):
-            staged, (old, new, at, lo, ln) = self._upload(off_old, off_new, r * self.cap + b, lv_old, lv_new)
-            rc = self.lib.gkv_paged_demote_entries(self.pool.data.data_ptr(), old, lo, new, ln, at, self.offs.data_ptr(),
-                                                   self.level.data_ptr(), self.ek.data_ptr(), self.ev.data_ptr(), n, self.D,
-                                                   BLOCK, self.group, _stream(dev))
+            staged, (d_old, d_new, d_at, d_lo, d_ln) = self._upload(buf, starts)
+            rc = lib.gkv_paged_demote_entries(self.pool.data.data_ptr(), d_old, d_lo, d_new, d_ln, d_at, self.offs.data_ptr(),
+                                              self.level.data_ptr(), self.ek.data_ptr(), self.ev.data_ptr(), n, self.D,
+                                              BLOCK, self.group, _stream(dev))
         _lib.check(rc, "gkv_paged_demote_entries")
-        self.offs_h[r, b] = off_new
-        self.level_h[r, b] = lv_new
         # the old slots are free for whatever is launched after the demotion kernel on this stream
-        for rung in LADDER[:-1]:
-            sel = np.nonzero(lv_old == rung)[0]
-            if sel.size:
-                self.pool.free(rung, off_old[sel])
+        self.pool._check(lib.gkv_table_apply_demotion(self.pool.handle, *table[:2], n, old, new, at, lo, ln), "a release")
         return n
 
     def maintain(self, budget_bits: float, **kw) -> int:
@@ -505,13 +461,7 @@ class PagedLayerCache:
 
     def release(self) -> None:
         """Give every slot back to the pool, also those that :meth:`reserve` opened and no token has reached."""
-        held = self.offs_h >= 0
-        for rung in LADDER:
-            sel = held & (self.level_h == rung)
-            if sel.any():
-                self.pool.free(rung, self.offs_h[sel])
-        self.offs_h[:] = -1
-        self.level_h[:] = 0
+        self.pool._check(self.lib.gkv_table_release(self.pool.handle, _addr(self.offs_h), _addr(self.level_h), self.offs_h.size), "a release")
         self.len_h[:] = 0
         dev = self.device
         with on(dev):

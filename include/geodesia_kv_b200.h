@@ -47,6 +47,8 @@ extern "C" {
 #define GKV_E_CUDA (-5)      /* a CUDA call failed; see gkv_last_cuda_error()             */
 #define GKV_E_ARG (-6)       /* an argument is out of range                               */
 #define GKV_E_STATIC_SCRATCH (-7) /* gkv_mixed_attn_decode_static: problem exceeds the built-in scratch */
+#define GKV_E_POOL (-8)      /* the block pool has no slots left for the request          */
+#define GKV_E_MEMORY (-9)    /* host memory ran out                                       */
 
 int gkv_abi_version(void);
 const char *gkv_error_string(int code); /* host string, static storage */
@@ -335,6 +337,39 @@ int gkv_paged_open_blocks(const int64_t *flat, const int64_t *offs, int n, int64
 /* A table without blocks: offs -1; level, valid, mass, the radii and the row lengths 0. */
 int gkv_paged_clear_table(int64_t *offs, int32_t *level, int32_t *valid, float *mass, float *ek, float *ev,
                           int32_t *lens, int rows, int cap, void *stream);
+
+/* Host bookkeeping of a block pool cut into n_slabs slabs of slab_bytes, each serving one rung (slot_bytes[5], by
+ * ladder index: rungs 16, 8, 4, 2, centroid); no CUDA call.  slab_rung (0 = unassigned) and slab_live (n_slabs each),
+ * free_slabs (n_slabs) and counters[8] (free slabs, bytes in use, their peak, height of each rung's stack of free
+ * slots) are the caller's memory and stay readable.  Slots are handed out low addresses first; a slab returns to the
+ * common list with its last slot.  alloc: GKV_E_POOL and no change when the request does not fit; free: GKV_E_ARG and
+ * no change when an offset is not of a slab of that rung.  Calls on one pool must not overlap.                       */
+void *gkv_pool_create(int64_t slab_bytes, int64_t n_slabs, const int64_t *slot_bytes, int32_t *slab_rung,
+                      int64_t *slab_live, int64_t *free_slabs, int64_t *counters);
+void gkv_pool_destroy(void *pool);
+const int64_t *gkv_pool_stack(void *pool, int rung_index);
+int gkv_pool_alloc(void *pool, int rung_index, int64_t n, int64_t *out);
+int gkv_pool_free(void *pool, int rung_index, int64_t n, const int64_t *offs);
+
+/* The host mirror (offs, level) of a block table of B * Hkv rows of `cap` entries, offs -1 where there is no slot.
+ * release: every slot back to the pool, the table empty.  enter: sequence b gets count[b] blocks from block first[b]
+ * on, at rung 16, in the slots its entries already hold or new ones; the lists of the launch that packs them
+ * (gkv_paged_enter_blocks) are filled, rows of T tokens of D elements, valid counts and row lengths from tokens[b]
+ * (NULL: whole blocks).  demotions: how many entries of the first blocks[b] the targets (rows, nb; ladder indices)
+ * demote; plan: the lists of the launch (gkv_paged_demote_entries) for those n, with new slots taken; apply: the table
+ * follows, the old slots go back.  What is refused (GKV_E_POOL) changes nothing.                                     */
+int gkv_table_release(void *pool, int64_t *offs, int32_t *level, int64_t entries);
+int gkv_table_enter(void *pool, int64_t *offs, int32_t *level, int B, int Hkv, int cap, int64_t T, int D,
+                    const int64_t *first, const int64_t *count, const int64_t *tokens, int64_t *src_off,
+                    int64_t *slots, int64_t *flat, int32_t *nvalid, int32_t *rung, int32_t *row_len);
+int64_t gkv_table_demotions(const int64_t *offs, const int32_t *level, int B, int Hkv, int cap,
+                            const int64_t *blocks, const int32_t *tgt, int nb);
+int gkv_table_plan_demotion(void *pool, const int64_t *offs, const int32_t *level, int B, int Hkv, int cap,
+                            const int64_t *blocks, const int32_t *tgt, int nb, int64_t n, int64_t *off_old,
+                            int64_t *off_new, int64_t *flat, int32_t *level_old, int32_t *level_new);
+int gkv_table_apply_demotion(void *pool, int64_t *offs, int32_t *level, int64_t n, const int64_t *off_old,
+                             const int64_t *off_new, const int64_t *flat, const int32_t *level_old,
+                             const int32_t *level_new);
 
 /* Distortion table and rung allocation (gkv_block_distortion, gkv_allocate_ragged) straight from a block
  * table: the ladder index follows from level, the blocks in use and what must stay exact (the first
