@@ -157,6 +157,8 @@ struct Params {
     int chunk;               // blocks per item (the last item of a rung's run may be shorter)
     int items_per_row, items;
     int per_row_meta;
+    int dealt;               // 1: CTA i takes the items i, i + grid, ...; 0: items are drawn from the counter
+    int clear_status;        // 1: this kernel is the first of its call and clears the status word itself
     int rows;
     int paged;               // 1: `data` is a block pool, offs are pool offsets, and the four scale planes of a quantised
                              // block sit right behind its bytes ([klo][kstep][vlo][vstep]); klo..vstep above are unused
@@ -728,16 +730,20 @@ __device__ __forceinline__ bool produce_item(const Params& p, const TensorMaps& 
 template <int D, int G>
 __device__ void scheduler_loop(const Params& p, Smem<D, G>& sm, int* abort_flag) {
     const int lane = threadIdx.x & 31;
-    int tot0 = 0, tot1 = 0, nfirst = 0;
+    int tot0 = 0, tot1 = 0, nfirst = 0, drawn = 0;
     bool ok = true;
     grid_wait();            // block lists, work counter and status word: this warp alone reads the first two, and everything
                             // the other warps do follows from what it announces
+    if (p.clear_status && blockIdx.x == 0 && lane == 0) *p.status = 0;      // whoever gives up sets it after milliseconds of waiting
     for (int j = 0; ok; ++j) {
         ItemDesc it;
         for (;;) {                                          // draw the next item that has blocks
             int id = 0;
-            if (lane == 0) id = atomicAdd(p.counter, 1);
-            id = __shfl_sync(0xffffffffu, id, 0);
+            if (p.dealt) id = (int)blockIdx.x + (int)gridDim.x * drawn++;
+            else {
+                if (lane == 0) id = atomicAdd(p.counter, 1);
+                id = __shfl_sync(0xffffffffu, id, 0);
+            }
             const Span sp = span_of(p, id);                 // same loads in every lane (broadcast)
             it.item = id; it.row = sp.row; it.level = sp.level; it.b_lo = sp.b_lo; it.nblk = sp.nblk;
             it.exit = id >= p.items ? 1 : 0;

@@ -70,3 +70,14 @@ def test_planes_at_equal_distances_and_apart_give_the_same_bits(ext, rep, D, gro
     odd = pool[4 * n:5 * n + 8]                                             # one plane at an address of its own
     three = ext.mixed_attn_decode(q, c.data, c.offs, c.klo, c.kstep, c.vlo, odd[8:].view(c.vstep.shape).copy_(c.vstep), c.level, c.valid, 64, group)
     assert torch.equal(one, two) and torch.equal(one, three)
+
+
+@pytest.mark.parametrize("nb", [419, 420, 421, 427])       # two rows: 148 item slots up to 420 blocks, 150 and 152 beyond
+def test_calls_around_one_item_slot_per_cta_start_from_any_scratch(ext, oracle, nb):
+    ext.set_decode_item_blocks(6)
+    c = oracle_cache(oracle, nb, 1, 2, nb, 128, 32, last_valid=11)
+    attend(ext, oracle, c, 8)
+    for ws in ext._workspaces.values():
+        ws.fill_(0xff)                                       # counter and status word hold anything before a call
+    attend(ext, oracle, c, 8)
+    assert ext.decode_status() == 0
