@@ -17,7 +17,7 @@ GPU at a bit budget (``README.md:243-248``) — needs demotion to hand memory ba
   the per-block softmax mass as a by-product), and maintenance runs the distortion, allocator and
   demotion kernels for all rows at once.
 
-Free lists live on the host (numpy): a maintenance step reads the allocator's result back once,
+Free lists and block tables are mirrored on the host (native code over numpy arrays): a maintenance step reads the allocator's result back once,
 for all rows (and, through :class:`PagedKVCache.maintain`, for all layers), which is the only
 host synchronisation of the serving loop; decode steps in between launch kernels only.
 """
