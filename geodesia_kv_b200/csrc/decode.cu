@@ -516,17 +516,20 @@ static TensorMapEncodeFn tensor_map_encoder() {
     return fn;
 }
 
-// The cache as a matrix of w-byte rows, a block as a box of `rows` of them.
-static bool encode_rows(CUtensorMap* map, const uint8_t* data, size_t total_bytes, int w, int rows) {
+// The cache as a matrix of w-byte rows, a block as a box of `rows` of them; `lines`: the rows in groups of kLineBytes.
+static bool encode_rows(CUtensorMap* map, const uint8_t* data, size_t total_bytes, int w, int rows, bool lines) {
     TensorMapEncodeFn enc = tensor_map_encoder();
-    if (!enc || w < 32 || rows > 256 || total_bytes / (size_t)w == 0) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)w, (cuuint64_t)(total_bytes / (size_t)w)};
-    const cuuint64_t strides[1] = {(cuuint64_t)w};
-    const cuuint32_t box[2] = {(cuuint32_t)w, (cuuint32_t)rows};
-    const cuuint32_t estr[2] = {1, 1};
+    const int per = lines ? mma::kLineBytes / w : rows;          // rows of the second dimension
+    if (!enc || w < 32 || rows > 256 || rows % per || total_bytes / (size_t)w == 0) return false;
+    const cuuint64_t groups = total_bytes / mma::kLineBytes;
+    if ((lines ? groups : total_bytes / (size_t)w) > 0x7fffffffu) return false;      // beyond the coordinates
+    const cuuint64_t dims[3] = {(cuuint64_t)w, lines ? (cuuint64_t)per : (cuuint64_t)(total_bytes / (size_t)w), groups};
+    const cuuint64_t strides[2] = {(cuuint64_t)w, (cuuint64_t)mma::kLineBytes};
+    const cuuint32_t box[3] = {(cuuint32_t)w, (cuuint32_t)per, (cuuint32_t)(rows / per)};
+    const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapSwizzle sw = w == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : w == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
                                                                                    : CU_TENSOR_MAP_SWIZZLE_32B;
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(data), dims, strides, box, estr,
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, lines ? 3 : 2, const_cast<uint8_t*>(data), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -557,14 +560,17 @@ static void make_tensor_maps(mma::TensorMaps& tm, const mma::Params& p, size_t t
     if (!p.paged) tm.planes_tiled = encode_planes(&tm.planes, p, mma::Cfg<D, G>::KSCALE) ? 1 : 0;
     if (reinterpret_cast<uintptr_t>(data) & 15) return;             // the copy engine wants a 16-byte aligned base
     bool ok = true;
+    constexpr int narrow = mma::Lay<D, G, 4>::TILED ? mma::Lay<D, G, 4>::W : mma::Lay<D, G, 8>::W;
+    const bool lines = total_bytes / narrow > 0x7fffffffu;
     // rows per block = both halves of the block (2 x 64 token rows) in tile rows of w bytes
-    { using L = mma::Lay<D, G, 16>; ok = ok && encode_rows(&tm.m[0], data, total_bytes, L::W, 2 * kP * L::RB / L::W); }
-    { using L = mma::Lay<D, G, 8>;  ok = ok && encode_rows(&tm.m[1], data, total_bytes, L::W, 2 * kP * L::RB / L::W); }
+    { using L = mma::Lay<D, G, 16>; ok = ok && encode_rows(&tm.m[0], data, total_bytes, L::W, 2 * kP * L::RB / L::W, lines); }
+    { using L = mma::Lay<D, G, 8>;  ok = ok && encode_rows(&tm.m[1], data, total_bytes, L::W, 2 * kP * L::RB / L::W, lines); }
     if (mma::Lay<D, G, 4>::TILED) {
         using L = mma::Lay<D, G, 4>;
-        ok = ok && encode_rows(&tm.m[2], data, total_bytes, L::W, 2 * kP * L::RB / L::W);
+        ok = ok && encode_rows(&tm.m[2], data, total_bytes, L::W, 2 * kP * L::RB / L::W, lines);
     }
     tm.usable = ok ? 1 : 0;
+    tm.lines = lines ? 1 : 0;
 }
 
 template <class... KArgs, class... Args>

@@ -73,12 +73,18 @@ namespace mma {
 // consecutive token rows then sit in eight different bank groups, which is what makes the
 // ldmatrix.trans fetches of the value codes (eight rows per matrix) conflict-free: measured on the
 // plain row-major layout, those fetches alone cost 4 to 8 shared-memory wavefronts per matrix.
+//
+// A tile row's number is a signed 32-bit coordinate, which rows of 32 bytes exceed from 64 GiB on and rows of 64 bytes from
+// 128 GiB on; a copy from beyond it ends in an illegal instruction.  Caches that long are described by lines of 128 bytes,
+// each of one, two or four rows: the same bytes in the same order, up to 256 GiB.
+constexpr int kLineBytes = 128;     // blocks start on it wherever their sizes are packed without gaps; others are copied by hand
 struct alignas(64) TensorMaps {
     CUtensorMap m[3];   // 0: raw bf16 rows, 1: 8-bit codes, 2: 4-bit codes
     CUtensorMap planes; // row form: the four scale planes as (plane, block, bytes), when they lie at equal distances
     int usable;         // 0: no tiled copies (base pointer not 16-byte aligned, or no encoder): blocks are copied by hand
     int planes_tiled;   // 1: `planes` is valid, a block's four planes are one copy
-    int pad[14];
+    int lines;          // 1: `m` has three dimensions, (bytes, rows of a line, lines of kLineBytes): more tile rows than a coordinate counts
+    int pad[13];
 };
 
 constexpr int kConsumerWarps = 12;       // three warpgroups
@@ -676,10 +682,11 @@ __device__ __forceinline__ bool produce_item(const Params& p, const TensorMaps& 
                     mbar_expect_tx(&full[my_slot], planes);
                     tma_tile3_g2s(ring + my_dst + dbytes, &tm.planes, 0, it.row * p.nb + (int)cur.w, 0, &full[my_slot]);
                 }
-                if (tw && tm.usable && (soff & (unsigned long long)(tw - 1)) == 0) {
+                if (tw && tm.usable && (soff & (unsigned long long)((tm.lines ? kLineBytes : tw) - 1)) == 0) {
                     // a box of tile rows, written swizzled (row = byte offset / row width)
                     mbar_arrive_tx(&full[my_slot], dbytes + behind);
-                    tma_tile_g2s(ring + my_dst, tmap, 0, (int)(soff >> twl), &full[my_slot]);
+                    if (tm.lines) tma_tile3_g2s(ring + my_dst, tmap, 0, 0, (int)(soff / kLineBytes), &full[my_slot]);
+                    else tma_tile_g2s(ring + my_dst, tmap, 0, (int)(soff >> twl), &full[my_slot]);
                     if (behind) bulk_g2s(ring + my_dst + dbytes, src + dbytes, behind, &full[my_slot]);
                 } else if (!tw && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
                     mbar_arrive_tx(&full[my_slot], dbytes + behind);
