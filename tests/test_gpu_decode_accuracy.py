@@ -56,3 +56,26 @@ def test_a_long_8_bit_row_is_as_accurate_for_eight_heads_as_for_four(ext):
         del cache
     rms = lambda e: float(torch.stack(e).square().mean().sqrt())
     assert rms(eight) < 1.6 * rms(four)
+
+
+@pytest.mark.parametrize("rep", [1, 2, 4, 5, 8])
+@pytest.mark.parametrize("D,group", [(128, 32), (64, 16)])
+def test_a_token_that_takes_the_whole_weight_comes_out_as_it_was_stored(ext, rep, D, group):
+    """Raw blocks: the largest weight is 1, which its two bf16 halves hold exactly.  The query is 70 to 88 times one
+    key of length 1, so the other tokens' weights vanish.  The rounding of an exponent cancels in the division; what is left
+    are two truncations, 2^-22.  Weights one rounding of 16 bits off differ by up to 2^-17."""
+    from geodesia_kv_b200.pack_layout import pack_cache
+    gen = torch.Generator(device="cuda").manual_seed(rep * D)
+    T, Hkv = 64 * 12, 2
+    k = torch.nn.functional.normalize(torch.randn(1, Hkv, T, D, device="cuda", generator=gen), dim=-1).to(torch.bfloat16)
+    v = torch.randn(1, Hkv, T, D, device="cuda", generator=gen).to(torch.bfloat16)
+    cache = pack_cache(k, v, torch.full((1, Hkv, T // 64), 16, dtype=torch.int32, device="cuda"), group)
+    at = torch.randint(0, T, (Hkv, rep), device="cuda", generator=gen)
+    picked = k[0, torch.arange(Hkv, device="cuda")[:, None], at].float()
+    q = (picked * torch.linspace(70.0, 88.0, rep, device="cuda")[None, :, None]).reshape(1, Hkv * rep, D).contiguous()
+    scores = torch.einsum("hrd,htd->hrt", q.view(Hkv, rep, D).double(), k[0].double())
+    rest = torch.softmax(scores, -1).scatter(-1, at[..., None], 0.0).sum(-1).max()
+    assert rest < 2.0 ** -24                                   # the case is what it says
+    out = ext.mixed_attn_decode(q, *cache.kernel_args()).view(Hkv, rep, D).double()
+    want = v[0, torch.arange(Hkv, device="cuda")[:, None], at].double()
+    assert ((out - want).norm(dim=-1) / want.norm(dim=-1)).max() < 2.0 ** -21
