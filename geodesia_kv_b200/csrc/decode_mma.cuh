@@ -1693,22 +1693,30 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // operand of O[head][channel], weight halves in the rows).  So O's columns 2t and 2t+1 of this thread are the D / 4 channels
 // from t * D / 4, whole runs of its record.
 //
+// Both operands are two fp16 halves of 22 bits; what is added up stays in fp32 and is rounded, not truncated: every MMA starts
+// from zero and its result is added by the FP32 pipes (sixteen blocks at a time that costs nothing: 42.3 us for 128 x 16k
+// tokens of eight heads per row with and without), and scores, reference and record are in natural units, a power of two
+// away from the products.  Against 64 bits the error of a row of centroids alone is that of FP32 arithmetic throughout: 1.2e-7
+// of the result's norm at 2000 and at 16k tokens, 2.0e-7 where a few tokens dominate; sums kept in the MMAs' accumulators
+// and scores in units of log2: 2.5e-7 at 2000 tokens, 4.5e-7 where a few dominate.
+//
 // On the FP32 pipes, a block at a time with a shuffle reduction per head, a block took a warp 4200 cycles, as much as one of
-// 64 tokens at 4 bits.  32 x 16k tokens, all centroids: 64.8 -> 39.3 us with four heads per row, 76.6 -> 45.3 with eight; 256
-// ragged sequences demoted to 4 bits 381 -> 350; one of a million tokens 209 -> 197.  Against 64 bits the error of such a
-// cache is what it was (4.2e-5 of the result's norm at worst, 4.3e-5 before).
+// 64 tokens at 4 bits.  32 x 16k tokens, all centroids, four heads per row 62 -> 35 us; 128 x 16k, two rows of eight heads
+// 78 -> 42; 256 ragged sequences demoted to 4 bits 404 -> 338 with the other changes of that time, 343 before the sums
+// left the accumulators.
 template <int D, int G, bool MASS>
 __device__ __forceinline__ void centroid_item(const Params& p, const Ctx<D, G>& c, const ItemDesc& it, const uint4* tab,
-                                              int first, float f, size_t rec0) {
+                                              int first, float qscale, size_t rec0) {
     using C = Cfg<D, G>;
     constexpr int NK = C::DT / 8;                         // 16-byte pieces of this thread's key channels
     constexpr int VC = D / 8, NV = VC / 8;                // its value channels per token, and their 16-byte pieces
     constexpr float kScale = 256.f;                       // weights are at most 64: well inside fp16, and far from its subnormals
     const int tiles = (it.nblk + 15) >> 4;
-    float o[VC][4];
+    const float unscale = 1.0f / qscale;                  // a power of two
+    float o[VC][2];
 #pragma unroll
-    for (int i = 0; i < VC; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    float m = -INFINITY, l = 0.f;
+    for (int i = 0; i < VC; ++i) o[i][0] = o[i][1] = 0.f;
+    float m = -INFINITY, l = 0.f;                         // natural-log domain
     for (int tile = first; tile < tiles; tile += kConsumerWarps) {
         const int b0 = tile * 16;
         // entries beyond the item repeat its last one; their scores are masked
@@ -1732,26 +1740,22 @@ __device__ __forceinline__ void centroid_item(const Params& p, const Ctx<D, G>& 
             cnt[j] = b0 + i < it.nblk ? (float)((e.z >> 8) & 0xffu) : 0.f;
             orig[j] = (int)e.w;
         }
-        float z[4];
-        {
-            float acc[2][4];
+        float z[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int i = 0; i < C::CH; ++i) {
-                const uint4 qa = qchunk(c, 0, i), qb = qchunk(c, 1, i);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const uint4 w = kw[j][i % NK];
-                    if (i == 0) mma_f16_z(acc[j], qa.x, qa.y, qa.z, qa.w, w.x, w.y);
-                    else mma_f16(acc[j], qa.x, qa.y, qa.z, qa.w, w.x, w.y);
-                    mma_f16(acc[j], qb.x, qb.y, qb.z, qb.w, w.z, w.w);
-                }
-            }
+        for (int i = 0; i < C::CH; ++i) {
+            const uint4 qa = qchunk(c, 0, i), qb = qchunk(c, 1, i);
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                z[2 * j] = cnt[2 * j] > 0.f ? (acc[j][0] + acc[j][2]) * f : -INFINITY;          // log2 domain
-                z[2 * j + 1] = cnt[2 * j + 1] > 0.f ? (acc[j][1] + acc[j][3]) * f : -INFINITY;
+                const uint4 w = kw[j][i % NK];
+                float a[4], b[4];
+                mma_f16_z(a, qa.x, qa.y, qa.z, qa.w, w.x, w.y);
+                mma_f16_z(b, qb.x, qb.y, qb.z, qb.w, w.z, w.w);
+                z[2 * j] += (a[0] + b[0]) + (a[2] + b[2]);
+                z[2 * j + 1] += (a[1] + b[1]) + (a[3] + b[3]);
             }
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) z[j] = cnt[j] > 0.f ? z[j] * unscale : -INFINITY;
         uint4 vw[4][NV];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -1764,20 +1768,20 @@ __device__ __forceinline__ void centroid_item(const Params& p, const Ctx<D, G>& 
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         if (__any_sync(0xffffffffu, mx > m)) {
             const float mn = fmaxf(m, mx);
-            const float corr = m > -INFINITY ? ex2(m - mn) : 0.f;         // rows are heads, on both operands
+            const float corr = m > -INFINITY ? expf(m - mn) : 0.f;        // rows are heads, on both operands
             l *= corr;
 #pragma unroll
-            for (int i = 0; i < VC; ++i) { o[i][0] *= corr; o[i][1] *= corr; o[i][2] *= corr; o[i][3] *= corr; }
+            for (int i = 0; i < VC; ++i) { o[i][0] *= corr; o[i][1] *= corr; }
             m = mn;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            z[j] = ex2(z[j] - m) * cnt[j];
+            z[j] = ex2((z[j] - m) * 1.4426950408889634f) * cnt[j];
             l += z[j];
             if (MASS && c.r < p.rep && cnt[j] > 0.f) {   // the block's whole mass is reported as its first unit
                 constexpr int UPB = kP / G;
                 float2* mp = p.mass_part + ((size_t)it.row * p.nb + orig[j]) * UPB * p.rep + c.r;
-                mp[0] = make_float2(m * 0.6931471805599453f, z[j]);
+                mp[0] = make_float2(m, z[j]);
                 for (int u = 1; u < UPB; ++u) mp[(size_t)u * p.rep] = make_float2(-INFINITY, 0.f);
             }
         }
@@ -1791,21 +1795,24 @@ __device__ __forceinline__ void centroid_item(const Params& p, const Ctx<D, G>& 
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;
-                mma_f16(o[8 * h + i], ph[0], pl[0], ph[1], pl[1], prmt(x0[i >> 1], x1[i >> 1], sel), prmt(x2[i >> 1], x3[i >> 1], sel));
+                float d[4];
+                mma_f16_z(d, ph[0], pl[0], ph[1], pl[1], prmt(x0[i >> 1], x1[i >> 1], sel), prmt(x2[i >> 1], x3[i >> 1], sel));
+                o[8 * h + i][0] += d[0] + d[2];
+                o[8 * h + i][1] += d[1] + d[3];
             }
         }
     }
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
     if (c.r < p.rep) {
-        if (c.t == 0) p.part_ml[rec0 + c.r] = make_float2(m * 0.6931471805599453f, l);
+        if (c.t == 0) p.part_ml[rec0 + c.r] = make_float2(m, l);
         if (first < tiles) {                              // the merge does not read the rows of a record without blocks
             float* out = p.part + (rec0 + c.r) * D + 2 * VC * c.t;
 #pragma unroll
             for (int i = 0; i < VC; i += 4) {
                 float a[4], b[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) { a[k] = (o[i + k][0] + o[i + k][2]) / kScale; b[k] = (o[i + k][1] + o[i + k][3]) / kScale; }
+                for (int k = 0; k < 4; ++k) { a[k] = o[i + k][0] / kScale; b[k] = o[i + k][1] / kScale; }
                 store_run<4>(out + i, a);
                 store_run<4>(out + VC + i, b);
             }
@@ -1838,7 +1845,7 @@ __device__ void consumer_loop(const Params& p, Smem<D, G>& sm, int* abort_flag) 
         const size_t rec0 = (rec_idx * kConsumerWarps + warp) * p.rep;
         if (it.level == 1) {
             // a short item is the work of a few warps: they take turns
-            centroid_item<D, G, MASS>(p, c, it, sm.item_tab + is * kMaxItemBlocks, (warp + 4 * iseq) % kConsumerWarps, sm.sf[ib * 16 + c.r], rec0);
+            centroid_item<D, G, MASS>(p, c, it, sm.item_tab + is * kMaxItemBlocks, (warp + 4 * iseq) % kConsumerWarps, sm.sf[ib * 16 + 8 + c.r], rec0);
         }
         else {
             const int end = stream ? it.end_seq1 : it.end_seq0;

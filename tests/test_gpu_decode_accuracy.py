@@ -79,3 +79,15 @@ def test_a_token_that_takes_the_whole_weight_comes_out_as_it_was_stored(ext, rep
     out = ext.mixed_attn_decode(q, *cache.kernel_args()).view(Hkv, rep, D).double()
     want = v[0, torch.arange(Hkv, device="cuda")[:, None], at].double()
     assert ((out - want).norm(dim=-1) / want.norm(dim=-1)).max() < 2.0 ** -21
+
+
+@pytest.mark.parametrize("T,peak,bound", [(2000, 1.0, 2.0e-7), (16384, 6.0, 3.3e-7)])
+@pytest.mark.parametrize("Hq,Hkv", [(16, 2), (4, 4)])
+def test_rows_of_centroids_are_as_accurate_as_fp32(ext, T, peak, bound, Hq, Hkv):
+    """FP32 arithmetic throughout has 1.2e-7 (one unit of 2^-23) and, with scores six times as large, 2.2e-7; the bounds are one
+    and a half times that, over enough rows for the spread to average out."""
+    got = []
+    for seed in range(12):
+        gen, cache = packed(100 + seed, Hkv, T, 128, 32, 1)
+        got.append(errors(ext, cache, torch.randn(1, Hq, 128, device="cuda", generator=gen) * (peak * 128 ** -0.5)))
+    assert float(torch.stack(got).square().mean().sqrt()) < bound
