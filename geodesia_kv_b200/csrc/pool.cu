@@ -67,15 +67,19 @@ static int pool_alloc(Pool& p, int r, int64_t n, int64_t* out) {
     return GKV_OK;
 }
 
-static int pool_free(Pool& p, int r, int64_t n, const int64_t* offs) {
-    if (n <= 0) return GKV_OK;
+// Everything that can refuse a release, before anything of it is done.
+static int check_free(Pool& p, int r, int64_t n, const int64_t* offs) {
     const int32_t rung = ladder_level(r);
     for (int64_t i = 0; i < n; ++i) {
         const int64_t s = offs[i] >= 0 ? offs[i] / p.slab_bytes : -1;
         if (s < 0 || s >= p.n_slabs || p.slab_rung[s] != rung) return GKV_E_ARG;
     }
+    return grow(p.stack[r], p.room[r], p.n[kTop + r] + n) && grow(p.emptied, p.emptied_room, std::min(n, p.n_slabs)) ? GKV_OK : GKV_E_MEMORY;
+}
+
+static void do_free(Pool& p, int r, int64_t n, const int64_t* offs) {
+    const int32_t rung = ladder_level(r);
     int64_t& top = p.n[kTop + r];
-    if (!grow(p.stack[r], p.room[r], top + n) || !grow(p.emptied, p.emptied_room, std::min(n, p.n_slabs))) return GKV_E_MEMORY;
     for (int64_t i = 0; i < n; ++i) {
         p.stack[r][top++] = offs[i];
         --p.slab_live[offs[i] / p.slab_bytes];
@@ -97,6 +101,12 @@ static int pool_free(Pool& p, int r, int64_t n, const int64_t* offs) {
         std::sort(p.emptied, p.emptied + m);
         for (int64_t i = m - 1; i >= 0; --i) p.free_slabs[p.n[kFreeSlabs]++] = p.emptied[i];
     }
+}
+
+static int pool_free(Pool& p, int r, int64_t n, const int64_t* offs) {
+    if (n <= 0) return GKV_OK;
+    if (const int rc = check_free(p, r, n, offs)) return rc;
+    do_free(p, r, n, offs);
     return GKV_OK;
 }
 
@@ -120,7 +130,8 @@ static int free_by_rung(Pool& p, const int64_t* offs, const int32_t* level, int6
     int64_t start[kRungs + 1];
     by_rung(offs, level, n, sorted, start);
     int rc = GKV_OK;
-    for (int r = 0; r < kRungs && rc == GKV_OK; ++r) rc = pool_free(p, r, start[r + 1] - start[r], sorted + start[r]);
+    for (int r = 0; r < kRungs && rc == GKV_OK; ++r) rc = check_free(p, r, start[r + 1] - start[r], sorted + start[r]);
+    for (int r = 0; r < kRungs && rc == GKV_OK; ++r) do_free(p, r, start[r + 1] - start[r], sorted + start[r]);
     free(sorted);
     return rc;
 }
@@ -271,8 +282,9 @@ int gkv_table_plan_demotion(void* pool, const int64_t* offs, const int32_t* leve
 int gkv_table_apply_demotion(void* pool, int64_t* offs, int32_t* level, int64_t n, const int64_t* off_old, const int64_t* off_new,
                              const int64_t* flat, const int32_t* level_old, const int32_t* level_new) {
     if (!pool || !offs || !level || (n > 0 && (!off_old || !off_new || !flat || !level_old || !level_new))) return GKV_E_NULL;
+    if (const int rc = gkv::free_by_rung(*static_cast<gkv::Pool*>(pool), off_old, level_old, n)) return rc;
     for (int64_t i = 0; i < n; ++i) { offs[flat[i]] = off_new[i]; level[flat[i]] = level_new[i]; }
-    return gkv::free_by_rung(*static_cast<gkv::Pool*>(pool), off_old, level_old, n);
+    return GKV_OK;
 }
 
 }  // extern "C"

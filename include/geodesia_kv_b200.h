@@ -357,7 +357,7 @@ int gkv_pool_free(void *pool, int rung_index, int64_t n, const int64_t *offs);
  * (gkv_paged_enter_blocks) are filled, rows of T tokens of D elements, valid counts and row lengths from tokens[b]
  * (NULL: whole blocks).  demotions: how many entries of the first blocks[b] the targets (rows, nb; ladder indices)
  * demote; plan: the lists of the launch (gkv_paged_demote_entries) for those n, with new slots taken; apply: the table
- * follows, the old slots go back.  What is refused (GKV_E_POOL) changes nothing.                                     */
+ * follows, the old slots go back.  What is refused (GKV_E_POOL, GKV_E_ARG, GKV_E_MEMORY) changes nothing.           */
 int gkv_table_release(void *pool, int64_t *offs, int32_t *level, int64_t entries);
 int gkv_table_enter(void *pool, int64_t *offs, int32_t *level, int B, int Hkv, int cap, int64_t T, int D,
                     const int64_t *first, const int64_t *count, const int64_t *tokens, int64_t *src_off,
