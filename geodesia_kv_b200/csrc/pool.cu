@@ -45,13 +45,25 @@ static bool grow(int64_t*& a, int64_t& room, int64_t need) {
     return true;
 }
 
-static int pool_alloc(Pool& p, int r, int64_t n, int64_t* out) {
-    if (n <= 0) return GKV_OK;
-    const int64_t size = p.slot[r], per_slab = p.slab_bytes / size;
-    int64_t& top = p.n[kTop + r];
-    const int64_t need = n > top ? (n - top + per_slab - 1) / per_slab : 0;
+// Slabs that n slots of a rung take from the common list.
+static int64_t slabs_for(const Pool& p, int r, int64_t n) {
+    const int64_t per_slab = p.slab_bytes / p.slot[r], top = p.n[kTop + r];
+    return n > top ? (n - top + per_slab - 1) / per_slab : 0;
+}
+
+// Everything that can refuse slots of all rungs together, before any is handed out.
+static int check_alloc(Pool& p, const int64_t (&n)[kRungs]) {
+    int64_t need = 0;
+    for (int r = 0; r < kRungs; ++r) need += slabs_for(p, r, n[r]);
     if (need > p.n[kFreeSlabs]) return GKV_E_POOL;
-    if (!grow(p.stack[r], p.room[r], top + need * per_slab)) return GKV_E_MEMORY;
+    for (int r = 0; r < kRungs; ++r)
+        if (!grow(p.stack[r], p.room[r], p.n[kTop + r] + slabs_for(p, r, n[r]) * (p.slab_bytes / p.slot[r]))) return GKV_E_MEMORY;
+    return GKV_OK;
+}
+
+static void do_alloc(Pool& p, int r, int64_t n, int64_t* out) {
+    const int64_t size = p.slot[r], per_slab = p.slab_bytes / size, need = slabs_for(p, r, n);
+    int64_t& top = p.n[kTop + r];
     for (int64_t i = 0; i < need; ++i) {
         const int64_t s = p.free_slabs[--p.n[kFreeSlabs]];
         p.slab_rung[s] = ladder_level(r);
@@ -64,6 +76,14 @@ static int pool_alloc(Pool& p, int r, int64_t n, int64_t* out) {
     }
     p.n[kBytes] += n * size;
     p.n[kPeak] = std::max(p.n[kPeak], p.n[kBytes]);
+}
+
+static int pool_alloc(Pool& p, int r, int64_t n, int64_t* out) {
+    if (n <= 0) return GKV_OK;
+    int64_t want[kRungs] = {0};
+    want[r] = n;
+    if (const int rc = check_alloc(p, want)) return rc;
+    do_alloc(p, r, n, out);
     return GKV_OK;
 }
 
@@ -261,22 +281,17 @@ int gkv_table_plan_demotion(void* pool, const int64_t* offs, const int32_t* leve
     }
     if (k != n) return GKV_E_ARG;
     if (n == 0) return GKV_OK;
+    if (const int rc = gkv::check_alloc(p, want)) return rc;
     int64_t* got = static_cast<int64_t*>(malloc((size_t)n * sizeof(int64_t)));
     if (!got) return GKV_E_MEMORY;
     int64_t start[gkv::kRungs + 1] = {0};
-    int rc = GKV_OK;
     for (int r = 0; r < gkv::kRungs; ++r) {
-        rc = gkv::pool_alloc(p, r, want[r], got + start[r]);
-        if (rc) {                                        // smaller slots are refused whole: the ones taken go back
-            for (int u = 0; u < r; ++u) gkv::pool_free(p, u, want[u], got + start[u]);
-            break;
-        }
+        gkv::do_alloc(p, r, want[r], got + start[r]);
         start[r + 1] = start[r] + want[r];
     }
-    if (rc == GKV_OK)
-        for (int64_t i = 0; i < n; ++i) off_new[i] = got[start[gkv::ladder_index(level_new[i])]++];
+    for (int64_t i = 0; i < n; ++i) off_new[i] = got[start[gkv::ladder_index(level_new[i])]++];
     free(got);
-    return rc;
+    return GKV_OK;
 }
 
 int gkv_table_apply_demotion(void* pool, int64_t* offs, int32_t* level, int64_t n, const int64_t* off_old, const int64_t* off_new,

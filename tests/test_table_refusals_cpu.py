@@ -4,6 +4,8 @@ import pytest
 
 from geodesia_kv_b200.paged import LADDER, PagedLayerCache, PagedPool, PoolExhausted, _addr
 
+P = 64
+
 
 def state(pool):
     return [s.tolist() for s in pool._stack.values()] + [pool._free_slabs, pool._slab_rung.tolist(), pool._slab_live.tolist(), pool._counters.tolist()]
@@ -30,3 +32,19 @@ def test_a_release_or_a_demotion_that_is_refused_changes_nothing(wrong):
     c.offs_h[1, wrong] = good
     assert c.lib.gkv_table_release(pool.handle, _addr(c.offs_h), _addr(c.level_h), 8) == 0
     assert pool.bytes_in_use == pool.slot[LADDER[(LADDER.index(levels[1, wrong]) + 2) % 5]] and (c.level_h == 0).all()
+
+
+def test_a_demotion_that_does_not_fit_changes_nothing():
+    """Slots of 8 bits would fit, slots of 4 bits would not: the former are not taken, so neither the peak nor the order in which
+    slots are handed out changes."""
+    pool = PagedPool(4 * 1474560, 128, 32, device="cpu")         # four slabs
+    eights = pool.alloc(8, 3 * 80)
+    c = PagedLayerCache(pool, 1, 1)
+    c.offs_h[0, :40], c.level_h[0, :40], c.len_h[0] = pool.alloc(16, 40), 16, 40 * P
+    pool.free(8, eights[7:27])
+    pool._counters[2] = pool._counters[1]
+    before, tgt = state(pool), np.zeros((1, 40), dtype=np.int32)
+    tgt[0, 10:20], tgt[0, 20:30] = LADDER.index(8), LADDER.index(4)
+    with pytest.raises(PoolExhausted):
+        c.apply_demotion(tgt)
+    assert state(pool) == before and (c.level_h[0, :40] == 16).all()
