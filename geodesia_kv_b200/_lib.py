@@ -55,6 +55,7 @@ SIGNATURES = {
     "gkv_pool_create": (_vp, [_i64, _i64] + [_vp] * 5),
     "gkv_pool_destroy": (None, [_vp]),
     "gkv_pool_stack": (_vp, [_vp, _i]),
+    "gkv_pool_restore_stack": (_i, [_vp, _i, _i64, _vp]),
     "gkv_pool_alloc": (_i, [_vp, _i, _i64, _vp]),
     "gkv_pool_free": (_i, [_vp, _i, _i64, _vp]),
     "gkv_table_release": (_i, [_vp] * 3 + [_i64]),

@@ -195,6 +195,16 @@ const int64_t* gkv_pool_stack(void* pool, int rung_index) {
     return pool && rung_index >= 0 && rung_index < gkv::kRungs ? static_cast<gkv::Pool*>(pool)->stack[rung_index] : nullptr;
 }
 
+int gkv_pool_restore_stack(void* pool, int rung_index, int64_t n, const int64_t* slots) {
+    if (!pool || (n > 0 && !slots)) return GKV_E_NULL;
+    if (rung_index < 0 || rung_index >= gkv::kRungs || n < 0) return GKV_E_ARG;
+    gkv::Pool& p = *static_cast<gkv::Pool*>(pool);
+    if (!gkv::grow(p.stack[rung_index], p.room[rung_index], n)) return GKV_E_MEMORY;
+    if (n > 0) memcpy(p.stack[rung_index], slots, (size_t)n * sizeof(int64_t));
+    p.n[gkv::kTop + rung_index] = n;
+    return GKV_OK;
+}
+
 int gkv_pool_alloc(void* pool, int rung_index, int64_t n, int64_t* out) {
     if (!pool || (n > 0 && !out)) return GKV_E_NULL;
     if (rung_index < 0 || rung_index >= gkv::kRungs) return GKV_E_ARG;

@@ -67,6 +67,44 @@ class PoolExhausted(RuntimeError):
     pass
 
 
+class _Books:
+    """The native bookkeeping of a pool (csrc/pool.cu) with the arrays that are its memory; the stacks of free slots are its
+    own.  Shared by shallow copies of the pool; deep copies and pickles carry the state to a new one."""
+
+    def __init__(self, slab_bytes: int, n_slabs: int, slot_bytes: Sequence[int]):
+        self.args = (slab_bytes, n_slabs, tuple(slot_bytes))
+        self.slab_rung = np.zeros(n_slabs, dtype=np.int32)           # 0 = unassigned
+        self.slab_live = np.zeros(n_slabs, dtype=np.int64)
+        self.free_slabs = np.empty(n_slabs, dtype=np.int64)
+        self.counters = np.zeros(8, dtype=np.int64)      # free slabs, bytes in use, their peak, height of each rung's stack
+        lib = _lib.load()
+        self.handle = lib.gkv_pool_create(slab_bytes, n_slabs, (C.c_int64 * 5)(*slot_bytes), *map(_addr, self._arrays()))
+        if not self.handle:
+            raise MemoryError("no memory for the pool's bookkeeping")
+        weakref.finalize(self, lib.gkv_pool_destroy, self.handle)
+
+    def _arrays(self):
+        return self.slab_rung, self.slab_live, self.free_slabs, self.counters
+
+    def stacks(self) -> list:
+        """Free slot offsets of every rung, the next one to hand out last (copies)."""
+        lib = _lib.load()
+        return [np.array((C.c_int64 * n).from_address(lib.gkv_pool_stack(self.handle, i)) if n else (), dtype=np.int64)
+                for i, n in enumerate(self.counters[3:].tolist())]
+
+    def __getstate__(self):
+        return self.args, [a.copy() for a in self._arrays()], self.stacks()
+
+    def __setstate__(self, state):
+        args, arrays, stacks = state
+        self.__init__(*args)
+        for mine, a in zip(self._arrays(), arrays):
+            mine[:] = a
+        for i, s in enumerate(stacks):
+            if _lib.load().gkv_pool_restore_stack(self.handle, i, s.size, _addr(s)):
+                raise MemoryError("no memory for the pool's bookkeeping")
+
+
 class PagedPool:
     """Byte pool with one free list per rung (host-side bookkeeping, device-side bytes)."""
 
@@ -84,19 +122,29 @@ class PagedPool:
         if self.n_slabs < 1:
             raise ValueError(f"capacity below one slab of {self.slab_bytes} bytes")
         self.data = torch.empty(self.n_slabs * self.slab_bytes, dtype=torch.uint8, device=self.device)
-        # The bookkeeping itself is native (csrc/pool.cu); these arrays are its memory, the stacks of free slots are its own.
-        self._slab_rung = np.zeros(self.n_slabs, dtype=np.int32)           # 0 = unassigned
-        self._slab_live = np.zeros(self.n_slabs, dtype=np.int64)
-        self._slabs = np.empty(self.n_slabs, dtype=np.int64)
-        self._counters = np.zeros(8, dtype=np.int64)     # free slabs, bytes in use, their peak, height of each rung's stack
-        self.lib = lib
-        self.handle = lib.gkv_pool_create(self.slab_bytes, self.n_slabs, (C.c_int64 * 5)(*(self.slot[r] for r in LADDER)),
-                                          _addr(self._slab_rung), _addr(self._slab_live), _addr(self._slabs), _addr(self._counters))
-        if not self.handle:
-            raise MemoryError("no memory for the pool's bookkeeping")
-        weakref.finalize(self, lib.gkv_pool_destroy, self.handle)
+        self._books = _Books(self.slab_bytes, self.n_slabs, [self.slot[r] for r in LADDER])
+
+    @property
+    def lib(self):
+        return _lib.load()
+
+    @property
+    def handle(self) -> int:
+        return self._books.handle
 
     # -- accounting ---------------------------------------------------------------------------
+    @property
+    def _slab_rung(self) -> np.ndarray:
+        return self._books.slab_rung
+
+    @property
+    def _slab_live(self) -> np.ndarray:
+        return self._books.slab_live
+
+    @property
+    def _counters(self) -> np.ndarray:
+        return self._books.counters
+
     @property
     def bytes_in_use(self) -> int:
         """Bytes of the slots handed out."""
@@ -108,7 +156,7 @@ class PagedPool:
 
     @property
     def _free_slabs(self) -> list:
-        return self._slabs[:self._counters[0]].tolist()
+        return self._books.free_slabs[:self._counters[0]].tolist()
 
     @property
     def _top(self) -> dict:
@@ -117,8 +165,7 @@ class PagedPool:
     @property
     def _stack(self) -> dict:
         """Free slot offsets of every rung (a copy)."""
-        return {r: np.array((C.c_int64 * n).from_address(self.lib.gkv_pool_stack(self.handle, i)) if n else (), dtype=np.int64)
-                for i, (r, n) in enumerate(self._top.items())}
+        return dict(zip(LADDER, self._books.stacks()))
 
     @property
     def capacity_bytes(self) -> int:

@@ -343,11 +343,13 @@ int gkv_paged_clear_table(int64_t *offs, int32_t *level, int32_t *valid, float *
  * free_slabs (n_slabs) and counters[8] (free slabs, bytes in use, their peak, height of each rung's stack of free
  * slots) are the caller's memory and stay readable.  Slots are handed out low addresses first; a slab returns to the
  * common list with its last slot.  alloc: GKV_E_POOL and no change when the request does not fit; free: GKV_E_ARG and
- * no change when an offset is not of a slab of that rung.  Calls on one pool must not overlap.                       */
+ * no change when an offset is not of a slab of that rung.  A copy of a pool is a new one that is given the contents of
+ * the arrays and, by restore_stack, of the stacks.  Calls on one pool must not overlap.                              */
 void *gkv_pool_create(int64_t slab_bytes, int64_t n_slabs, const int64_t *slot_bytes, int32_t *slab_rung,
                       int64_t *slab_live, int64_t *free_slabs, int64_t *counters);
 void gkv_pool_destroy(void *pool);
 const int64_t *gkv_pool_stack(void *pool, int rung_index);
+int gkv_pool_restore_stack(void *pool, int rung_index, int64_t n, const int64_t *slots);
 int gkv_pool_alloc(void *pool, int rung_index, int64_t n, int64_t *out);
 int gkv_pool_free(void *pool, int rung_index, int64_t n, const int64_t *offs);
 
