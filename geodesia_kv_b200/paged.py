@@ -466,8 +466,14 @@ class PagedLayerCache:
     def apply_demotion(self, tgt_idx_host: np.ndarray) -> int:
         """Demote to the allocator's result (host array (rows, nb) of ladder indices): allocate the
         smaller slots, re-quantise on the device, free the larger slots.  Returns blocks demoted."""
-        tgt = np.ascontiguousarray(np.broadcast_to(tgt_idx_host, (self.rows, tgt_idx_host.shape[1])), dtype=np.int32)
-        nb, lib, dev = tgt.shape[1], self.lib, self.device
+        nb, lib, dev = tgt_idx_host.shape[1], self.lib, self.device
+        if nb > self.cap:
+            raise ValueError(f"targets for {nb} blocks, the table has {self.cap}")
+        if tgt_idx_host.dtype != np.int32:
+            if tgt_idx_host.dtype.kind not in "iub":
+                raise IndexError("targets are ladder indices, which are integers")
+            tgt_idx_host = np.clip(tgt_idx_host, 0, 4)                # whatever is out of range stays so in 32 bits
+        tgt = np.ascontiguousarray(np.broadcast_to(tgt_idx_host, (self.rows, nb)), dtype=np.int32)
         blocks = self.blocks_per_seq()
         table = (_addr(self.offs_h), _addr(self.level_h), self.B, self.Hkv, self.cap, _addr(blocks), _addr(tgt), nb)
         n = int(lib.gkv_table_demotions(*table))

@@ -48,3 +48,40 @@ def test_a_demotion_that_does_not_fit_changes_nothing():
     with pytest.raises(PoolExhausted):
         c.apply_demotion(tgt)
     assert state(pool) == before and (c.level_h[0, :40] == 16).all()
+
+
+def demotable(B=1, Hkv=2, nb=4):
+    """A table of raw blocks whose demotions stop before the launch, with the rungs they chose."""
+    c = PagedLayerCache(PagedPool(10 * 1474560, 128, 32, device="cpu"), B, Hkv, cap_blocks=nb)
+    c.offs_h[:], c.level_h[:], c.len_h[:] = c.pool.alloc(16, c.rows * nb).reshape(c.rows, nb), 16, nb * P
+
+    class Planned(Exception):
+        pass
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(c.pool.lib, name)
+
+        def gkv_table_demotions(self, offs, level, B, Hkv, cap, blocks, tgt, nb):
+            import ctypes
+            raise Planned(np.clip(np.array((ctypes.c_int32 * (B * Hkv * nb)).from_address(tgt)), 0, 4).tolist())
+
+    c.lib = Lib()
+    return c, Planned
+
+
+@pytest.mark.parametrize("tgt,error", [(np.zeros((2, 5), np.int32), ValueError), (np.zeros((3, 4), np.int32), ValueError),
+                                       (np.full((2, 4), 1.9), IndexError), (np.zeros((2, 4), complex), IndexError)])
+def test_targets_that_no_table_of_ladder_indices_can_be_are_refused(tgt, error):
+    c, _ = demotable()
+    with pytest.raises(error):
+        c.apply_demotion(tgt)
+
+
+@pytest.mark.parametrize("dtype,big", [(np.int64, 1 << 32), (np.uint32, (1 << 32) - 1), (np.int32, 1 << 30), (np.uint8, 255), (np.int64, -(1 << 33))])
+def test_targets_of_every_integer_type_count_as_the_nearest_rung(dtype, big):
+    c, planned = demotable()
+    tgt = np.array([[0, 1, 4, big]] * 2).astype(dtype)
+    with pytest.raises(planned) as e:
+        c.apply_demotion(tgt)
+    assert e.value.args[0] == [0, 1, 4, 0 if big < 0 else 4] * 2
