@@ -150,9 +150,18 @@ class PagedPool:
         """Bytes of the slots handed out."""
         return int(self._counters[1])
 
+    @bytes_in_use.setter
+    def bytes_in_use(self, n: int) -> None:
+        self._counters[1] = n
+
     @property
     def peak_bytes_in_use(self) -> int:
+        """The most it has been; may be set, for instance back to ``bytes_in_use``."""
         return int(self._counters[2])
+
+    @peak_bytes_in_use.setter
+    def peak_bytes_in_use(self, n: int) -> None:
+        self._counters[2] = n
 
     @property
     def _free_slabs(self) -> list:

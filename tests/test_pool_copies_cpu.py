@@ -49,3 +49,11 @@ def test_a_shallow_copy_shares_the_bookkeeping_for_as_long_as_either_lives():
     gc.collect()
     assert books(other) == before
     other.free(8, a)
+
+
+def test_the_peak_can_be_set_back():
+    pool, held = used_pool()
+    assert pool.peak_bytes_in_use > pool.bytes_in_use
+    pool.peak_bytes_in_use = pool.bytes_in_use
+    pool.alloc(16, 1)
+    assert pool.peak_bytes_in_use == pool.bytes_in_use
