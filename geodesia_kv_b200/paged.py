@@ -25,6 +25,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import operator
 import weakref
 from typing import Sequence
 
@@ -36,7 +37,7 @@ from ._cuda import on, stream as _stream
 
 BLOCK = 64
 LADDER = (16, 8, 4, 2, 1)
-_LADDER_NP = np.array(LADDER, dtype=np.int32)
+_INDEX = {r: i for i, r in enumerate(LADDER)}
 _DT = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
 
 
@@ -200,16 +201,17 @@ class PagedPool:
 
     def alloc(self, rung: int, n: int) -> np.ndarray:
         """Offsets of n free slots of a rung (int64); refused with every slab where it was: smaller slots may still fit."""
-        out = np.empty(max(int(n), 0), dtype=np.int64)
-        if out.size:
-            self._check(self.lib.gkv_pool_alloc(self.handle, LADDER.index(rung), out.size, _addr(out)), f"{n} slots of rung {rung}")
+        if n <= 0:
+            return np.empty(0, dtype=np.int64)
+        out = np.empty(operator.index(n), dtype=np.int64)
+        self._check(self.lib.gkv_pool_alloc(self.handle, _INDEX[rung], out.size, _addr(out)), f"{n} slots of rung {rung}")
         return out
 
     def free(self, rung: int, offs: np.ndarray) -> None:
         """Give slots of a rung back; slabs left without a live slot return to the common list."""
         offs = np.ascontiguousarray(offs, dtype=np.int64)
         if offs.size:
-            self._check(self.lib.gkv_pool_free(self.handle, LADDER.index(rung), offs.size, _addr(offs)), "a release")
+            self._check(self.lib.gkv_pool_free(self.handle, _INDEX.get(rung, -1), offs.size, _addr(offs)), "a release")
 
 
 class PagedLayerCache:

@@ -85,3 +85,14 @@ def test_targets_of_every_integer_type_count_as_the_nearest_rung(dtype, big):
     with pytest.raises(planned) as e:
         c.apply_demotion(tgt)
     assert e.value.args[0] == [0, 1, 4, 0 if big < 0 else 4] * 2
+
+
+def test_slots_are_asked_for_by_whole_numbers_of_a_rung_on_the_ladder():
+    pool = PagedPool(2 * 1474560, 128, 32, device="cpu")
+    with pytest.raises(TypeError):
+        pool.alloc(16, 2.5)
+    with pytest.raises(KeyError):
+        pool.alloc(3, 1)
+    with pytest.raises(ValueError):
+        pool.free(3, pool.alloc(16, 1))
+    assert pool.alloc(3, 0).size == 0 and pool.alloc(np.int32(8), np.int64(3)).size == 3
