@@ -803,6 +803,8 @@ const char* gkv_error_string(int code) {
         case GKV_E_CUDA: return "a CUDA call failed (see gkv_last_cuda_error)";
         case GKV_E_ARG: return "an argument is out of range";
         case GKV_E_STATIC_SCRATCH: return "problem too large for the built-in scratch of gkv_mixed_attn_decode_static";
+        case GKV_E_POOL: return "the block pool has no slots left for the request";
+        case GKV_E_MEMORY: return "host memory ran out";
         default: return "unknown error code";
     }
 }

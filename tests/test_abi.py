@@ -88,3 +88,11 @@ def test_get_ext_follows_the_reference_contract(monkeypatch):
         import pytest
         with pytest.raises(RuntimeError, match="no CPU path"):
             cuda_ext.mixed_attn_decode(*([None] * 9))
+
+
+def test_every_error_code_of_the_header_has_a_text_of_its_own():
+    from geodesia_kv_b200 import _lib
+    codes = {n: int(v) for n, v in re.findall(r"#define (GKV_E_[A-Z_]+) \((-\d+)\)", (ROOT / "include" / "geodesia_kv_b200.h").read_text())}
+    assert codes["GKV_E_MEMORY"] == -9
+    texts = [_lib.load().gkv_error_string(c) for c in codes.values()]
+    assert len(set(texts) | {b"unknown error code"}) == len(codes) + 1
