@@ -31,7 +31,7 @@ struct CombineParams {
     int per_seg;         //      a (segs, rows) list of records
     float2* ml_out;      // optional, final level only: (M, L) of every output row (for the per-block softmax mass)
     // Internal layout written by the tensor-core kernel: a row's used item slots are a prefix of its
-    // slots (the rest hold "empty" records), and how many are used follows from the row's rung-class
+    // slots (nothing is written to the rest), and how many are used follows from the row's rung-class
     // counts — so the merge reads only the records that exist.  Null for other producers.
     const int32_t* plan_tab;
     int chunk, tab_per_row, warps_per_item;
@@ -713,10 +713,10 @@ static int decode_impl(const float* q, const uint8_t* data, const int64_t* offs,
         mp.plan = plan; mp.rows = rows;
         mp.plan_tab = reinterpret_cast<const int32_t*>(reinterpret_cast<const uint8_t*>(plan) + perm_entries_bytes(meta_rows, nb));
         combine_tab = mp.plan_tab;
-        mp.q = q; mp.data = data; mp.offs = offs;
+        mp.q = q; mp.data = data;
         mp.klo = static_cast<const __half*>(klo); mp.kstep = static_cast<const __half*>(kstep);
         mp.vlo = static_cast<const __half*>(vlo); mp.vstep = static_cast<const __half*>(vstep);
-        mp.level = level; mp.valid = valid; mp.part = records; mp.part_ml = records_ml; mp.counter = header; mp.status = header + 1;
+        mp.part = records; mp.part_ml = records_ml; mp.counter = header; mp.status = header + 1;
         mp.mass_part = mass_part;
         mp.B = B; mp.Hq = Hq; mp.Hkv = Hkv; mp.nb = nb; mp.rep = rep; mp.chunk = pl.bps;
         mp.items_per_row = pl.nsplit; mp.items = rows * pl.nsplit; mp.per_row_meta = meta_rows != 1;

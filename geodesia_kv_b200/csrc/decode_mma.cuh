@@ -144,21 +144,18 @@ struct ItemDesc {       // one work item; published one item ahead of its blocks
 struct Params {
     const float* q;
     const uint8_t* data;
-    const int64_t* offs;
     const __half* klo;
     const __half* kstep;
     const __half* vlo;
     const __half* vstep;
-    const int32_t* level;
-    const int32_t* valid;
     const uint4* plan;       // (metadata rows, nb) block entries of every row sorted by rung, from plan_kernel
     const int32_t* plan_tab; // (metadata rows, kPlanTabInts) start of each rung class in that list
     float* part;             // (rows, items per row, consumer warps, rep, D): o of every record
     float2* part_ml;         // (rows, items per row, consumer warps, rep): its (m, l)
-    float2* mass_part;       // optional (rows, nb, 2 units, rep): (reference, sum of weights against it) per block half and head,
+    float2* mass_part;       // optional (rows, nb, 64 / G units, rep): (reference, sum of weights against it) per unit and head,
                              // natural-log domain; the by-product from which the per-block softmax mass is made
-    int* counter;            // work-item counter (zeroed before launch)
-    int* status;             // error word (zeroed before launch)
+    int* counter;            // work-item counter (zeroed before launch; not read when items are dealt)
+    int* status;             // error word (zeroed before launch, or by this kernel: clear_status)
     int B, Hq, Hkv, nb, rep;
     int chunk;               // blocks per item (the last item of a rung's run may be shorter)
     int items_per_row, items;
@@ -166,7 +163,7 @@ struct Params {
     int dealt;               // 1: CTA i takes the items i, i + grid, ...; 0: items are drawn from the counter
     int clear_status;        // 1: this kernel is the first of its call and clears the status word itself
     int rows;
-    int paged;               // 1: `data` is a block pool, offs are pool offsets, and the four scale planes of a quantised
+    int paged;               // 1: `data` is a block pool, the lists hold pool offsets, and the four scale planes of a quantised
                              // block sit right behind its bytes ([klo][kstep][vlo][vstep]); klo..vstep above are unused
     int64_t stride_bh;
 };
@@ -654,8 +651,7 @@ __device__ __forceinline__ bool produce_item(const Params& p, const TensorMaps& 
         }
         // What the lanes have seen released, all of them have (the warp barrier); and the copies below may land on bytes that
         // ordinary stores put there (planes and blocks copied by this warp's lanes, cleared tails): every lane fences before
-        // the copy it starts.  One fence per batch here, not one per block in the warps that release the slots: 32 x 16k
-        // tokens 221.6 against 222.4 us, one sequence of 1M tokens 208.3 against 211.7.
+        // the copy it starts: one fence per batch here, not one per block in the warps that release the slots.
         __syncwarp();
         fence_before_bulk();
         bool withhold = false;
@@ -732,8 +728,8 @@ __device__ __forceinline__ bool produce_item(const Params& p, const TensorMaps& 
 // The scheduler warp draws the work items (an atomic counter), looks up what each one is, fetches
 // its block entries into the item's table in shared memory and announces it — up to kItemSlots - 1
 // items ahead of the consumers, so none of this global-memory latency is ever waited for by the
-// producers or the consumers.  Items without blocks are not announced: their records are marked
-// empty right here.
+// producers or the consumers.  Items without blocks are not announced, and nothing is written to their records: the merge
+// works out how many of a row's records exist and reads no others.
 template <int D, int G>
 __device__ void scheduler_loop(const Params& p, Smem<D, G>& sm, int* abort_flag) {
     const int lane = threadIdx.x & 31;
@@ -823,7 +819,7 @@ __device__ void producer_loop(const Params& p, const TensorMaps& tm, Smem<D, G>&
 }
 
 // ================================ query warp ==================================================
-// For every announced item: the row's query heads as fp32 (for the centroid path), a per-head
+// For every announced item: the row's query heads, a per-head
 // power-of-two scale, and the MMA A-fragment planes (hi, lo) in the channel arrangement of the
 // item's rung, into the buffer of the item's parity.  Runs one item ahead of the consumers.
 //
@@ -967,7 +963,6 @@ struct WarpState {
 template <int D, int G>
 struct Ctx {                             // per-thread constants of the consumer role
     uint32_t qprep;                      // shared address of this lane's first prepared-query chunk (hi plane)
-    uint32_t sq;                         // shared address of the fp32 query rows
     float f;                             // 2^-eq * log2(e) of this thread's head
     int r, t, lane;
     bool part;                           // with head pairs in the rows: this thread feeds the lo column of its head
@@ -1839,7 +1834,6 @@ __device__ void consumer_loop(const Params& p, Smem<D, G>& sm, int* abort_flag) 
         if (it.exit) return;
         if (!mbar_wait(&sm.qready[ib], (uint32_t)(iseq >> 1) & 1u)) { code = 3; break; }
         c.qprep = smem_u32(sm.qprep) + (uint32_t)(ib * C::QPREP_BYTES) + (uint32_t)lane * 16u;
-        c.sq = smem_u32(sm.sq) + (uint32_t)(ib * C::SQ_BYTES);
         c.f = sm.sf[ib * 16 + (DUP ? c.t : c.r)];
         const size_t rec_idx = (size_t)it.row * p.items_per_row + (size_t)(it.item / p.rows);
         const size_t rec0 = (rec_idx * kConsumerWarps + warp) * p.rep;
