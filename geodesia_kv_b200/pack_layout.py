@@ -106,7 +106,8 @@ def layout_offsets(level: torch.Tensor, D: int, align: int = 1):
 def _scale_planes(B: int, Hkv: int, nb: int, D: int, group: int, dev) -> list:
     """klo, kstep (B, Hkv, nb, G, D) and vlo, vstep (B, Hkv, nb, 64, gv).  Where groups divide block and row evenly the four are
     of one size and parts of one buffer: at equal distances a block's share of all four is one tiled copy of the decode
-    kernel (as four allocations 32 x 16k tokens at 4 bits take 174 us instead of 165)."""
+    kernel (as four allocations 32 x 16k tokens at 4 bits take 174 us instead of 165).  One plane alone keeps the buffer of all
+    four alive, and ``torch.save`` writes it whole: ``clone`` a plane that is to be kept or saved without the others."""
     G, gv = (BLOCK + group - 1) // group, (D + group - 1) // group
     if G * D == BLOCK * gv and G * D % 8 == 0:            # every part on a 16-byte boundary
         klo, kstep, vlo, vstep = torch.empty(4, B, Hkv, nb, G, D, dtype=torch.float16, device=dev).unbind(0)
