@@ -523,13 +523,15 @@ static bool encode_rows(CUtensorMap* map, const uint8_t* data, size_t total_byte
     if (!enc || w < 32 || rows > 256 || rows % per || total_bytes / (size_t)w == 0) return false;
     const cuuint64_t groups = total_bytes / mma::kLineBytes;
     if ((lines ? groups : total_bytes / (size_t)w) > 0x7fffffffu) return false;      // beyond the coordinates
-    const cuuint64_t dims[3] = {(cuuint64_t)w, lines ? (cuuint64_t)per : (cuuint64_t)(total_bytes / (size_t)w), groups};
-    const cuuint64_t strides[2] = {(cuuint64_t)w, (cuuint64_t)mma::kLineBytes};
+    // one form of copy for both: choosing it block by block cost the producers 1 % of a mix of rungs (ten batch sizes)
+    const cuuint64_t all = total_bytes / (size_t)w;
+    const cuuint64_t dims[3] = {(cuuint64_t)w, lines ? (cuuint64_t)per : all, lines ? groups : 1};
+    const cuuint64_t strides[2] = {(cuuint64_t)w, lines ? (cuuint64_t)mma::kLineBytes : all * (cuuint64_t)w};
     const cuuint32_t box[3] = {(cuuint32_t)w, (cuuint32_t)per, (cuuint32_t)(rows / per)};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapSwizzle sw = w == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : w == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
                                                                                    : CU_TENSOR_MAP_SWIZZLE_32B;
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, lines ? 3 : 2, const_cast<uint8_t*>(data), dims, strides, box, estr,
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(data), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }

@@ -67,7 +67,7 @@ namespace gkv {
 namespace mma {
 
 // Tensor maps of the cache bytes, one per rung whose blocks are fetched with a TILED bulk copy: the
-// cache is described as a 2-D byte matrix of `w`-byte rows (w = bytes of a token row, at most 128),
+// cache is described as a byte matrix of `w`-byte rows (w = bytes of a token row, at most 128),
 // a block is a box of consecutive rows, and the copy engine writes the box into shared memory with
 // the 16-byte chunks of every row XOR-permuted by the row number (the hardware swizzle).  Eight
 // consecutive token rows then sit in eight different bank groups, which is what makes the
@@ -83,7 +83,7 @@ struct alignas(64) TensorMaps {
     CUtensorMap planes; // row form: the four scale planes as (plane, block, bytes), when they lie at equal distances
     int usable;         // 0: no tiled copies (base pointer not 16-byte aligned, or no encoder): blocks are copied by hand
     int planes_tiled;   // 1: `planes` is valid, a block's four planes are one copy
-    int lines;          // 1: `m` has three dimensions, (bytes, rows of a line, lines of kLineBytes): more tile rows than a coordinate counts
+    int lines;          // `m` is (bytes, rows, 1), or 1: (bytes, rows of a line, lines of kLineBytes), for more tile rows than a coordinate counts
     int pad[13];
 };
 
@@ -269,11 +269,6 @@ template <int D, int G, int BITS>
 __device__ __forceinline__ uint32_t swz_term(int r, int b0) {
     using L = Lay<D, G, BITS>;
     return ((((uint32_t)r * L::RB + (uint32_t)b0) >> 7) & L::XMASK) << 4;
-}
-
-__device__ __forceinline__ void tma_tile_g2s(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void tma_tile3_g2s(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
@@ -611,7 +606,8 @@ __device__ __forceinline__ bool produce_item(const Params& p, const TensorMaps& 
     // tiled copies: log2 of the tile row width of the item's rung (0: plain bulk copy) and its tensor map
     constexpr int W4 = Lay<D, G, 4>::W;
     const int tw = lv == 16 ? Lay<D, G, 16>::W : lv == 8 ? Lay<D, G, 8>::W : lv == 4 ? W4 : 0;
-    const int twl = tw == 128 ? 7 : tw == 64 ? 6 : 5;
+    const int at_shift = tw == 128 || tm.lines ? 7 : tw == 64 ? 6 : 5;
+    const unsigned long long at_mask = (1ull << at_shift) - 1;
     const CUtensorMap* tmap = &tm.m[lv == 16 ? 0 : lv == 8 ? 1 : 2];
     uint64_t* full = sm.full + s * kNSlot;
     uint64_t* empty = sm.empty + s * kNSlot;
@@ -678,11 +674,11 @@ __device__ __forceinline__ bool produce_item(const Params& p, const TensorMaps& 
                     mbar_expect_tx(&full[my_slot], planes);
                     tma_tile3_g2s(ring + my_dst + dbytes, &tm.planes, 0, it.row * p.nb + (int)cur.w, 0, &full[my_slot]);
                 }
-                if (tw && tm.usable && (soff & (unsigned long long)((tm.lines ? kLineBytes : tw) - 1)) == 0) {
+                if (tw && tm.usable && (soff & at_mask) == 0) {
                     // a box of tile rows, written swizzled (row = byte offset / row width)
                     mbar_arrive_tx(&full[my_slot], dbytes + behind);
-                    if (tm.lines) tma_tile3_g2s(ring + my_dst, tmap, 0, 0, (int)(soff / kLineBytes), &full[my_slot]);
-                    else tma_tile_g2s(ring + my_dst, tmap, 0, (int)(soff >> twl), &full[my_slot]);
+                    const int at = (int)(soff >> at_shift);
+                    tma_tile3_g2s(ring + my_dst, tmap, 0, tm.lines ? 0 : at, tm.lines ? at : 0, &full[my_slot]);
                     if (behind) bulk_g2s(ring + my_dst + dbytes, src + dbytes, behind, &full[my_slot]);
                 } else if (!tw && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
                     mbar_arrive_tx(&full[my_slot], dbytes + behind);
